@@ -242,10 +242,7 @@ constexpr int kSelCand = kSelThreads;
 // Device control block of one selection, followed in memory by 3 * kSelBins
 // histogram words; the launcher zeroes both.
 struct SelectCtl {
-  unsigned int bar_count;
-  unsigned int bar_gen;
-  int err;
-  int pad;
+  GridBar bar;
   unsigned long long ncand;
 };
 
@@ -304,6 +301,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectArgs a) {
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned int nctas = gridDim.x;
   SelectCtl *ctl = a.ctl;
+  unsigned int round = 0;
   // ---- 1. variances, keys, histogram of the top 12 bits --------------------
   for (int i = threadIdx.x; i < kSelBins; i += blockDim.x) h[i] = 0;
   __syncthreads();
@@ -319,7 +317,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectArgs a) {
   __syncthreads();
   for (int i = threadIdx.x; i < kSelBins; i += blockDim.x)
     if (h[i]) atomicAdd(&a.hist[i], h[i]);
-  bool ok = grid_barrier(&ctl->bar_count, &ctl->bar_gen, &ctl->err, a.spin_limit, nctas);
+  bool ok = grid_barrier(&ctl->bar, round++, a.spin_limit, nctas);
   // ---- 2. radix select of rank idx -----------------------------------------
   unsigned long long k = a.idx, prefix = 0, mask = 0;
   int shift = 52, bits = 12, pass = 0;
@@ -355,7 +353,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectArgs a) {
     unsigned int *gh2 = a.hist + (pass % 3) * kSelBins;
     for (int i = threadIdx.x; i < kSelBins; i += blockDim.x)
       if (h[i]) atomicAdd(&gh2[i], h[i]);
-    ok = grid_barrier(&ctl->bar_count, &ctl->bar_gen, &ctl->err, a.spin_limit, nctas);
+    ok = grid_barrier(&ctl->bar, round++, a.spin_limit, nctas);
   }
   if (ok && shift != 0) {
     // the bucket's keys (at most one per thread of a CTA), ranked by counting
@@ -366,7 +364,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectArgs a) {
         if (pos < (unsigned long long)kSelCand) a.cand[pos] = key;
       }
     }
-    ok = grid_barrier(&ctl->bar_count, &ctl->bar_gen, &ctl->err, a.spin_limit, nctas);
+    ok = grid_barrier(&ctl->bar, round++, a.spin_limit, nctas);
     if (ok) {
       if (threadIdx.x == 0) {
         s_nc = __ldcg(&ctl->ncand);

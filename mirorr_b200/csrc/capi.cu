@@ -2001,7 +2001,6 @@ mirorr_status mirorr_pyramid_level(mirorr_ctx c, const mirorr_geometry *ig, cons
 // pinned host buffers the graph's copies read).
 namespace {
 
-constexpr int kLtsCtas = 2;  // CTAs per LTS fit in the batched launch
 
 struct BatchCallBufs {
   DevBuf stats, wand, prep, xs, chunked, fb, best, second, match, status, tiles;
@@ -2053,7 +2052,7 @@ size_t slot_bytes(const mirorr_geometry &fg, const mirorr_geometry &mg, const mi
   b += ncall * (10 * V + 3 * V / 2 + (32 + 256 + 4 + 13) * NB + 2 * V + 64 * 1024);
   if (p.bm.block_keep < 1.0) b += ncall * (17 * NB + 2048);  // variance selection
   b += 2 * 3 * 8 * ncall * NB;                                 // point pairs
-  b += lts_fit_scratch_bytes((long long)(ncall * NB), kLtsCtas);
+  b += lts_fit_scratch_bytes((long long)(ncall * NB));
   return b;
 }
 
@@ -2270,7 +2269,7 @@ mirorr_status batch_check_slot(mirorr_ctx c, const BatchSlot &s) {
             need(s.lvl_m, sizeof(float) * vox(s.lm.size), "lvl_m") &&
             need(s.pts_i, sizeof(double) * 3 * ncall * nb, "pts_i") &&
             need(s.pts_m, sizeof(double) * 3 * ncall * nb, "pts_m") &&
-            need(s.lts_scratch, lts_fit_scratch_bytes(ncall * nb, kLtsCtas), "lts_scratch");
+            need(s.lts_scratch, lts_fit_scratch_bytes(ncall * nb), "lts_scratch");
   if (ok && !s.has_fm) ok = need(c->ones, vox(s.fg.size), "ones (fixed)");
   if (ok && !s.has_mm) ok = need(c->ones, vox(s.mg.size), "ones (moving)");
   for (int k = 0; ok && k < ncall; ++k) {
@@ -2328,8 +2327,7 @@ mirorr_status batch_issue(mirorr_batch b, int njobs, long long max_vox, int ncal
   MB2_TRY(launch_match16_batch(b->storage, ncalls, b->h_calls.as<Match16Call>(), b->d_calls, st,
                                true));
   MB2_TRY(launch_postfilter_batch(b->d_pf.as<PfCall>(), ncalls, max_blocks, st));
-  MB2_TRY(lts_batch_launch(b->fits.data(), nfits, kLtsCtas, c->ltsw.spin_limit, b->d_lts_args,
-                           b->h_lts_args, st));
+  MB2_TRY(lts_batch_launch(b->fits.data(), nfits, b->d_lts_args, b->h_lts_args, st));
   // read back: fit states, point counts, the search's and the fits' give-up flags
   unsigned char *rd = b->h_rd.as<unsigned char>();
   MB2_CUDA_TRY(cudaMemcpyAsync(rd, b->d_states.ptr, sizeof(LtsState) * S, cudaMemcpyDeviceToHost, st));
@@ -2810,7 +2808,7 @@ mirorr_status mirorr_batch_submit(mirorr_batch b, const mirorr_geometry *fg, con
   }
   E(s.pts_i, sizeof(double) * 3 * ncall * max_blocks);
   E(s.pts_m, sizeof(double) * 3 * ncall * max_blocks);
-  E(s.lts_scratch, lts_fit_scratch_bytes(ncall * max_blocks, kLtsCtas));
+  E(s.lts_scratch, lts_fit_scratch_bytes(ncall * max_blocks));
   st = slot_carve(b, s, bufs);
   if (st == MIRORR_OK) st = upload(c, s.in_f, fixed, es * vox(fg->size));
   if (st == MIRORR_OK) st = upload(c, s.in_m, moving, es * vox(mg->size));

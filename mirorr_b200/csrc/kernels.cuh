@@ -252,7 +252,7 @@ mirorr_status launch_smooth_axis(const int size[3], const void *in, float *out, 
                                  int in_dtype = MIRORR_DTYPE_F32);
 mirorr_status launch_fill_u8(uint8_t *p, long long n, uint8_t v, cudaStream_t s);
 
-// LTS fit on device (one cooperative launch for the whole inner loop).
+// LTS fit on device (one launch for the whole inner loop).
 struct LtsWork {
   DevBuf state;     // LtsState
   DevBuf resid;     // double per point
@@ -297,7 +297,7 @@ const unsigned int *ncc_timeout_flag(const BmWork &w);
 mirorr_status ncc_give_up_flag(BmWork &w, cudaStream_t s, unsigned int **flag);
 // One fit of lts_batch_launch: its state (uploaded after lts_begin), point
 // pairs, the two device counters whose sum is the pair count, and scratch of
-// lts_fit_scratch_bytes(n_max, ncta) bytes (256-byte aligned).
+// lts_fit_scratch_bytes(n_max) bytes (256-byte aligned).
 struct LtsFit {
   LtsState *state;
   const double *init;
@@ -305,14 +305,14 @@ struct LtsFit {
   const long long *n_dev;
   void *scratch;
 };
-size_t lts_fit_scratch_bytes(long long n_max, int ncta);
+size_t lts_fit_scratch_bytes(long long n_max);
 // Bytes of one fit's launch arguments (lts_batch_launch's staging).
 size_t lts_args_bytes();
-// Runs nfits LTS fits in one cooperative launch, ncta CTAs each (every CTA of
-// the launch resident at once); zeroes each fit's barrier and histograms
-// first.  args_dev / args_host: argument staging reused across calls.
-mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, int ncta, long long spin_limit,
-                               DevBuf &args_dev, HostBuf &args_host, cudaStream_t st);
+// Runs nfits LTS fits in one launch, a thread-block cluster each; zeroes each
+// fit's control and histograms first.  args_dev / args_host: argument staging
+// reused across calls.
+mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, DevBuf &args_dev,
+                               HostBuf &args_host, cudaStream_t st);
 // The device word of a fit's scratch that is non-zero when one of its
 // barrier waits gave up.
 const int *lts_fit_error_flag(const void *scratch);

@@ -1,20 +1,29 @@
 // lts.cu -- the least-trimmed-squares fit on the device.
 //
-// One cooperative launch runs the whole inner loop of OptimizeTransform
-// (classic: itkMirorrRegistrationMethod.txx:785-999; symmetric:
+// One launch runs the whole inner loop of OptimizeTransform (classic:
+// itkMirorrRegistrationMethod.txx:785-999; symmetric:
 // itkSymMirorrRegistrationMethod.txx:771-1442).  Per inner iteration:
 //   residuals r_i (FP64) under the current final transform(s);
 //   the threshold r_nth: the maximum on the first iteration, otherwise the
-//     exact value of rank min(floor(f N), N-1) by an MSD radix select on the
-//     residual bit patterns (grid-wide histograms until at most one CTA's
-//     worth of keys share the prefix, then those keys ranked by counting);
+//     exact value of rank min(floor(f N), N-1) by a radix select on the
+//     residual bit patterns (histograms over narrowing key ranges until at
+//     most one CTA's worth of keys is left, then those keys ranked by counting);
 //   subset {r_i <= r_nth}: count, first and second moments of the
 //     (initial, moved) pairs about the first pair in one sweep, reduced per
 //     CTA and summed in a fixed order (deterministic), then centred;
 //   the FP64 solve (affine normal equations / Horn quaternion, symmetric
-//     half-space algebra) in one thread, and the loop test.
-// CTAs meet at a software grid barrier whose wait is bounded (about one
-// second); a timeout raises an error flag and every CTA returns.
+//     half-space algebra) in one warp, and the loop test.
+//
+// What bounds it is latency: a fit is some 2 to 60 dependent iterations of
+// barriers, short passes over a few thousand to a few hundred thousand pairs
+// and a serial solve.  So the CTAs of a fit of at most kClusterPairs pairs are
+// one thread-block cluster, which meets at the hardware cluster barrier, and a
+// batch runs one such cluster per fit; a larger fit spreads over a CTA per SM,
+// which meet at a software grid barrier whose wait is bounded (about one
+// second; a timeout raises an error flag and every CTA returns).  Per inner
+// iteration of a rigid fit: 84K cycles with a software barrier over 2 to 16
+// CTAs and the matrices of the solve in local memory, 39K now at 7,300 pairs;
+// of a symmetric affine one at 590,000 pairs 150K, now 81K.
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -26,19 +35,30 @@ namespace mb2 {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kBins = 4096;
+constexpr int kThreads = 512;
+constexpr int kWarps = kThreads / 32;
+constexpr int kBins = 2048;
 constexpr int kCandMax = kThreads;  // keys left for the final rank (one per thread)
+constexpr int kRankMax = 96;  // keys ranked by counting without a further histogram
+constexpr int kUnroll = 2;   // pairs a thread has in flight
 constexpr int kPartial = 32;  // doubles per CTA partial
+constexpr int kSums = 28;     // count, 6 first and 21 second moments
+constexpr int kClusterCtas = 8;  // CTAs of a cluster (the portable limit)
+// Pairs up to which one cluster is faster than a CTA per SM: an iteration
+// (rigid) takes 28K + 1.2 n cycles on a cluster (39K at 7,500 pairs, 59K at
+// 25,600, 67K at 47,500) and about 46K on the whole GPU.
+constexpr long long kClusterPairs = 16384;
+// The first histogram's keys: 64 bins per octave over [2^-12, 2^20) mm^2 (a
+// residual's bit pattern above kKeyLo in steps of 2^46), one bin below and one
+// above.
+constexpr unsigned long long kKeyLo = (1023ULL - 12ULL) << 52;
+constexpr int kKeyShift = 46;
 // Polls of a grid-barrier wait (about 0.84 s with the 100 ns back-off) before
 // the wait gives up, raises the error flag and every CTA returns.
 constexpr long long kDefaultSpinLimit = 1LL << 23;
 
 struct LtsCtl {
-  unsigned int bar_count;
-  unsigned int bar_gen;
-  int err;
-  int pad;
+  GridBar bar;
   unsigned long long maxkey;
   unsigned long long ncand;
 };
@@ -49,16 +69,30 @@ struct LtsArgs {
   const double *moved;
   const long long *n_dev;
   double *resid;
-  double *partial;        // gridDim.x * kPartial
+  double *partial;        // kPartial per CTA: sum q of CTA b at q * CTAs + b
   unsigned int *hist;     // 3 * kBins
   unsigned long long *cand;
   LtsCtl *ctl;
   long long spin_limit;   // polls of a grid-barrier wait before it gives up
 };
 
-__device__ inline bool grid_sync(LtsCtl *ctl, long long spin_limit, unsigned int nctas) {
-  return grid_barrier(&ctl->bar_count, &ctl->bar_gen, &ctl->err, spin_limit, nctas);
-}
+// How the CTAs of a fit meet.  A cluster's barrier orders their global writes
+// at cluster scope and cannot time out (its CTAs are resident together and
+// none leaves early).
+struct GridSync {
+  LtsCtl *ctl;
+  long long spin_limit;
+  unsigned int nctas;
+  unsigned int round;
+  __device__ bool operator()() { return grid_barrier(&ctl->bar, round++, spin_limit, nctas); }
+};
+struct ClusterSync {
+  __device__ bool operator()() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::
+                     : "memory");
+    return true;
+  }
+};
 
 __device__ inline void load_cg(void *dst, const void *src, int bytes) {
   const unsigned long long *s = static_cast<const unsigned long long *>(src);
@@ -66,39 +100,66 @@ __device__ inline void load_cg(void *dst, const void *src, int bytes) {
   for (int i = threadIdx.x; i < bytes / 8; i += blockDim.x) d[i] = __ldcg(s + i);
 }
 
-// Sums each of v[0, N) over the CTA (per value: shuffle tree within each
-// warp, then the warps in order); out[q] in shared memory, valid for every
-// thread on return.
-template <int N>
-__device__ inline void block_sums(const double (&v)[N], double *red /* N * 32 */, double *out) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Sums each of v[0, kSums) over the CTA; out[q] in shared memory, valid for
+// every thread on return.  Within a warp the values are summed by halving:
+// at distance 16 a lane sends the half of its values that its partner keeps
+// and adds what it gets, then 8, 4, 2, 1, after which lane l holds value l:
+// 31 exchanges instead of the 140 of a shuffle tree per value (the shuffle
+// unit was the bound).  Then the warps in order.
+__device__ inline void block_sums(const double (&v)[kSums], double (*red)[kWarps], double *out) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double x[32];
 #pragma unroll
-  for (int q = 0; q < N; ++q) {
-    double x = v[q];
-    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-    if (lane == 0) red[q * 32 + wid] = x;
+  for (int q = 0; q < 32; ++q) x[q] = q < kSums ? v[q] : 0.0;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const bool up = (lane & d) != 0;
+#pragma unroll
+    for (int q = 0; q < d; ++q) {
+      const double send = up ? x[q] : x[q + d];
+      const double keep = up ? x[q + d] : x[q];
+      x[q] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+    }
   }
+  red[lane][wid] = x[0];
   __syncthreads();
-  if (threadIdx.x < N) {
+  if (threadIdx.x < kSums) {
     double r = 0.0;
-    for (int w = 0; w < nw; ++w) r += red[threadIdx.x * 32 + w];
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) r += red[threadIdx.x][w];
     out[threadIdx.x] = r;
   }
   __syncthreads();
 }
 
-// out[q] = sum over the grid's CTAs b of part[b * kPartial + q0 + q], q < nq:
-// warp q % nwarps takes value q, its lanes stride over b, then a shuffle tree
-// (a fixed order).  out in shared memory, valid for every thread on return.
-__device__ inline void grid_partial_sums(const double *part, int q0, int nq, double *out,
-                                         int nctas) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int q = wid; q < nq; q += nw) {
-    double x = 0.0;
-    for (int b = lane; b < nctas; b += 32) x += __ldcg(&part[(long long)b * kPartial + q0 + q]);
-    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-    if (lane == 0) out[q] = x;
+// out[q] = sum over the fit's CTAs b of part[q * nctas + b], q < kSums: warp
+// q % kWarps takes value q, its lanes stride over b, then a shuffle tree (a
+// fixed order).  out in shared memory, valid for every thread on return.
+__device__ inline void grid_partial_sums(const double *part, double *out, int nctas) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  constexpr int NQ = (kSums + kWarps - 1) / kWarps;
+  double x[NQ];
+#pragma unroll
+  for (int j = 0; j < NQ; ++j) x[j] = 0.0;
+  for (int b0 = lane; b0 < nctas; b0 += 4 * 32) {
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      const int q = wid + j * kWarps;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int b = b0 + 32 * u;
+        if (q < kSums && b < nctas) x[j] += __ldcg(&part[(long long)q * nctas + b]);
+      }
+    }
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) x[j] += __shfl_down_sync(0xffffffffu, x[j], off);
+  if (lane == 0)
+#pragma unroll
+    for (int j = 0; j < NQ; ++j)
+      if (wid + j * kWarps < kSums) out[wid + j * kWarps] = x[j];
   __syncthreads();
 }
 
@@ -118,41 +179,146 @@ __device__ inline double residual(const LtsState &s, const double *x, const doub
   return r;
 }
 
-// The LTS loop run by `ncta` CTAs (index `cta` among them) that meet at the
-// bounded grid barrier of a.ctl.
-__device__ void lts_body(const LtsArgs &a, int cta, int ncta) {
+// Bin of a key in the first histogram (see kKeyLo), and the keys [lo, hi] of a
+// bin.
+__device__ inline unsigned int first_bin(unsigned long long key) {
+  if (key < kKeyLo) return 0;
+  const unsigned long long b = (key - kKeyLo) >> kKeyShift;
+  return b < (unsigned long long)(kBins - 2) ? (unsigned int)b + 1u : (unsigned int)(kBins - 1);
+}
+__device__ inline void first_range(int bin, unsigned long long &lo, unsigned long long &hi) {
+  if (bin == 0) {
+    lo = 0;
+    hi = kKeyLo - 1;
+  } else {
+    lo = kKeyLo + ((unsigned long long)(bin - 1) << kKeyShift);
+    hi = bin == kBins - 1 ? ~0ULL : lo + ((1ULL << kKeyShift) - 1);
+  }
+}
+
+// What the solve needs of the subset (shared memory).
+struct Subset {
+  double mean[6];  // barycentres of the initial and the moved points
+  double Z[36];    // second moments about them
+  double zn[36];   // Z divided by the subset's size
+};
+
+__device__ inline double other_half(double v) { return __shfl_xor_sync(0xffffffffu, v, 4); }
+
+// The solve, by one whole warp.  Every lane runs it: the lanes of a quad hold
+// the same values (each takes one of three angles where trigonometric
+// functions come in threes), and in the symmetric fit odd quads hold the
+// backward half and even quads the forward one.  Lane 0 (and lane 4) write s.
+__device__ __noinline__ void solve_classic(LtsState &s, const Subset &m) {
+  Tfm T = s.fin;
+  double np[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) np[i] = 0.0;
+  classic_fit(T, m.mean, m.mean + 3, m.Z, m.zn, np);
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    s.fin = T;
+    lts_delta(s, np);
+  }
+}
+
+__device__ __noinline__ void solve_symmetric(LtsState &s, const Subset &m) {
+  const int lane = threadIdx.x & 31, h = (lane >> 2) & 1;
+  Tfm T = h ? s.finb : s.fin, iT;
+  double np[12], inv[9], K[9], ot[3], m12[16];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) np[i] = 0.0;
+  sym_fit(T, h, m.mean, m.mean + 3, m.Z, m.zn, np, inv);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    K[i] = (T.M[i] + other_half(inv[i])) / 2.0;
+    const double o = other_half(K[i]);
+    if (T.kind == KIND_RIGID && h) K[i] = o;  // both halves take the forward mean
+  }
+  // (a backward half is left alone when the forward one rejects its matrix)
+  const Tfm T0 = T;
+  const bool took = sym_mean(T, h, K);
+  __syncwarp();
+  const unsigned ok = __ballot_sync(0xffffffffu, took);
+  if (h && !(ok & 1u)) T = T0;
+  sym_to_origin(T, iT);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 9; ++i) K[i] = other_half(iT.M[i]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) ot[i] = other_half(iT.t[i]);
+  sym_half(T, K, ot, m12);
+  __syncwarp();
+  const Tfm T1 = T;
+  const bool fin = sym_finish(T, m12, false);
+  __syncwarp();
+  if (!__all_sync(0xffffffffu, fin)) {
+    T = T1;
+    sym_finish(T, m12, true);
+  }
+  const double tr[3] = {m12[3], m12[7], m12[11]};
+  tfm_set_translation(T, tr);
+  __syncwarp();
+  if (lane == 0) {
+    s.fin = T;
+    if ((ok & 0x11u) != 0x11u) s.failed = 1;
+    lts_delta(s, np);
+  } else if (lane == 4) {
+    s.finb = T;
+  }
+  __syncwarp();
+}
+
+// The LTS loop run by `ncta` CTAs (index `cta` among them) that meet at `sync`.
+template <class Sync>
+__device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
   __shared__ __align__(16) LtsState s;
   __shared__ unsigned int h[kBins];
   __shared__ unsigned long long ck[kCandMax];
-  __shared__ double red_n[28 * 32];
+  __shared__ double red[32][kWarps];
+  __shared__ double s_out[kSums];
+  __shared__ Subset sub;
   __shared__ double s_nth;
   __shared__ unsigned long long s_key;
   __shared__ unsigned long long s_pair[2];
   const long long n = __ldcg(&a.n_dev[0]) + __ldcg(&a.n_dev[1]);
-  const long long gstride = (long long)ncta * blockDim.x;
-  const long long gtid = (long long)cta * blockDim.x + threadIdx.x;
+  const long long gstride = (long long)ncta * kThreads;
+  const long long gtid = (long long)cta * kThreads + threadIdx.x;
 
   for (int guard = 0; guard < 200; ++guard) {
     load_cg(&s, a.state, sizeof(LtsState));
+    for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
+    if (cta == 0)
+      for (int i = threadIdx.x; i < kBins; i += kThreads) a.hist[kBins + i] = 0;  // next pass's
     __syncthreads();
     if (!s.running || n <= 0) break;
     const bool first = s.fraction > 0.99999;
     // ---- residuals (+ max or first histogram) ----------------------------
-    for (int i = threadIdx.x; i < kBins; i += blockDim.x) h[i] = 0;
-    if (cta == 0)
-      for (int i = threadIdx.x; i < kBins; i += blockDim.x) {
-        a.hist[kBins + i] = 0;  // next two passes' buffers
-      }
-    __syncthreads();
     unsigned long long kmax = 0;
-    for (long long i = gtid; i < n; i += gstride) {
-      double r = residual(s, a.init + 3 * i, a.moved + 3 * i);
-      a.resid[i] = r;
-      unsigned long long key = (unsigned long long)__double_as_longlong(r);
-      if (first) {
-        if (key > kmax) kmax = key;
-      } else {
-        hist_add(h, (unsigned)(key >> 52) & (kBins - 1));
+    for (long long i0 = gtid; i0 < n; i0 += kUnroll * gstride) {
+      // kUnroll pairs' loads are issued before the first is used
+      double x[kUnroll][3], y[kUnroll][3];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const long long i = i0 + u * gstride < n ? i0 + u * gstride : i0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          x[u][c] = __ldcg(&a.init[3 * i + c]);
+          y[u][c] = __ldcg(&a.moved[3 * i + c]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        if (i0 + u * gstride >= n) break;
+        const double r = residual(s, x[u], y[u]);
+        a.resid[i0 + u * gstride] = r;
+        const unsigned long long key = (unsigned long long)__double_as_longlong(r);
+        if (first) {
+          if (key > kmax) kmax = key;
+        } else {
+          hist_add(h, first_bin(key));
+        }
       }
     }
     if (first) {
@@ -163,87 +329,113 @@ __device__ void lts_body(const LtsArgs &a, int cta, int ncta) {
       if ((threadIdx.x & 31) == 0 && kmax) atomicMax(&a.ctl->maxkey, kmax);
     } else {
       __syncthreads();
-      for (int i = threadIdx.x; i < kBins; i += blockDim.x)
+      for (int i = threadIdx.x; i < kBins; i += kThreads)
         if (h[i]) atomicAdd(&a.hist[i], h[i]);
     }
-    if (!grid_sync(a.ctl, a.spin_limit, (unsigned)ncta)) return;
+    if (!sync()) return;
     double nth;
     if (first) {
       if (threadIdx.x == 0) s_key = __ldcg(&a.ctl->maxkey);
       __syncthreads();
       nth = __longlong_as_double((long long)s_key);
     } else {
-      // ---- radix select of rank k -----------------------------------------
+      // ---- radix select of rank k ------------------------------------------
       unsigned long long k = (unsigned long long)(unsigned int)(s.fraction * (double)n);
       if (k > (unsigned long long)(n - 1)) k = n - 1;
-      unsigned long long prefix = 0, mask = 0;
-      int shift = 52, bits = 12, pass = 0;
-      unsigned long long bucket = 0;
+      unsigned long long lo = 0, hi = 0;  // the keys left lie in [lo, hi]
+      int shift = 0, pass = 0;
       while (true) {
         // every CTA scans the global histogram of this pass identically
         const unsigned int *gh = a.hist + (pass % 3) * kBins;
         __syncthreads();
-        for (int i = threadIdx.x; i < kBins; i += blockDim.x) h[i] = __ldcg(&gh[i]);
+        for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = __ldcg(&gh[i]);
         __syncthreads();
         int d = 0;
         unsigned long long cum = 0;
-        find_bucket<kBins, kThreads>(h, k, 1 << bits, s_pair, &d, &cum);
-        bucket = h[d];
+        find_bucket<kBins, kThreads>(h, k, kBins, s_pair, &d, &cum);
+        const unsigned long long bucket = h[d];
         k -= cum;
-        prefix |= (unsigned long long)d << shift;
-        mask |= ((1ULL << bits) - 1ULL) << shift;
+        if (pass == 0) {
+          first_range(d, lo, hi);
+        } else {
+          const unsigned long long top = hi;
+          lo += (unsigned long long)d << shift;
+          hi = lo + ((1ULL << shift) - 1);
+          if (hi > top) hi = top;
+        }
         __syncthreads();
-        if (bucket <= (unsigned long long)kCandMax || shift == 0) break;
-        // more than one CTA's worth of keys share the prefix: refine it
-        // next pass
+        if (bucket <= (unsigned long long)kCandMax || lo == hi) break;
+        // more than one CTA's worth of keys is left: the next histogram, of
+        // [lo, hi] in kBins steps
         ++pass;
-        bits = shift >= 12 ? 12 : shift;
-        shift -= bits;
+        shift = 0;
+        while (((hi - lo) >> shift) >= (unsigned long long)kBins) ++shift;
         if (cta == 0) {
           unsigned int *zb = a.hist + ((pass + 1) % 3) * kBins;
-          for (int i = threadIdx.x; i < kBins; i += blockDim.x) zb[i] = 0;
+          for (int i = threadIdx.x; i < kBins; i += kThreads) zb[i] = 0;
         }
-        for (int i = threadIdx.x; i < kBins; i += blockDim.x) h[i] = 0;
+        for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
         __syncthreads();
         for (long long i = gtid; i < n; i += gstride) {
-          unsigned long long key = (unsigned long long)__double_as_longlong(a.resid[i]);
-          if ((key & mask) == prefix) hist_add(h, (unsigned)(key >> shift) & ((1u << bits) - 1u));
+          const unsigned long long key = (unsigned long long)__double_as_longlong(a.resid[i]);
+          if (key >= lo && key <= hi) hist_add(h, (unsigned int)((key - lo) >> shift));
         }
         __syncthreads();
         unsigned int *gh2 = a.hist + (pass % 3) * kBins;
-        for (int i = threadIdx.x; i < kBins; i += blockDim.x)
+        for (int i = threadIdx.x; i < kBins; i += kThreads)
           if (h[i]) atomicAdd(&gh2[i], h[i]);
-        if (!grid_sync(a.ctl, a.spin_limit, (unsigned)ncta)) return;
+        if (!sync()) return;
       }
-      if (shift == 0) {
-        // every bit fixed: the bucket's keys all equal the prefix
-        nth = __longlong_as_double((long long)prefix);
+      if (lo == hi) {
+        nth = __longlong_as_double((long long)lo);  // the keys left are equal
       } else {
-        // ---- gather the bucket's keys (at most one per thread) and rank them
+        // ---- gather the keys left (at most one per thread) and rank them
         for (long long i = gtid; i < n; i += gstride) {
-          unsigned long long key = (unsigned long long)__double_as_longlong(a.resid[i]);
-          if ((key & mask) == prefix) {
-            unsigned long long pos = atomicAdd(&a.ctl->ncand, 1ULL);
+          const unsigned long long key = (unsigned long long)__double_as_longlong(a.resid[i]);
+          if (key >= lo && key <= hi) {
+            const unsigned long long pos = atomicAdd(&a.ctl->ncand, 1ULL);
             if (pos < (unsigned long long)kCandMax) a.cand[pos] = key;
           }
         }
-        if (!grid_sync(a.ctl, a.spin_limit, (unsigned)ncta)) return;
+        if (!sync()) return;
         if (threadIdx.x == 0) s_key = __ldcg(&a.ctl->ncand);
+        unsigned long long mine = __ldcg(&a.cand[threadIdx.x]);
         __syncthreads();
-        const int nc = (int)(s_key < (unsigned long long)kCandMax ? s_key : kCandMax);
-        const unsigned long long kk = k < (unsigned long long)nc ? k : (nc > 0 ? nc - 1 : 0);
+        int nc = (int)(s_key < (unsigned long long)kCandMax ? s_key : kCandMax);
+        bool have = threadIdx.x < nc;
+        unsigned long long kk = k < (unsigned long long)nc ? k : (nc > 0 ? nc - 1 : 0);
+        if (nc > kRankMax) {
+          // one more histogram, of this CTA alone, so that few keys are ranked
+          shift = 0;
+          while (((hi - lo) >> shift) >= (unsigned long long)kBins) ++shift;
+          for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
+          __syncthreads();
+          if (have) atomicAdd(&h[(mine - lo) >> shift], 1u);
+          __syncthreads();
+          int d = 0;
+          unsigned long long cum = 0;
+          find_bucket<kBins, kThreads>(h, kk, kBins, s_pair, &d, &cum);
+          kk -= cum;
+          nc = (int)h[d];
+          have = have && (int)((mine - lo) >> shift) == d;
+          if (threadIdx.x == 0) s_pair[0] = 0;
+          __syncthreads();
+          if (have) ck[atomicAdd(&s_pair[0], 1ULL)] = mine;
+        } else if (have) {
+          ck[threadIdx.x] = mine;
+        }
+        __syncthreads();
         // rank by counting: key i has rank kk iff lo_i <= kk < lo_i + eq_i
-        for (int i = threadIdx.x; i < nc; i += blockDim.x) ck[i] = __ldcg(&a.cand[i]);
-        __syncthreads();
-        if (threadIdx.x < nc) {
-          const unsigned long long v = ck[threadIdx.x];
-          int lo = 0, eq = 0;
+        if (have) {
+          const unsigned long long v = mine;
+          int below = 0, eq = 0;
+#pragma unroll 8
           for (int j = 0; j < nc; ++j) {
             const unsigned long long u = ck[j];
-            lo += u < v;
+            below += u < v;
             eq += u == v;
           }
-          if ((unsigned long long)lo <= kk && kk < (unsigned long long)(lo + eq))
+          if ((unsigned long long)below <= kk && kk < (unsigned long long)(below + eq))
             s_nth = __longlong_as_double((long long)v);
         }
         __syncthreads();
@@ -258,87 +450,104 @@ __device__ void lts_body(const LtsArgs &a, int cta, int ncta) {
       z0[c] = __ldg(&a.init[c]);
       z0[3 + c] = __ldg(&a.moved[c]);
     }
-    double acc[28];
+    double acc[kSums];
 #pragma unroll
-    for (int q = 0; q < 28; ++q) acc[q] = 0.0;
-    for (long long i = gtid; i < n; i += gstride) {
-      if (a.resid[i] <= nth) {
-        double z[6];
+    for (int q = 0; q < kSums; ++q) acc[q] = 0.0;
+    for (long long i0 = gtid; i0 < n; i0 += kUnroll * gstride) {
+      double z[kUnroll][6], r[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const long long i = i0 + u * gstride < n ? i0 + u * gstride : i0;
+        r[u] = a.resid[i];
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-          z[c] = a.init[3 * i + c] - z0[c];
-          z[3 + c] = a.moved[3 * i + c] - z0[3 + c];
+          z[u][c] = __ldcg(&a.init[3 * i + c]);
+          z[u][3 + c] = __ldcg(&a.moved[3 * i + c]);
         }
-        acc[0] += 1.0;
+      }
 #pragma unroll
-        for (int r = 0; r < 6; ++r) acc[1 + r] += z[r];
-        int q = 7;
+      for (int u = 0; u < kUnroll; ++u) {
+        if (i0 + u * gstride < n && r[u] <= nth) {
 #pragma unroll
-        for (int r = 0; r < 6; ++r)
+          for (int c = 0; c < 6; ++c) z[u][c] -= z0[c];
+          acc[0] += 1.0;
 #pragma unroll
-          for (int c = r; c < 6; ++c) acc[q++] += z[r] * z[c];
+          for (int p = 0; p < 6; ++p) acc[1 + p] += z[u][p];
+          int q = 7;
+#pragma unroll
+          for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int c = p; c < 6; ++c) acc[q++] += z[u][p] * z[u][c];
+        }
       }
     }
-    __shared__ double s_out[28];
-    block_sums<28>(acc, red_n, s_out);
-    if (threadIdx.x < 28) a.partial[(long long)cta * kPartial + threadIdx.x] = s_out[threadIdx.x];
-    if (!grid_sync(a.ctl, a.spin_limit, (unsigned)ncta)) return;
-    if (cta == 0) grid_partial_sums(a.partial, 0, 28, s_out, ncta);
-    // the solve: warp 0 of CTA 0; the symmetric fit's two square roots run
-    // on lanes 0 and 1 at once
-    __shared__ SymHalf s_half;
-    __shared__ double s_root[2][16];
-    if (cta == 0 && threadIdx.x < 32) {
-      if (threadIdx.x == 0) {
-        LtsMoments mo;
-        const double cnt = s_out[0];
-        double m[6];
-        for (int r = 0; r < 6; ++r) m[r] = s_out[1 + r] / cnt;
-        mo.n = cnt;
-        for (int c = 0; c < 3; ++c) { mo.mean_i[c] = z0[c] + m[c]; mo.mean_m[c] = z0[3 + c] + m[3 + c]; }
-        int q = 7;
-        for (int r = 0; r < 6; ++r)
-          for (int c = r; c < 6; ++c) {
-            const double zz = s_out[q++] - cnt * m[r] * m[c];
-            mo.Z[6 * r + c] = zz;
-            mo.Z[6 * c + r] = zz;
-          }
-        if (s.symmetric) lts_symmetric_pre(s, mo, s_half);
-        else lts_classic_step(s, mo);
-      }
-      __syncwarp();
-      if (s.symmetric && threadIdx.x < 2)
-        half_step(s_half.K[threadIdx.x], s_half.t[threadIdx.x], s_root[threadIdx.x]);
-      __syncwarp();
-      if (threadIdx.x == 0) {
-        if (s.symmetric) lts_symmetric_post(s, s_half, s_root[0], s_root[1]);
-        s.fraction = s.lts_keep;
-        s.iter += 1;
-        s.running = lts_continue(s) ? 1 : 0;
-        if (s.iter > 101) s.running = 0;
-        // reset select scratch for the next iteration
-        a.ctl->maxkey = 0;
-        a.ctl->ncand = 0;
-        *a.state = s;
-        __threadfence();
-      }
-    }
+    block_sums(acc, red, s_out);
+    if (threadIdx.x < kSums) a.partial[(long long)threadIdx.x * ncta + cta] = s_out[threadIdx.x];
+    if (!sync()) return;
     if (cta == 0) {
-      __syncthreads();
-      for (int i = threadIdx.x; i < kBins; i += blockDim.x) a.hist[i] = 0;
+      grid_partial_sums(a.partial, s_out, ncta);
+      if (threadIdx.x < 32) {
+        const int l = threadIdx.x;
+        const double cnt = s_out[0];
+        // the moments about the barycentres, entry (r, c) of the upper
+        // triangle by lane q
+        double zz = 0.0;
+        int r = 0, c = 0;
+        if (l < 21) {
+          int q = l;
+          while (q >= 6 - r) { q -= 6 - r; ++r; }
+          c = r + q;
+          zz = s_out[7 + l] - cnt * (s_out[1 + r] / cnt) * (s_out[1 + c] / cnt);
+          sub.Z[6 * r + c] = zz;
+          sub.Z[6 * c + r] = zz;
+          zz /= cnt;
+          sub.zn[6 * r + c] = zz;
+          sub.zn[6 * c + r] = zz;
+        } else if (l < 27) {
+          sub.mean[l - 21] =
+              (l < 24 ? __ldg(&a.init[l - 21]) : __ldg(&a.moved[l - 24])) + s_out[1 + l - 21] / cnt;
+        }
+        __syncwarp();
+        if (s.symmetric) solve_symmetric(s, sub);
+        else solve_classic(s, sub);
+        __syncwarp();
+        if (l == 0) {
+          s.fraction = s.lts_keep;
+          s.iter += 1;
+          s.running = lts_continue(s) ? 1 : 0;
+          if (s.iter > 101) s.running = 0;
+          // reset select scratch for the next iteration
+          a.ctl->maxkey = 0;
+          a.ctl->ncand = 0;
+        }
+        __syncwarp();
+        const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&s);
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(a.state);
+        for (int i = l; i < (int)(sizeof(LtsState) / 8); i += 32) dst[i] = src[i];
+      } else {
+        for (int i = threadIdx.x - 32; i < kBins; i += kThreads - 32) a.hist[i] = 0;
+      }
     }
-    if (!grid_sync(a.ctl, a.spin_limit, (unsigned)ncta)) return;
+    if (!sync()) return;
   }
 }
 
 __global__ void __launch_bounds__(kThreads) lts_kernel(LtsArgs a) {
-  lts_body(a, blockIdx.x, gridDim.x);
+  lts_body(a, GridSync{a.ctl, a.spin_limit, gridDim.x, 0u}, blockIdx.x, gridDim.x);
 }
 
-// Several independent fits in one cooperative launch: fit f runs on CTAs
-// [f ncta, (f + 1) ncta) with its own arguments and barrier.
-__global__ void __launch_bounds__(kThreads) lts_batch_kernel(const LtsArgs *args, int ncta) {
-  const LtsArgs a = args[blockIdx.x / ncta];
-  lts_body(a, blockIdx.x % ncta, ncta);
+// One fit by one cluster.
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
+    lts_cluster_kernel(LtsArgs a) {
+  lts_body(a, ClusterSync{}, blockIdx.x, kClusterCtas);
+}
+
+// Several independent fits in one launch, a cluster each: fit f runs on CTAs
+// [f kClusterCtas, (f + 1) kClusterCtas) with its own arguments.
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
+    lts_batch_kernel(const LtsArgs *args) {
+  const LtsArgs a = args[blockIdx.x / kClusterCtas];
+  lts_body(a, ClusterSync{}, blockIdx.x % kClusterCtas, kClusterCtas);
 }
 
 // Zeroes each fit's barrier, select control and histograms (CTA f: fit f) so
@@ -346,6 +555,26 @@ __global__ void __launch_bounds__(kThreads) lts_batch_kernel(const LtsArgs *args
 __global__ void lts_batch_zero_kernel(const LtsArgs *args, unsigned long long words) {
   uint4 *p = reinterpret_cast<uint4 *>(args[blockIdx.x].ctl);
   for (unsigned long long i = threadIdx.x; i < words; i += blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// CTAs of a fit of at most n pairs: one cluster, or up to max_ctas that meet at
+// the grid barrier (two pairs a thread).
+int fit_ctas(long long n, int max_ctas) {
+  if (n <= kClusterPairs) return kClusterCtas;
+  const long long want = (n + 2 * kThreads - 1) / (2 * kThreads);
+  return (int)(want < max_ctas ? want : max_ctas);
+}
+
+mirorr_status launch_fit(LtsArgs &a, long long n, int ctas, cudaStream_t st) {
+  if (n <= kClusterPairs) {
+    lts_cluster_kernel<<<kClusterCtas, kThreads, 0, st>>>(a);
+    MB2_LAUNCH_CHECK();
+    return MIRORR_OK;
+  }
+  void *args[] = {&a};
+  MB2_CUDA_TRY(cudaLaunchCooperativeKernel((void *)lts_kernel, dim3(ctas), dim3(kThreads), args, 0, st));
+  ++g_launches;
+  return MIRORR_OK;
 }
 
 }  // namespace
@@ -398,8 +627,7 @@ mirorr_status lts_issue(LtsWork &w, const LtsState *state_in, const double *init
     }
     w.max_ctas = sms * (per > 1 ? 1 : per);
   }
-  long long want = (n + 4 * kThreads - 1) / (4 * kThreads);
-  int grid = (int)(want < 1 ? 1 : (want > w.max_ctas ? w.max_ctas : want));
+  const int grid = fit_ctas(n, w.max_ctas);
   MB2_TRY(w.state.ensure(sizeof(LtsState)));
   MB2_TRY(w.resid.ensure(sizeof(double) * n));
   MB2_TRY(w.partial.ensure(sizeof(double) * kPartial * (size_t)grid));
@@ -425,9 +653,7 @@ mirorr_status lts_issue(LtsWork &w, const LtsState *state_in, const double *init
   a.cand = w.cand.as<unsigned long long>();
   a.ctl = w.ctrl.as<LtsCtl>();
   a.spin_limit = w.spin_limit > 0 ? w.spin_limit : kDefaultSpinLimit;
-  void *args[] = {&a};
-  MB2_CUDA_TRY(cudaLaunchCooperativeKernel((void *)lts_kernel, dim3(grid), dim3(kThreads), args, 0, st));
-  ++g_launches;
+  MB2_TRY(launch_fit(a, n, grid, st));
   MB2_CUDA_TRY(cudaMemcpyAsync(&o->state, w.state.ptr, sizeof(LtsState), cudaMemcpyDeviceToHost, st));
   MB2_CUDA_TRY(cudaMemcpyAsync(&o->ctl, w.ctrl.ptr, sizeof(LtsCtl), cudaMemcpyDeviceToHost, st));
   MB2_CUDA_TRY(cudaMemcpyAsync(o->n, n_dev, sizeof(o->n), cudaMemcpyDeviceToHost, st));
@@ -444,7 +670,7 @@ mirorr_status lts_collect(LtsWork &w, const void *out_host, LtsState &hs, int *i
   hs = o->state;
   if (watch_host) *watch_host = o->watch;
   if (n_used) *n_used = o->n[0] + o->n[1];
-  if (o->ctl.err) {
+  if (o->ctl.bar.err) {
     set_error("LTS grid barrier timed out");
     return MIRORR_ETIMEOUT;
   }
@@ -453,34 +679,26 @@ mirorr_status lts_collect(LtsWork &w, const void *out_host, LtsState &hs, int *i
   return MIRORR_OK;
 }
 
-// ---- many fits in one cooperative launch ----------------------------------------
+// ---- many fits in one launch ----------------------------------------------------
 //
-// Fit f's CTAs meet at their own barrier (its LtsCtl); each fit has its own
-// state, counters and scratch (LtsFit, all device pointers).  The caller has
+// Each fit is one cluster with its own state, counters and scratch (LtsFit, all
+// device pointers); the fits need not be resident together.  The caller has
 // run lts_begin on every state it uploaded and runs lts_finish on each after
 // reading it back.  A fit whose state is not running returns at once.
 size_t lts_args_bytes() { return sizeof(LtsArgs); }
 
-size_t lts_fit_scratch_bytes(long long n_max, int ncta) {
+size_t lts_fit_scratch_bytes(long long n_max) {
   const size_t a = 256;
   auto up = [&](size_t v) { return (v + a - 1) / a * a; };
   return up(sizeof(LtsCtl)) + up(sizeof(unsigned int) * 3 * kBins) +
-         up(sizeof(unsigned long long) * kCandMax) + up(sizeof(double) * kPartial * (size_t)ncta) +
+         up(sizeof(unsigned long long) * kCandMax) +
+         up(sizeof(double) * kPartial * (size_t)kClusterCtas) +
          up(sizeof(double) * (size_t)(n_max > 0 ? n_max : 1));
 }
 
-mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, int ncta, long long spin_limit,
-                               DevBuf &args_dev, HostBuf &args_host, cudaStream_t st) {
+mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, DevBuf &args_dev,
+                               HostBuf &args_host, cudaStream_t st) {
   if (nfits <= 0) return MIRORR_OK;
-  int dev = 0, sms = 0, per = 0;
-  MB2_CUDA_TRY(cudaGetDevice(&dev));
-  MB2_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MB2_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lts_batch_kernel, kThreads, 0));
-  if ((long long)nfits * ncta > (long long)sms * per) {
-    set_error("%d fits of %d CTAs exceed the %d co-resident CTAs of the LTS kernel", nfits, ncta,
-              sms * per);
-    return MIRORR_EINVAL;
-  }
   MB2_TRY(args_dev.ensure(sizeof(LtsArgs) * nfits));
   MB2_TRY(args_host.ensure(sizeof(LtsArgs) * nfits));
   LtsArgs *ha = args_host.as<LtsArgs>();
@@ -500,9 +718,9 @@ mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, int ncta, long lon
     a.cand = reinterpret_cast<unsigned long long *>(p);
     p += up(sizeof(unsigned long long) * kCandMax);
     a.partial = reinterpret_cast<double *>(p);
-    p += up(sizeof(double) * kPartial * (size_t)ncta);
+    p += up(sizeof(double) * kPartial * (size_t)kClusterCtas);
     a.resid = reinterpret_cast<double *>(p);
-    a.spin_limit = spin_limit > 0 ? spin_limit : kDefaultSpinLimit;
+    a.spin_limit = kDefaultSpinLimit;
   }
   MB2_CUDA_TRY(cudaMemcpyAsync(args_dev.ptr, ha, sizeof(LtsArgs) * nfits, cudaMemcpyHostToDevice, st));
   const LtsArgs *dargs = args_dev.as<LtsArgs>();
@@ -511,17 +729,14 @@ mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, int ncta, long lon
   const size_t zbytes = up(sizeof(LtsCtl)) + up(sizeof(unsigned int) * 3 * kBins);
   lts_batch_zero_kernel<<<nfits, 256, 0, st>>>(dargs, (unsigned long long)(zbytes / 16));
   MB2_LAUNCH_CHECK();
-  ++g_launches;
-  void *kargs[] = {(void *)&dargs, (void *)&ncta};
-  MB2_CUDA_TRY(cudaLaunchCooperativeKernel((void *)lts_batch_kernel, dim3(nfits * ncta),
-                                           dim3(kThreads), kargs, 0, st));
-  ++g_launches;
+  lts_batch_kernel<<<nfits * kClusterCtas, kThreads, 0, st>>>(dargs);
+  MB2_LAUNCH_CHECK();
   return MIRORR_OK;
 }
 
 // Error flag of fit f's barrier (device word of its scratch).
 const int *lts_fit_error_flag(const void *scratch) {
-  return &static_cast<const LtsCtl *>(scratch)->err;
+  return &static_cast<const LtsCtl *>(scratch)->bar.err;
 }
 
 // ---- allocation-free variant ----------------------------------------------------
@@ -533,8 +748,8 @@ const int *lts_fit_error_flag(const void *scratch) {
 //   [0, 4096)        LtsState (uploaded each call)
 //   [4096, 4352)     LtsCtl (zeroed each call)
 //   [4352, 4608)     point-pair counters {n, 0} (uploaded each call)
-//   [4608, +48 KB)   3 radix histograms of 4096 bins (zeroed each call)
-//   then             256 candidate keys, kNaMaxCtas * 32 partial sums,
+//   [4608, +24 KB)   3 histograms of 2048 bins (zeroed each call)
+//   then             512 candidate keys, kNaMaxCtas * 32 partial sums,
 //                    MIRORR_LTS_NOALLOC_MAX_POINTS residuals.
 // Two calls in flight on one device share the array and race.
 
@@ -619,8 +834,7 @@ mirorr_status lts_run_noalloc(LtsState &hs, const double *init_dev, const double
   int max_ctas = 0;
   MB2_TRY(na_setup(dev, &base, &max_ctas));
   if (max_ctas > kNaMaxCtas) max_ctas = kNaMaxCtas;
-  long long want = (n + 4 * kThreads - 1) / (4 * kThreads);
-  int grid = (int)(want < 1 ? 1 : (want > max_ctas ? max_ctas : want));
+  const int grid = fit_ctas(n, max_ctas);
   long long counts[2] = {n, 0};
   MB2_CUDA_TRY(cudaMemcpyAsync(base + kNaState, &hs, sizeof(LtsState), cudaMemcpyHostToDevice, st));
   MB2_CUDA_TRY(cudaMemcpyAsync(base + kNaCount, counts, sizeof(counts), cudaMemcpyHostToDevice, st));
@@ -637,14 +851,12 @@ mirorr_status lts_run_noalloc(LtsState &hs, const double *init_dev, const double
   a.cand = reinterpret_cast<unsigned long long *>(base + kNaCand);
   a.ctl = reinterpret_cast<LtsCtl *>(base + kNaCtl);
   a.spin_limit = kDefaultSpinLimit;
-  void *args[] = {&a};
-  MB2_CUDA_TRY(cudaLaunchCooperativeKernel((void *)lts_kernel, dim3(grid), dim3(kThreads), args, 0, st));
-  ++g_launches;
+  MB2_TRY(launch_fit(a, n, grid, st));
   LtsCtl ctl;
   MB2_CUDA_TRY(cudaMemcpyAsync(&hs, base + kNaState, sizeof(LtsState), cudaMemcpyDeviceToHost, st));
   MB2_CUDA_TRY(cudaMemcpyAsync(&ctl, base + kNaCtl, sizeof(LtsCtl), cudaMemcpyDeviceToHost, st));
   MB2_CUDA_TRY(cudaStreamSynchronize(st));
-  if (ctl.err) {
+  if (ctl.bar.err) {
     set_error("LTS grid barrier timed out");
     return MIRORR_ETIMEOUT;
   }

@@ -19,10 +19,15 @@
 
 #include <math.h>
 
+// Every loop over matrix entries has constant bounds and is unrolled on the
+// device, and every index is a constant then, so the matrices live in
+// registers (an index known only at run time would put them into local memory).
 #ifdef __CUDACC__
 #define MB2_HD __host__ __device__ inline
+#define MB2_UNROLL _Pragma("unroll")
 #else
 #define MB2_HD inline
+#define MB2_UNROLL
 #endif
 
 namespace mb2 {
@@ -60,32 +65,48 @@ MB2_HD double m3_det(const double *a) {
 }
 
 // Gauss-Jordan inverse with partial pivoting; returns false when singular.
+// The pivot row is found by comparisons in row order and brought up by
+// selects on constant indices.
 template <int N>
 MB2_HD bool mn_inverse(const double *a, double *o) {
   double m[N][2 * N];
+  MB2_UNROLL
   for (int i = 0; i < N; ++i)
+    MB2_UNROLL
     for (int j = 0; j < N; ++j) {
       m[i][j] = a[N * i + j];
       m[i][N + j] = (i == j) ? 1.0 : 0.0;
     }
+  MB2_UNROLL
   for (int c = 0; c < N; ++c) {
     int p = c;
     double best = fabs(m[c][c]);
+    MB2_UNROLL
     for (int r = c + 1; r < N; ++r)
       if (fabs(m[r][c]) > best) { best = fabs(m[r][c]); p = r; }
     if (best == 0.0) return false;
-    if (p != c)
-      for (int j = 0; j < 2 * N; ++j) { double t = m[c][j]; m[c][j] = m[p][j]; m[p][j] = t; }
-    double inv = 1.0 / m[c][c];
+    MB2_UNROLL
+    for (int r = c + 1; r < N; ++r)
+      MB2_UNROLL
+      for (int j = 0; j < 2 * N; ++j) {
+        const double u = m[c][j], v = m[r][j];
+        m[c][j] = p == r ? v : u;
+        m[r][j] = p == r ? u : v;
+      }
+    const double inv = 1.0 / m[c][c];
+    MB2_UNROLL
     for (int j = 0; j < 2 * N; ++j) m[c][j] *= inv;
+    MB2_UNROLL
     for (int r = 0; r < N; ++r) {
       if (r == c) continue;
-      double f = m[r][c];
-      if (f != 0.0)
-        for (int j = 0; j < 2 * N; ++j) m[r][j] -= f * m[c][j];
+      const double f = m[r][c];
+      MB2_UNROLL
+      for (int j = 0; j < 2 * N; ++j) m[r][j] -= f * m[c][j];
     }
   }
+  MB2_UNROLL
   for (int i = 0; i < N; ++i)
+    MB2_UNROLL
     for (int j = 0; j < N; ++j) o[N * i + j] = m[i][N + j];
   return true;
 }
@@ -102,75 +123,145 @@ MB2_HD void mn_mul(const double *a, const double *b, double *o) {
   for (int i = 0; i < N * N; ++i) o[i] = r[i];
 }
 
-// Cyclic Jacobi eigen-decomposition of a symmetric NxN matrix.  On return
-// w[] holds eigenvalues in ascending order and column k of v is the
-// eigenvector of w[k].
+// 1 / sqrt(x) for x in [1e-36, 1e36]: on the device a single-precision seed
+// and two Newton steps y (3 - x y^2) / 2 (the seed's error of 2^-22 squares
+// twice), without the branches that would keep two of them from overlapping.
+MB2_HD double inv_sqrt(double x) {
+#ifdef __CUDA_ARCH__
+  double y = (double)rsqrtf((float)x);
+  const double hx = 0.5 * x;
+  MB2_UNROLL
+  for (int i = 0; i < 2; ++i) {
+    const double e = fma(-hx * y, y, 0.5);
+    y = fma(y, e, y);
+  }
+  return y;
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
+
+// One Jacobi rotation of the symmetric matrix a (upper triangle) in the plane
+// (P, Q), accumulated into the columns of v.
+template <int N, int P, int Q>
+MB2_HD void jacobi_rotate(double *a, double *v) {
+  const double apq = a[N * P + Q], app = a[N * P + P], aqq = a[N * Q + Q];
+  // with d = aqq - app and e = 2 apq the smaller angle has cos 2x = |d| r and
+  // |sin 2x| = |e| r, r = 1 / sqrt(d^2 + e^2); its sign is positive when d = 0
+  // or d and e agree.  c = sqrt((1 + cos 2x) / 2) and w = 1 / c, so a rotation
+  // is two reciprocal square roots and no division.
+  // An entry below 1e-18 (of a matrix scaled to a largest entry of about one) is
+  // taken as zero.
+  const double d = aqq - app, e = 2.0 * apq, h2 = d * d + e * e;
+  const bool skip = !(fabs(apq) > 1e-18);
+  const double r = inv_sqrt(skip ? 1.0 : h2), x = 0.5 + 0.5 * (fabs(d) * r), w = inv_sqrt(x);
+  const double neg = (d != 0.0 && (d > 0.0) != (e > 0.0)) ? -0.5 : 0.5;
+  const double c = skip ? 1.0 : x * w;
+  const double s = skip ? 0.0 : neg * (fabs(e) * r) * w;
+  const double t = s * w;
+  a[N * P + P] = app - t * apq;
+  a[N * Q + Q] = aqq + t * apq;
+  a[N * P + Q] = 0.0;
+  MB2_UNROLL
+  for (int k = 0; k < N; ++k) {
+    if (k == P || k == Q) continue;
+    double &akp = a[k < P ? N * k + P : N * P + k], &akq = a[k < Q ? N * k + Q : N * Q + k];
+    const double x = akp, y = akq;
+    akp = c * x - s * y;
+    akq = s * x + c * y;
+  }
+  MB2_UNROLL
+  for (int k = 0; k < N; ++k) {
+    const double x = v[N * k + P], y = v[N * k + Q];
+    v[N * k + P] = c * x - s * y;
+    v[N * k + Q] = s * x + c * y;
+  }
+}
+
+// Cyclic Jacobi eigen-decomposition of a symmetric NxN matrix (N = 3 or 4).
+// On return w[] holds eigenvalues in ascending order and column k of v is the
+// eigenvector of w[k].  For N = 4 a sweep takes the planes in three pairs of
+// disjoint ones, whose angles depend on different entries: the two divisions
+// and square roots of a pair overlap.
 template <int N>
 MB2_HD void jacobi_eigen(const double *a_in, double *w, double *v) {
-  double a[N * N];
-  for (int i = 0; i < N * N; ++i) a[i] = a_in[i];
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) v[N * i + j] = (i == j) ? 1.0 : 0.0;
+  static_assert(N == 3 || N == 4, "3x3 or 4x4");
+  double a[N * N], u[N * N], big = 0.0;
+  MB2_UNROLL
+  for (int i = 0; i < N * N; ++i) big = fmax(big, fabs(a_in[i]));
+  // scaled by a power of two (exactly) to a largest entry in [1/2, 1)
+  int ex = 0;
+  if (big > 1e-300 && big < 1e300) frexp(big, &ex);
+  const double down = ldexp(1.0, -ex), up = ldexp(1.0, ex);
+  MB2_UNROLL
+  for (int i = 0; i < N * N; ++i) {
+    a[i] = a_in[i] * down;
+    u[i] = (i % (N + 1) == 0) ? 1.0 : 0.0;
+  }
   for (int sweep = 0; sweep < 64; ++sweep) {
     double off = 0.0, diag = 0.0;
+    MB2_UNROLL
     for (int i = 0; i < N; ++i) {
       diag += a[N * i + i] * a[N * i + i];
+      MB2_UNROLL
       for (int j = i + 1; j < N; ++j) off += a[N * i + j] * a[N * i + j];
     }
     if (off <= 1e-32 * diag || off == 0.0) break;
-    for (int p = 0; p < N; ++p)
-      for (int q = p + 1; q < N; ++q) {
-        double apq = a[N * p + q];
-        if (apq == 0.0) continue;
-        double app = a[N * p + p], aqq = a[N * q + q];
-        double theta = (aqq - app) / (2.0 * apq);
-        double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
-        for (int k = 0; k < N; ++k) {
-          double akp = a[N * k + p], akq = a[N * k + q];
-          a[N * k + p] = c * akp - s * akq;
-          a[N * k + q] = s * akp + c * akq;
-        }
-        for (int k = 0; k < N; ++k) {
-          double apk = a[N * p + k], aqk = a[N * q + k];
-          a[N * p + k] = c * apk - s * aqk;
-          a[N * q + k] = s * apk + c * aqk;
-        }
-        for (int k = 0; k < N; ++k) {
-          double vkp = v[N * k + p], vkq = v[N * k + q];
-          v[N * k + p] = c * vkp - s * vkq;
-          v[N * k + q] = s * vkp + c * vkq;
-        }
-      }
-  }
-  for (int i = 0; i < N; ++i) w[i] = a[N * i + i];
-  // sort ascending (selection sort on columns)
-  for (int i = 0; i < N; ++i) {
-    int m = i;
-    for (int j = i + 1; j < N; ++j)
-      if (w[j] < w[m]) m = j;
-    if (m != i) {
-      double t = w[i]; w[i] = w[m]; w[m] = t;
-      for (int k = 0; k < N; ++k) { double u = v[N * k + i]; v[N * k + i] = v[N * k + m]; v[N * k + m] = u; }
+    if constexpr (N == 4) {
+      jacobi_rotate<N, 0, 1>(a, u);
+      jacobi_rotate<N, 2, 3>(a, u);
+      jacobi_rotate<N, 0, 2>(a, u);
+      jacobi_rotate<N, 1, 3>(a, u);
+      jacobi_rotate<N, 0, 3>(a, u);
+      jacobi_rotate<N, 1, 2>(a, u);
+    } else {
+      jacobi_rotate<N, 0, 1>(a, u);
+      jacobi_rotate<N, 0, 2>(a, u);
+      jacobi_rotate<N, 1, 2>(a, u);
     }
   }
+  double d[N];
+  MB2_UNROLL
+  for (int i = 0; i < N; ++i) d[i] = a[N * i + i] * up;
+  // sort ascending (exchanges of columns)
+  MB2_UNROLL
+  for (int i = 0; i < N; ++i)
+    MB2_UNROLL
+    for (int j = i + 1; j < N; ++j) {
+      const bool sw = d[j] < d[i];
+      const double x = d[i], y = d[j];
+      d[i] = sw ? y : x;
+      d[j] = sw ? x : y;
+      MB2_UNROLL
+      for (int k = 0; k < N; ++k) {
+        const double p = u[N * k + i], q = u[N * k + j];
+        u[N * k + i] = sw ? q : p;
+        u[N * k + j] = sw ? p : q;
+      }
+    }
+  MB2_UNROLL
+  for (int i = 0; i < N; ++i) w[i] = d[i];
+  MB2_UNROLL
+  for (int i = 0; i < N * N; ++i) v[i] = u[i];
 }
 
 // Orthogonal polar factor U V^T of a (non-singular) 3x3 matrix:
 // M (M^T M)^(-1/2), computed from the eigen-decomposition of M^T M.
 MB2_HD void orthogonalize3(const double *m, double *o) {
-  double mt[9], mtm[9], w[3], v[9];
+  double mt[9], mtm[9], w[3], v[9], l[3];
   m3_transpose(m, mt);
   m3_mul(mt, m, mtm);
   jacobi_eigen<3>(mtm, w, v);
+  MB2_UNROLL
+  for (int k = 0; k < 3; ++k) l[k] = w[k] > 0.0 ? 1.0 / sqrt(w[k]) : 0.0;
   double isq[9];
+  MB2_UNROLL
   for (int i = 0; i < 3; ++i)
+    MB2_UNROLL
     for (int j = 0; j < 3; ++j) {
       double s = 0.0;
-      for (int k = 0; k < 3; ++k) {
-        double lk = w[k] > 0.0 ? 1.0 / sqrt(w[k]) : 0.0;
-        s += v[3 * i + k] * lk * v[3 * j + k];
-      }
+      MB2_UNROLL
+      for (int k = 0; k < 3; ++k) s += v[3 * i + k] * l[k] * v[3 * j + k];
       isq[3 * i + j] = s;
     }
   m3_mul(m, isq, o);
@@ -205,34 +296,73 @@ MB2_HD bool affine4_inverse(const double *m, double *o) {
 // itkSymMirorrRegistrationMethod.txx.  Every iterate keeps the last row
 // 0 0 0 1, so the inverses are the affine ones.
 MB2_HD void matrix_sqrt4(const double *m, double *y_out) {
-  double y[16], z[16], iy[16], iz[16], d[16];
+  double y[16], z[16], iy[16], iz[16];
+  MB2_UNROLL
   for (int i = 0; i < 16; ++i) { y[i] = m[i]; z[i] = (i % 5 == 0) ? 1.0 : 0.0; }
   double dd = 1.7976931348623157e308;
   int it = 0;
   while (dd > 1e-14 && it < 50) {
     affine4_inverse(z, iz);
     affine4_inverse(y, iy);
-    for (int i = 0; i < 16; ++i) {
+    MB2_UNROLL
+    for (int i = 0; i < 12; ++i) {
       const double ny = 0.5 * (y[i] + iz[i]), nz = 0.5 * (z[i] + iy[i]);
       y[i] = ny;
       z[i] = nz;
     }
     ++it;
-    mn_mul<4>(y, y, d);
+    // y y - m over the first three rows (the last ones are 0 0 0 1)
     dd = 0.0;
-    for (int i = 0; i < 16; ++i) {
-      double a = fabs(d[i] - m[i]);
-      if (a > dd) dd = a;
-    }
+    MB2_UNROLL
+    for (int i = 0; i < 3; ++i)
+      MB2_UNROLL
+      for (int j = 0; j < 4; ++j) {
+        double d = y[4 * i] * y[j] + y[4 * i + 1] * y[4 + j] + y[4 * i + 2] * y[8 + j];
+        if (j == 3) d += y[4 * i + 3];
+        const double e = fabs(d - m[4 * i + j]);
+        if (e > dd) dd = e;
+      }
   }
+  MB2_UNROLL
   for (int i = 0; i < 16; ++i) y_out[i] = y[i];
 }
 
 // ---- Euler3D (Z*X*Y) -------------------------------------------------------
+// Three angles at once.  On the device the four lanes of an aligned quad call
+// these together with the same arguments and each takes one angle: the time of
+// one evaluation instead of three in a row.
+MB2_HD void sincos3(const double *ang, double *s, double *c) {
+#ifdef __CUDA_ARCH__
+  const unsigned lane = threadIdx.x & 31u, quad = 0xFu << (lane & 28u);
+  const double x = (lane & 3u) == 0 ? ang[0] : ((lane & 3u) == 1 ? ang[1] : ang[2]);
+  double sv, cv;
+  sincos(x, &sv, &cv);
+  MB2_UNROLL
+  for (int k = 0; k < 3; ++k) {
+    s[k] = __shfl_sync(quad, sv, k, 4);
+    c[k] = __shfl_sync(quad, cv, k, 4);
+  }
+#else
+  for (int k = 0; k < 3; ++k) { s[k] = sin(ang[k]); c[k] = cos(ang[k]); }
+#endif
+}
+MB2_HD void atan2_3(const double *y, const double *x, double *ang) {
+#ifdef __CUDA_ARCH__
+  const unsigned lane = threadIdx.x & 31u, quad = 0xFu << (lane & 28u);
+  const double yy = (lane & 3u) == 0 ? y[0] : ((lane & 3u) == 1 ? y[1] : y[2]);
+  const double xx = (lane & 3u) == 0 ? x[0] : ((lane & 3u) == 1 ? x[1] : x[2]);
+  const double a = atan2(yy, xx);
+  MB2_UNROLL
+  for (int k = 0; k < 3; ++k) ang[k] = __shfl_sync(quad, a, k, 4);
+#else
+  for (int k = 0; k < 3; ++k) ang[k] = atan2(y[k], x[k]);
+#endif
+}
+
 MB2_HD void euler_zxy_matrix(const double *ang, double *o) {
-  double cx = cos(ang[0]), sx = sin(ang[0]);
-  double cy = cos(ang[1]), sy = sin(ang[1]);
-  double cz = cos(ang[2]), sz = sin(ang[2]);
+  double s3[3], c3[3];
+  sincos3(ang, s3, c3);
+  const double cx = c3[0], sx = s3[0], cy = c3[1], sy = s3[1], cz = c3[2], sz = s3[2];
   double rx[9] = {1, 0, 0, 0, cx, -sx, 0, sx, cx};
   double ry[9] = {cy, 0, sy, 0, 1, 0, -sy, 0, cy};
   double rz[9] = {cz, -sz, 0, sz, cz, 0, 0, 0, 1};
@@ -246,14 +376,14 @@ MB2_HD void euler_zxy_angles(const double *m, double *ang) {
   if (s > 1.0) s = 1.0;
   if (s < -1.0) s = -1.0;
   ang[0] = asin(s);
-  double a = cos(ang[0]);
-  if (fabs(a) > 0.00005) {
-    ang[1] = atan2(-m[6] / a, m[8] / a);
-    ang[2] = atan2(-m[1] / a, m[4] / a);
-  } else {
-    ang[2] = 0.0;
-    ang[1] = atan2(m[3], m[0]);
-  }
+  const double a = cos(ang[0]);
+  const bool regular = fabs(a) > 0.00005;
+  const double y[3] = {0.0, regular ? -m[6] / a : m[3], regular ? -m[1] / a : 0.0};
+  const double x[3] = {1.0, regular ? m[8] / a : m[0], regular ? m[4] / a : 1.0};
+  double t[3];
+  atan2_3(y, x, t);
+  ang[1] = t[1];
+  ang[2] = regular ? t[2] : 0.0;
 }
 
 // ---- transform -------------------------------------------------------------
@@ -406,15 +536,11 @@ MB2_HD void quat_euler_angles(const double *q, double *ang) {
   quat_rotation(q, r);
   m3_transpose(r, rt);
   double xy = sqrt(rt[0] * rt[0] + rt[1] * rt[1]);
-  if (xy > 2.220446049250313e-16 * 8.0) {
-    ang[0] = atan2(rt[5], rt[8]);
-    ang[1] = atan2(-rt[2], xy);
-    ang[2] = atan2(rt[1], rt[0]);
-  } else {
-    ang[0] = atan2(-rt[7], rt[4]);
-    ang[1] = atan2(-rt[2], xy);
-    ang[2] = 0.0;
-  }
+  const bool regular = xy > 2.220446049250313e-16 * 8.0;
+  const double y[3] = {regular ? rt[5] : -rt[7], -rt[2], rt[1]};
+  const double x[3] = {regular ? rt[8] : rt[4], xy, rt[0]};
+  atan2_3(y, x, ang);
+  if (!regular) ang[2] = 0.0;
 }
 MB2_HD void quat_axis_angle(const double *q, double *axis, double *angle) {
   double mag = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]);
@@ -541,14 +667,6 @@ MB2_HD void horn_quaternion(const double *Z, double *q) {
 }
 
 // ---- LTS steps ---------------------------------------------------------------
-// Moments of the LTS subset of one inner iteration.
-struct LtsMoments {
-  double n;         // subset size
-  double mean_i[3]; // barycentre of initial points
-  double mean_m[3]; // barycentre of moved points
-  double Z[36];     // second moments of (initial - mean_i, moved - mean_m), summed
-};
-
 // Working state of one LTS fit (one OptimizeTransform call).
 struct LtsState {
   int kind;
@@ -586,18 +704,20 @@ MB2_HD void lts_begin(LtsState &s) {
   s.failed = 0;
 }
 
-MB2_HD void cov_from_Z(const double *Z, int ra, int cb, double n, double *o) {
-  // o[r][c] = sum A[r] * B[c] / n with A = z[ra..ra+2], B = z[cb..cb+2]
-  for (int r = 0; r < 3; ++r)
-    for (int c = 0; c < 3; ++c) o[3 * r + c] = Z[6 * (ra + r) + (cb + c)] / n;
-}
-
-// Least-squares affine A = Cov(y, x) Cov(x, x)^-1, skipping the inverse when
-// |det Cov(x, x)| < 1e-4 (itkMirorrRegistrationMethod.txx:871-883).
-MB2_HD void affine_ls(const double *Z, int xo, int yo, double n, double *rot) {
+// Least-squares affine A = Cov(y, x) Cov(x, x)^-1 with x the initial and y the
+// moved points (back: the other way), skipping the inverse when
+// |det Cov(x, x)| < 1e-4 (itkMirorrRegistrationMethod.txx:871-883).  zn: the
+// second moments divided by the subset's size.
+MB2_HD void affine_ls_n(const double *zn, bool back, double *rot) {
   double oxy[9], oxx[9];
-  cov_from_Z(Z, yo, xo, n, oxy);
-  cov_from_Z(Z, xo, xo, n, oxx);
+  MB2_UNROLL
+  for (int r = 0; r < 3; ++r)
+    MB2_UNROLL
+    for (int c = 0; c < 3; ++c) {
+      oxy[3 * r + c] = back ? zn[6 * r + 3 + c] : zn[6 * (3 + r) + c];
+      oxx[3 * r + c] = back ? zn[6 * (3 + r) + 3 + c] : zn[6 * r + c];
+    }
+  MB2_UNROLL
   for (int i = 0; i < 9; ++i) rot[i] = oxy[i];
   if (fabs(m3_det(oxx)) >= 1e-4) {
     double inv[9];
@@ -606,37 +726,33 @@ MB2_HD void affine_ls(const double *Z, int xo, int yo, double n, double *rot) {
 }
 
 // One inner iteration of the classic fit, after the subset moments are known
-// (itkMirorrRegistrationMethod.txx:841-998).
-MB2_HD void lts_classic_step(LtsState &s, const LtsMoments &mo) {
-  double np[12];
-  for (int i = 0; i < 12; ++i) np[i] = s.last_params[i];
-  const double *im = mo.mean_i, *mm = mo.mean_m;
-  double mfc[3], ifc[3];
-  for (int i = 0; i < 3; ++i) { mfc[i] = mm[i] - s.rc[i]; ifc[i] = im[i] - s.rc[i]; }
-  double rot[9];
-  if (s.kind == KIND_AFFINE) {
-    affine_ls(mo.Z, 0, 3, mo.n, rot);
-    double ri[3];
+// (itkMirorrRegistrationMethod.txx:841-998): T (whose centre is the previous
+// subset's barycentre) from the subset; np: the new parameters.  im, mm: the
+// subset's barycentres; Z, zn: its second moments, and those divided by its
+// size.
+MB2_HD void classic_fit(Tfm &T, const double *im, const double *mm, const double *Z,
+                        const double *zn, double *np) {
+  double mfc[3], ifc[3], rot[9], ri[3];
+  MB2_UNROLL
+  for (int i = 0; i < 3; ++i) { mfc[i] = mm[i] - T.c[i]; ifc[i] = im[i] - T.c[i]; }
+  if (T.kind == KIND_AFFINE) {
+    affine_ls_n(zn, false, rot);
     m3_vec(rot, ifc, ri);
+    MB2_UNROLL
     for (int i = 0; i < 9; ++i) np[i] = rot[i];
+    MB2_UNROLL
     for (int i = 0; i < 3; ++i) np[9 + i] = mfc[i] - ri[i];
   } else {
-    double q[4];
-    horn_quaternion(mo.Z, q);
+    double q[4], ang[3];
+    horn_quaternion(Z, q);
     quat_rotation(q, rot);
-    double ri[3], ang[3];
     m3_vec(rot, ifc, ri);
     quat_euler_angles(q, ang);
+    MB2_UNROLL
     for (int i = 0; i < 3; ++i) { np[i] = ang[i]; np[3 + i] = mfc[i] - ri[i]; }
   }
-  s.last_delta = s.delta;
-  double d = 0.0;
-  int npar = tfm_nparams(s.fin);
-  for (int i = 0; i < npar; ++i) { double e = s.last_params[i] - np[i]; d += e * e; }
-  s.delta = d;
-  for (int i = 0; i < 3; ++i) s.rc[i] = im[i];
-  tfm_set_center(s.fin, s.rc);
-  tfm_set_params(s.fin, np);
+  tfm_set_center(T, im);
+  tfm_set_params(T, np);
 }
 
 MB2_HD void half_step(const double *K, const double *trans, double *m12) {
@@ -650,119 +766,127 @@ MB2_HD void half_step(const double *K, const double *trans, double *m12) {
   matrix_sqrt4(m, m12);
 }
 
-// One inner iteration of the symmetric fit (itkSymMirorrRegistrationMethod.txx:865-1432)
-// in three parts: lts_symmetric_pre (the two least-squares fits and the
-// averaged half-way matrices Kf, Kb with translations tf, tb), the two
-// independent square roots half_step(Kf, tf) and half_step(Kb, tb), which the
-// device runs on two lanes at once, and lts_symmetric_post.
-struct SymHalf {
-  double np[12];
-  double K[2][9];
-  double t[2][3];
-};
+// One inner iteration of the symmetric fit (itkSymMirorrRegistrationMethod.txx:865-1432),
+// in stages that each work on one half (forward h = 0, backward h = 1) and see
+// the other half's result of the stage before: the device runs the two halves
+// on two lane groups at once, exchanging by shuffles.
+//   sym_fit      the half's least-squares fit in T; inv: T's inverse matrix
+//   sym_mean     T's matrix averaged with the other half's inverse; T moved to
+//                centre 0; iT: its inverse
+//   sym_half     the matrix and translation averaged with the other half's iT,
+//                then the half-way square root m12
+//   sym_finish   T from the square root
 
-MB2_HD void lts_symmetric_pre(LtsState &s, const LtsMoments &mo, SymHalf &h) {
-  double *np = h.np;
-  for (int i = 0; i < 12; ++i) np[i] = s.last_params[i];
-  const double *im = mo.mean_i, *mm = mo.mean_m;
-  double translation[3], ntrans[3];
-  for (int i = 0; i < 3; ++i) { translation[i] = mm[i] - im[i]; ntrans[i] = -translation[i]; }
-  Tfm &ff = s.fin;
-  Tfm &fb = s.finb;
-  if (s.kind == KIND_AFFINE) {
-    double rf[9], rb[9];
-    affine_ls(mo.Z, 0, 3, mo.n, rf);
-    affine_ls(mo.Z, 3, 0, mo.n, rb);
-    for (int i = 0; i < 9; ++i) np[i] = rf[i];
-    for (int i = 0; i < 3; ++i) np[9 + i] = translation[i];
-    double pf[12], pb[12];
-    for (int i = 0; i < 9; ++i) { pf[i] = rf[i]; pb[i] = rb[i]; }
-    for (int i = 0; i < 3; ++i) { pf[9 + i] = translation[i]; pb[9 + i] = ntrans[i]; }
-    tfm_set_center(ff, im); tfm_set_params(ff, pf);
-    tfm_set_center(fb, mm); tfm_set_params(fb, pb);
-    double ibm[9], ifm[9], K[9], Mb[9];
-    mn_inverse<3>(fb.M, ibm);
-    mn_inverse<3>(ff.M, ifm);
-    for (int i = 0; i < 9; ++i) { K[i] = (ff.M[i] + ibm[i]) / 2.0; Mb[i] = (ifm[i] + fb.M[i]) / 2.0; }
-    tfm_set_matrix(ff, K);
-    tfm_set_matrix(fb, Mb);
+// im, mm: the subset's barycentres; Z, zn: its second moments, and those
+// divided by its size; np: the new parameters (meaningful for h = 0).
+MB2_HD void sym_fit(Tfm &T, int h, const double *im, const double *mm, const double *Z,
+                    const double *zn, double *np, double *inv) {
+  double tr[3], p[12];
+  MB2_UNROLL
+  for (int i = 0; i < 3; ++i) tr[i] = h ? -(mm[i] - im[i]) : mm[i] - im[i];
+  if (T.kind == KIND_AFFINE) {
+    double rot[9];
+    affine_ls_n(zn, h != 0, rot);
+    MB2_UNROLL
+    for (int i = 0; i < 9; ++i) np[i] = p[i] = rot[i];
+    MB2_UNROLL
+    for (int i = 0; i < 3; ++i) np[9 + i] = p[9 + i] = tr[i];
   } else {
-    double q[4], ang[3], axis[3], angle, qf[4], qb[4], af[3], ab[3];
-    horn_quaternion(mo.Z, q);
+    double q[4], ang[3], axis[3], angle, qh[4], ah[3];
+    horn_quaternion(Z, q);
     quat_euler_angles(q, ang);
     quat_axis_angle(q, axis, &angle);
-    quat_from_axis_angle(axis, angle, qf);
-    quat_from_axis_angle(axis, -angle, qb);
-    quat_euler_angles(qf, af);
-    quat_euler_angles(qb, ab);
-    for (int i = 0; i < 3; ++i) { np[i] = ang[i]; np[3 + i] = translation[i]; }
-    double pf[6] = {af[0], af[1], af[2], translation[0], translation[1], translation[2]};
-    double pb[6] = {ab[0], ab[1], ab[2], ntrans[0], ntrans[1], ntrans[2]};
-    tfm_set_center(ff, im); tfm_set_params(ff, pf);
-    tfm_set_center(fb, mm); tfm_set_params(fb, pb);
-    double ibm[9], K[9], Ko[9], Kt[9];
-    mn_inverse<3>(fb.M, ibm);
-    for (int i = 0; i < 9; ++i) K[i] = (ff.M[i] + ibm[i]) / 2.0;
-    orthogonalize3(K, Ko);
-    m3_transpose(Ko, Kt);
-    if (!tfm_set_matrix(ff, Ko) || !tfm_set_matrix(fb, Kt)) s.failed = 1;
+    quat_from_axis_angle(axis, h ? -angle : angle, qh);
+    quat_euler_angles(qh, ah);
+    MB2_UNROLL
+    for (int i = 0; i < 3; ++i) {
+      np[i] = ang[i];
+      np[3 + i] = tr[i];
+      p[i] = ah[i];
+      p[3 + i] = tr[i];
+    }
   }
-  double offf[3] = {ff.off[0], ff.off[1], ff.off[2]};
-  double offb[3] = {fb.off[0], fb.off[1], fb.off[2]};
-  double zero[3] = {0, 0, 0};
-  tfm_set_center(ff, zero); tfm_set_center(fb, zero);
-  tfm_set_translation(ff, offf); tfm_set_translation(fb, offb);
-  Tfm iF, iB;
-  tfm_inverse(ff, iF);
-  tfm_inverse(fb, iB);
-  double Kf[9], Kb[9], tf[3], tb[3];
-  for (int i = 0; i < 9; ++i) { Kf[i] = (ff.M[i] + iB.M[i]) / 2.0; Kb[i] = (iF.M[i] + fb.M[i]) / 2.0; }
-  if (s.kind == KIND_RIGID) {
-    double a[9], b[9];
-    orthogonalize3(Kf, a); orthogonalize3(Kb, b);
-    for (int i = 0; i < 9; ++i) { Kf[i] = a[i]; Kb[i] = b[i]; }
-  }
-  for (int i = 0; i < 3; ++i) { tf[i] = (ff.t[i] + iB.t[i]) / 2.0; tb[i] = (iF.t[i] + fb.t[i]) / 2.0; }
-  for (int i = 0; i < 9; ++i) { h.K[0][i] = Kf[i]; h.K[1][i] = Kb[i]; }
-  for (int i = 0; i < 3; ++i) { h.t[0][i] = tf[i]; h.t[1][i] = tb[i]; }
+  tfm_set_center(T, h ? mm : im);
+  tfm_set_params(T, p);
+  MB2_UNROLL
+  for (int i = 0; i < 9; ++i) inv[i] = 0.0;
+  mn_inverse<3>(T.M, inv);
 }
 
-MB2_HD void lts_symmetric_post(LtsState &s, const SymHalf &h, const double *m12,
-                               const double *im12) {
-  const double *np = h.np;
-  Tfm &ff = s.fin;
-  Tfm &fb = s.finb;
-  double k3[9], l3[9];
+// T's matrix set to K (affine: the half's own mean; rigid: the orthogonalised
+// forward mean, transposed for the backward half).  Returns whether a rigid T
+// took it.
+MB2_HD bool sym_mean(Tfm &T, int h, const double *K) {
+  double k[9];
+  if (T.kind == KIND_AFFINE) {
+    MB2_UNROLL
+    for (int i = 0; i < 9; ++i) k[i] = K[i];
+  } else {
+    double o[9];
+    orthogonalize3(K, o);
+    MB2_UNROLL
+    for (int r = 0; r < 3; ++r)
+      MB2_UNROLL
+      for (int c = 0; c < 3; ++c) k[3 * r + c] = h ? o[3 * c + r] : o[3 * r + c];
+  }
+  return tfm_set_matrix(T, k);
+}
+
+MB2_HD void sym_to_origin(Tfm &T, Tfm &iT) {
+  const double off[3] = {T.off[0], T.off[1], T.off[2]};
+  const double zero[3] = {0, 0, 0};
+  tfm_set_center(T, zero);
+  tfm_set_translation(T, off);
+  tfm_identity(iT, T.kind);
+  tfm_inverse(T, iT);
+}
+
+MB2_HD void sym_half(const Tfm &T, const double *oM, const double *ot, double *m12) {
+  double K[9], t[3];
+  MB2_UNROLL
+  for (int i = 0; i < 9; ++i) K[i] = (T.M[i] + oM[i]) / 2.0;
+  if (T.kind == KIND_RIGID) {
+    double o[9];
+    orthogonalize3(K, o);
+    MB2_UNROLL
+    for (int i = 0; i < 9; ++i) K[i] = o[i];
+  }
+  MB2_UNROLL
+  for (int i = 0; i < 3; ++i) t[i] = (T.t[i] + ot[i]) / 2.0;
+  half_step(K, t, m12);
+}
+
+// T's matrix from the square root, and whether T took it; with reorth, the
+// orthogonalised one (SymMirorrRegistrationMethod re-orthogonalises both halves
+// when one is rejected, :1327-1342).
+MB2_HD bool sym_finish(Tfm &T, const double *m12, bool reorth) {
+  double k[9];
+  MB2_UNROLL
   for (int r = 0; r < 3; ++r)
-    for (int c = 0; c < 3; ++c) { k3[3 * r + c] = m12[4 * r + c]; l3[3 * r + c] = im12[4 * r + c]; }
-  Tfm ffs = ff, fbs = fb;
-  if (!tfm_set_matrix(ff, k3) || !tfm_set_matrix(fb, l3)) {
-    // SymMirorrRegistrationMethod re-orthogonalises both on rejection (:1327-1342)
-    ff = ffs; fb = fbs;
-    double ko[9], lo[9];
-    orthogonalize3(k3, ko);
-    orthogonalize3(l3, lo);
-    tfm_set_matrix(ff, ko);
-    tfm_set_matrix(fb, lo);
+    MB2_UNROLL
+    for (int c = 0; c < 3; ++c) k[3 * r + c] = m12[4 * r + c];
+  if (reorth) {
+    double o[9];
+    orthogonalize3(k, o);
+    MB2_UNROLL
+    for (int i = 0; i < 9; ++i) k[i] = o[i];
   }
-  double t12[3] = {m12[3], m12[7], m12[11]}, it12[3] = {im12[3], im12[7], im12[11]};
-  tfm_set_translation(ff, t12);
-  tfm_set_translation(fb, it12);
-  s.last_delta = s.delta;
-  double d = 0.0;
-  int npar = tfm_nparams(s.tfm);
-  for (int i = 0; i < npar; ++i) { double e = s.last_params[i] - np[i]; d += e * e; }
-  s.delta = d;
-  for (int i = 0; i < 12; ++i) s.last_params[i] = np[i];
+  return tfm_set_matrix(T, k);
 }
 
-MB2_HD void lts_symmetric_step(LtsState &s, const LtsMoments &mo) {
-  SymHalf h;
-  lts_symmetric_pre(s, mo, h);
-  double m12[16], im12[16];
-  half_step(h.K[0], h.t[0], m12);
-  half_step(h.K[1], h.t[1], im12);
-  lts_symmetric_post(s, h, m12, im12);
+// The loop's parameter change; the symmetric method compares with the last
+// parameters, the classic one with the identity's throughout.
+MB2_HD void lts_delta(LtsState &s, const double *np) {
+  double d = 0.0;
+  MB2_UNROLL
+  for (int i = 0; i < 12; ++i)
+    if (i < 6 || s.kind == KIND_AFFINE) {
+      const double e = s.last_params[i] - np[i];
+      d += e * e;
+      if (s.symmetric) s.last_params[i] = np[i];
+    }
+  s.last_delta = s.delta;
+  s.delta = d;
 }
 
 // After the inner loop: m_Transform->Compose(final, true) (classic) or the
