@@ -5,8 +5,11 @@
 //                   mu(p) (over all BW^3 voxels, unmasked, as
 //                   itkBlockMatcher.txx:57-68) and the masked sum of squares
 //                   Syy(p) = sum_{ms != 0} (y - mu)^2, both in FP64 in the
-//                   reference's raster order, stored as float2; the sign bit
-//                   of Syy is set when a search-mask voxel of the footprint is 0.
+//                   reference's raster order, stored as the float2
+//                   (mu, 1 / Syy), 0 for Syy = 0: the search multiplies by it
+//                   once per block and candidate (some 27 times a voxel); the
+//                   sign bit of the second is set when a search-mask voxel of
+//                   the footprint is 0.
 //   2. selection:   (optional) dead-code variance cut-off of
 //                   itkBlockMatcher.txx:664-719, FP64 per block, exact k-th
 //                   value by a device radix select.
@@ -15,6 +18,8 @@
 //                   deterministic raster-order compaction and block -> mm points
 //                   (itkAbstractBlockMatcher.h:271-287).
 #include <cuda_bf16.h>
+
+#include <cfloat>
 #include <type_traits>
 #include <cuda_fp16.h>
 
@@ -93,7 +98,8 @@ __device__ __noinline__ double box_ss64(const float *__restrict__ y,
 template <int BW>
 __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict__ y,
                                                         const uint8_t *__restrict__ ms, int nx,
-                                                        int ny, int nz, float2 *__restrict__ out) {
+                                                        int ny, int nz, int sp,
+                                                        float2 *__restrict__ out) {
   constexpr int PZ = kBoxPZ, NP = PZ + BW - 1;
   const int ngz = (nz + PZ - 1) / PZ;
   const long long n = (long long)nx * ny * ngz;
@@ -178,7 +184,8 @@ __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict_
 #pragma unroll
     for (int j = 0; j < PZ; ++j) {
       if (z0 + j >= nz) break;
-      float2 r = make_float2(0.f, 0.f);
+      // not a candidate (the footprint leaves the volume): NaN
+      float2 r = make_float2(0.f, __int_as_float(0x7fc00000));
       if (ok[j]) {
         double ss = (double)s32[j];
         // no masked voxel: zero; with a mean that is a float, v - mean is zero
@@ -187,9 +194,10 @@ __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict_
         if (any_in[j] && s32[j] < 1e-30f && (double)(float)mean[j] != mean[j])
           ss = box_ss64<BW>(y, ms, o + j * plane, nx, ny, mean[j]);
         const float fs = (float)ss;
-        r = make_float2((float)mean[j], all_in[j] ? fs : -fs);
+        const float rs = fs > 0.f ? fmaxf(fminf(__frcp_rn(fs), FLT_MAX), FLT_MIN) : fs;
+        r = make_float2((float)mean[j], all_in[j] ? rs : -rs);
       }
-      out[o + j * plane] = r;
+      out[((long long)(z0 + j) * ny + yy) * sp + x] = r;
     }
   }
 }
@@ -202,7 +210,7 @@ mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8
   if (blocks > (long long)sm_count() * 64) blocks = (long long)sm_count() * 64;
   switch (g.bw) {
 #define CASE(B) \
-  case B: box_stats_kernel<B><<<(unsigned)blocks, threads, 0, s>>>(search, smask, g.size[0], g.size[1], g.size[2], stats); break;
+  case B: box_stats_kernel<B><<<(unsigned)blocks, threads, 0, s>>>(search, smask, g.size[0], g.size[1], g.size[2], stats_pitch(g.size[0]), stats); break;
     CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
 #undef CASE
     default:

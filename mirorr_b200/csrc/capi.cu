@@ -331,8 +331,8 @@ mirorr_status run_match(mirorr_ctx c, const mirorr_bm_params &p, const MatchCall
     set_error("image smaller than one block or invalid block parameters");
     return MIRORR_EINVAL;
   }
-  long long nvox = (long long)mc.size[0] * mc.size[1] * mc.size[2];
-  if (!is16(mc.dtype)) MB2_TRY(c->bmw.stats.ensure(sizeof(float2) * nvox));
+  if (!is16(mc.dtype)) MB2_TRY(c->bmw.stats.ensure(sizeof(float2) * (size_t)stats_pitch(mc.size[0]) * mc.size[1] *
+                                                     mc.size[2]));
   MB2_TRY(best.ensure(sizeof(float) * g.nblocks));
   MB2_TRY(second.ensure(sizeof(float) * g.nblocks));
   MB2_TRY(match.ensure(sizeof(int32_t) * g.nblocks));

@@ -51,6 +51,12 @@ struct PointGeom {
 void point_geom(const double origin[3], const double spacing[3], const double direction[9],
                 int bw, PointGeom &pg);
 
+// Row pitch of the float32 search's statistics (float2 per candidate origin):
+// rows start on 16 bytes, so that a tensor map can address them.
+inline int stats_pitch(int nx) { return (nx + 1) & ~1; }
+// stats: (mean, 1 / masked sum of squares) per candidate origin; the second is
+// 0 when the sum is, NaN where the footprint leaves the volume, and its sign
+// bit is set when some voxel of the footprint is outside the search mask.
 mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8_t *smask,
                                float2 *stats, cudaStream_t s);
 // base: float32, or 16-bit when dtype is MIRORR_DTYPE_BF16 / _F16.
@@ -285,11 +291,6 @@ mirorr_status lts_run(LtsWork &w, LtsState &host_state, const double *init_dev,
                       cudaStream_t s, int *inner_iters, long long *n_used,
                       const unsigned int *watch_dev = nullptr,
                       unsigned int *watch_host = nullptr);
-// Window-AND of the footprint-in-mask flags of box statistics (sign bit of
-// the second field), per block of g: 1 when every candidate footprint of the
-// block's window that lies in the volume is wholly inside the search mask.
-mirorr_status launch_window_and(const BmGeom &g, const float2 *stats, DevBuf &buf,
-                                const uint8_t **wand, cudaStream_t s);
 // The NCC stage's give-up flag (device word), or nullptr before any search.
 const unsigned int *ncc_timeout_flag(const BmWork &w);
 // The give-up flag ncc_take_timeout reads, allocated (and zeroed) if the

@@ -18,7 +18,7 @@
 //      and the list of candidates whose FP32 score lies within 2*delta of the
 //      FP32 second-best (delta bounds |FP32 - FP64|), plus the first two
 //      degenerate candidates when fewer than two are non-degenerate.
-//        * ncc_xlane_kernel (block width 4, window 7 or 9) and
+//        * ncc_xlane_kernel (block width 4, window 5, 7 or 9) and
 //          ncc_warp_kernel (other widths): blocks whose base block and search
 //          window are wholly inside both masks, block gap 1; cross term only,
 //          one FMA per voxel and candidate.  They route the other blocks.
@@ -34,6 +34,8 @@
 //      Blocks whose list overflowed are re-scored entirely by
 //      ncc_fallback_kernel.
 #include <cuda.h>  // CUtensorMap (the encoder is fetched through the runtime)
+
+#include <cfloat>
 
 #include "kernels.cuh"
 
@@ -67,7 +69,8 @@ struct NccArgs {
   const uint8_t *bmask;
   const float *search;
   const uint8_t *smask;
-  const float2 *stats;
+  const float2 *stats;  // box_stats, rows of sp
+  int sp;
   const uint8_t *selected;
   const BlockStat *bstat;
   int nx, ny, nz;
@@ -128,6 +131,11 @@ __device__ inline bool block_window(const NccArgs &a, long long b, BlockWin &w) 
 
 __device__ inline long long lin(const NccArgs &a, int x, int y, int z) {
   return ((long long)z * a.ny + y) * a.nx + x;
+}
+
+// Index of the statistics of candidate origin (x, y, z).
+__device__ inline long long sidx(const NccArgs &a, int x, int y, int z) {
+  return ((long long)z * a.ny + y) * a.sp + x;
 }
 
 __device__ inline void write_final(const NccArgs &a, long long b, float best, float second,
@@ -214,10 +222,37 @@ __device__ inline void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-// box_stats stores Syy with its sign bit set when some search-mask voxel of
-// the candidate's footprint is zero.
-__device__ inline bool footprint_in_mask(float syy_field) { return !signbit(syy_field); }
-__device__ inline float syy_of(float syy_field) { return fabsf(syy_field); }
+// Packed pairs of FP32 values (one 64-bit register): one instruction works on
+// both halves, each rounded as the scalar operation.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float sum2(f32x2 v) {
+  float lo, hi;
+  unpack2(v, lo, hi);
+  return lo + hi;
+}
+
+// box_stats stores 1 / Syy (0 when Syy is) with its sign bit set when some
+// search-mask voxel of the candidate's footprint is zero.
+__device__ inline bool footprint_in_mask(float field) { return !signbit(field); }
+__device__ inline float rsyy_of(float field) { return fabsf(field); }
 
 __device__ inline void push_deg(int &d1, int &d2, int p) {
   if (d1 < 0) d1 = p;
@@ -283,7 +318,7 @@ __global__ void block_stat_kernel(NccArgs a) {
     s.sxx = (float)sxx;
     s.sxt = (float)sxt;
     s.mmode = nin == bw * bw * bw ? 1 : (nin == 0 ? 2 : 0);
-    s.c = __ldg(&a.stats[o]).x;
+    s.c = __ldg(&a.stats[sidx(a, a.stx + bx * a.G, a.sty + by * a.G, a.stz + bz * a.G)]).x;
     const_cast<BlockStat *>(a.bstat)[b] = s;
   }
 }
@@ -369,8 +404,9 @@ __device__ void finish_tile(const NccArgs &a, TileTail<C::BPC, C::TPB> &tt, cons
   }
   __syncthreads();
   {
-    const int wp = tid >> 5, ln = tid & 31;
-    if (wp < BPC && s_state[wp]) {
+    const int ln = tid & 31;
+    for (int wp = tid >> 5; wp < BPC; wp += C::NT / 32) {
+      if (!s_state[wp]) continue;
       float f1 = -3.f, f2 = -3.f;
       int e1 = -1, e2 = -1;
       for (int k = ln; k < TPB; k += 32) {
@@ -478,14 +514,13 @@ __global__ void __launch_bounds__(C::NT, 4) ncc_masked_kernel(NccArgs a) {
         s_o[tid][0] = ox - R;
         s_o[tid][1] = oy - R;
         s_o[tid][2] = oz - R;
-        const long long o = ((long long)oz * ny + oy) * nx + ox;
         const BlockStat st = a.bstat[b];
         if (st.mmode == 1) {
           state = 1;
           s_mean[tid] = st.mean;
           s_sxt[tid] = st.sxt;
           s_sxx[tid] = st.sxx;
-          s_c[tid] = __ldg(&a.stats[o]).x;  // the block's own position is a candidate
+          s_c[tid] = st.c;  // the block's own position is a candidate
         } else {
           unsigned int p = atomicAdd(&a.ctl[0], 1u);
           a.gen_list[p] = b;
@@ -615,19 +650,20 @@ __global__ void __launch_bounds__(C::NT, 4) ncc_masked_kernel(NccArgs a) {
         const int py = s_o[slot][1] + cy;
         const bool rowok = py >= 0 && py <= ny - BW && pz >= 0 && pz <= nz - BW;
         const long long prow = ((long long)pz * ny + py) * nx + s_o[slot][0];
+        const long long srow = sidx(a, s_o[slot][0], py, pz);
 #pragma unroll
         for (int x = 0; x < W; ++x) {
           const int px = s_o[slot][0] + x;
           const int cl = (cz * W + cy) * W + x;
           float s = -4.f;  // not a candidate
           if (rowok && px >= 0 && px <= nx - BW) {
-            const float2 st = __ldg(&a.stats[prow + x]);
-            const float syy = syy_of(st.y);
-            if (syy <= 0.f) {
+            const float2 st = __ldg(&a.stats[srow + x]);
+            const float rsyy = rsyy_of(st.y);
+            if (rsyy <= 0.f) {
               s = -2.f;
             } else if (footprint_in_mask(st.y)) {
               const float sxy = sc[j][x] - (st.x - cc) * sxt;
-              s = sxx_b <= 0.f ? -2.f : __fdividef(__fdividef(sxy * sxy, sxx_b), syy);
+              s = sxx_b <= 0.f ? -2.f : __fdividef(sxy * sxy, sxx_b) * rsyy;
             } else {
               // footprint across the mask edge: C1 kept, finished below
               slist[slot * NC + atomicAdd(&s_nstr[slot], 1)] = cl;
@@ -664,9 +700,9 @@ __global__ void __launch_bounds__(C::NT, 4) ncc_masked_kernel(NccArgs a) {
           }
         const long long p = ((long long)(s_o[slot][2] + czz) * ny + s_o[slot][1] + cy) * nx +
                             s_o[slot][0] + x;
-        const float2 st = __ldg(&a.stats[p]);
+        const float2 st = __ldg(&a.stats[sidx(a, s_o[slot][0] + x, s_o[slot][1] + cy, s_o[slot][2] + czz)]);
         const float sxy = scs[slot * NC + cl] - (st.x - cc) * c2;
-        const float s = c3 <= 0.f ? -2.f : __fdividef(__fdividef(sxy * sxy, c3), syy_of(st.y));
+        const float s = c3 <= 0.f ? -2.f : __fdividef(sxy * sxy, c3) * rsyy_of(st.y);
         scs[slot * NC + cl] = s;
         if (s == -2.f) min2_merge(d1, d2, (int)p, -1);  // list order: keep the two smallest
         top2_merge(l1, l2, s, -3.f);
@@ -786,7 +822,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
           const int py = s_o[slot][1] + cy0 + j, px = s_o[slot][0] + x;
           const bool ok = cy0 + j < W && px >= 0 && px <= nx - BW && py >= 0 && py <= ny - BW &&
                           pz >= 0 && pz <= nz - BW;
-          nmu[j][x] = ok ? -__ldg(&a.stats[((long long)pz * ny + py) * nx + px]).x : 0.f;
+          nmu[j][x] = ok ? -__ldg(&a.stats[sidx(a, px, py, pz)]).x : 0.f;
           s1[j][x] = 0.f;
           s2[j][x] = 0.f;
           s3[j][x] = 0.f;
@@ -974,7 +1010,7 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
         const int z = row / W, y = row - z * W;
         const int gx = ox + x, gy = oy + y, gz = oz + z;
         if (gx >= 0 && gy >= 0 && gz >= 0 && gx <= nx - BW && gy <= ny - BW && gz <= nz - BW)
-          cp_async8(sst + e, a.stats + ((long long)gz * ny + gy) * nx + gx);
+          cp_async8(sst + e, a.stats + sidx(a, gx, gy, gz));
         else
           sst[e] = make_float2(__int_as_float(0x7fc00000), 0.f);  // not a candidate (NaN)
       }
@@ -1062,9 +1098,9 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
           if (cy < W) {
             const float2 q = sst[(cz * W + cy) * W + x];
             if (q.x == q.x) {
-              const float syy = syy_of(q.y);
+              const float rsyy = rsyy_of(q.y);
               const float sxy = sc[j][x] - (q.x - cc) * sxt;
-              s = (sxx_b <= 0.f || syy <= 0.f) ? -2.f : __fdividef(__fdividef(sxy * sxy, sxx_b), syy);
+              s = (sxx_b <= 0.f || rsyy <= 0.f) ? -2.f : __fdividef(sxy * sxy, sxx_b) * rsyy;
               if (s == -2.f) push_deg(d1, d2, (int)(((long long)(oz + cz) * ny + oy + cy) * nx + ox + x));
               top2_merge(l1, l2, s, -3.f);
             }
@@ -1129,8 +1165,8 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
 // (y, z) row, then along y and z at block resolution; out-of-range positions
 // count as 1.
 // ---------------------------------------------------------------------------
-__global__ void wand_x_kernel(const float2 *stats, uint8_t *out, int nx, int ny, int nz, int nbx,
-                              int stx, int G, int W, int bw) {
+__global__ void wand_x_kernel(const float2 *stats, int sp, uint8_t *out, int nx, int ny, int nz,
+                              int nbx, int stx, int G, int W, int bw) {
   const int R = W / 2;
   const long long n = (long long)nbx * ny * nz;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -1141,7 +1177,7 @@ __global__ void wand_x_kernel(const float2 *stats, uint8_t *out, int nx, int ny,
     const int sx = stx + bx * G - R;
     unsigned v = 1;
     if (y <= ny - bw && z <= nz - bw) {
-      const float *fy = reinterpret_cast<const float *>(stats + yz * nx) + 1;
+      const float *fy = reinterpret_cast<const float *>(stats + yz * sp) + 1;
       for (int q = sx < 0 ? 0 : sx; q < sx + W && q <= nx - bw; ++q)
         v &= footprint_in_mask(__ldg(fy + 2 * q)) ? 1u : 0u;
     }
@@ -1180,42 +1216,110 @@ __global__ void wand_axis_kernel(const uint8_t *in, uint8_t *out, long long inne
 // volume, completing on an mbarrier whose wait is bounded; at every load the
 // lanes read consecutive floats of one row (no bank conflicts).  The lane's base
 // block (x~ = x - mean, 64 values) sits in registers and each window row is
-// read once, shifted by the block's constant c as it is read
+// shifted by the block's constant c as it is read
 // (Sxy = sum x~ (y - c) - (mu - c) sum x~ keeps the FP32 cross term free of
-// cancellation).  A window plane wz feeds the candidate planes wz - 3 .. wz;
-// their accumulators rotate through four register sets and a plane is scored
-// once its last window plane has been read.  The scores go to the shared
-// memory of a window plane every warp has consumed (a CTA barrier per plane
-// makes sure of it; lanes without a block run the loop on placeholder data
-// and write nothing); after the block-level top-2
-// reduction one pass over them lists the candidates within 2 delta of the
-// block's FP32 second-best.  Blocks whose window is partly masked (window-AND
-// of the footprint flags) go to the masked kernel, blocks with a partly
-// masked base block to the base-mask kernel.
+// cancellation).
+//
+// What bounds it is instruction issue: 64 multiply-adds a candidate on the FP32
+// pipe, and everything else beside them.  So
+//   * the multiply-adds are packed pairs over the base block's x (even and odd
+//     vx in the two halves, added at the end): half the instructions, with both
+//     operands as they lie in registers (a row's four values are two pairs);
+//   * the candidate planes are taken in groups of P.  A group's P W sums stay
+//     in registers while its P + 3 window planes pass, each feeding only the
+//     candidate planes that use it, so nothing is multiplied for planes that do
+//     not exist and no accumulator moves;
+//   * the statistics come as (mu, 1 / Syy) by one tensor copy per group.
+// After a group its first window planes are dead, and the scores go there (a
+// CTA barrier says so); lanes without a block run along on placeholder data
+// and write nothing.  After the block-level top-2 reduction a pass over the
+// scores lists the candidates within 2 delta of the block's FP32 second-best.
+// Measured (256 x 256 x 128, W = 9, spacing 3, 211 M candidates): 1.83 ms with
+// scalar multiply-adds, four accumulator planes rotating and a division per
+// candidate (14.7 TFLOP/s, 20 % of the nominal FP32 peak); 1.14 ms now (23.7
+// TFLOP/s).  7.1K instructions per warp and tile (were about 15K), 2.8K of them
+// packed multiply-adds.  W = 5 (131 x 117 x 61, spacing 2): 0.81 ms in the
+// general kernel, 0.10 ms here.
+//
+// Blocks whose window is partly masked (window-AND of the footprint flags) go
+// to the masked kernel, blocks with a partly masked base block to the base-mask
+// kernel.
 // ---------------------------------------------------------------------------
-constexpr int kXWarpsPerSM = 12;  // resident warps per SM aimed for
 constexpr int kXWarps = 2;        // warps per CTA
+constexpr int kXtPitch = 68;      // floats per staged base block (the blocks' banks differ)
+constexpr int kXCtasPerSM = 6;    // resident CTAs per SM aimed for
 
 struct XArgs {
   const uint8_t *wand;  // per block: window wholly inside the search mask
   int rpu;              // union row pitch in floats (multiple of 4, the box's x extent)
-  int nch;              // 16-byte chunks per union row
+  int spu;              // x extent of the statistics box (even)
+  int soff, xoff;       // where the statistics and the base blocks lie in shared memory (floats)
   int tpr;              // warp tiles per row of the block grid
   long long ntiles;
 };
 
-template <int W, int NW>
-__global__ void __launch_bounds__(32 * NW, kXWarpsPerSM / NW)
-    ncc_xlane_kernel(NccArgs a, XArgs xa, const __grid_constant__ CUtensorMap tmap) {
+// The candidate planes of group g: P from cz0 = min(g P, W - P); the group
+// scores those from cz0 up to the next group's first.
+template <int W, int P>
+struct XGroups {
+  static constexpr int N = (W + P - 1) / P;
+  static __device__ __forceinline__ int first(int g) { return min(g * P, W - P); }
+  static __device__ __forceinline__ int scored(int g) {
+    return (g + 1 < N ? first(g + 1) : W) - first(g);
+  }
+};
+
+// Window plane D (0 .. P + 2) of a group: its E rows (rp, rp + rpu, ...) read
+// once each, shifted by -c and fed to the candidate planes j with base plane
+// vz = D - j in 0 .. 3.
+template <int W, int P, int D>
+__device__ __forceinline__ void xlane_plane(f32x2 (&acc)[P][W], const f32x2 (&t)[32],
+                                            const float *rp, int rpu, f32x2 mc, float (&nx)[4]) {
+  constexpr int E = W + 3;
+#pragma unroll
+  for (int wy = 0; wy < E; ++wy) {
+    const f32x2 r[2] = {add2(pack2(nx[0], nx[1]), mc), add2(pack2(nx[2], nx[3]), mc)};
+    rp += rpu;
+    if (!(D == P + 2 && wy == E - 1)) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) nx[i] = rp[i];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < P; ++j)
+#pragma unroll
+        for (int vy = 0; vy < 4; ++vy) {
+          const int vz = D - j, cy = wy - vy;
+          if (vz < 0 || vz > 3 || cy < 0 || cy >= W) continue;
+          acc[j][cy] = fma2(t[(vz * 4 + vy) * 2 + h], r[h], acc[j][cy]);
+        }
+  }
+}
+template <int W, int P, int D = 0>
+__device__ __forceinline__ void xlane_group(f32x2 (&acc)[P][W], const f32x2 (&t)[32],
+                                            const float *rp, int rpu, f32x2 mc, float (&nx)[4]) {
+  xlane_plane<W, P, D>(acc, t, rp, rpu, mc, nx);
+  if constexpr (D + 1 < P + 3) xlane_group<W, P, D + 1>(acc, t, rp + (W + 3) * rpu, rpu, mc, nx);
+}
+
+// RPU > 0: the union row pitch known at compile time (every shared-memory
+// offset of the loop is a constant then); 0: xa.rpu.
+template <int W, int P, int NW, int RPU>
+__global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
+    ncc_xlane_kernel(NccArgs a, XArgs xa, const __grid_constant__ CUtensorMap tmap,
+                     const __grid_constant__ CUtensorMap smap) {
+  using Groups = XGroups<W, P>;
   constexpr int R = W / 2, E = W + 3, NL = 32 * NW, BPW = NL / W;
+  const int rpu = RPU > 0 ? RPU : xa.rpu;
   extern __shared__ __align__(16) float sm[];
-  __shared__ __align__(8) uint64_t s_bar;
-  // the tensor copy's destination starts on 128 bytes (the allocation has 128 spare)
+  __shared__ __align__(8) uint64_t s_bar, s_sbar;
+  // the tensor copies' destinations start on 128 bytes (the allocation has 128 spare)
   float *const sma = reinterpret_cast<float *>(
       sm + ((128u - ((unsigned int)__cvta_generic_to_shared(sm) & 127u)) & 127u) / sizeof(float));
   float *win = sma;                     // E * E * rpu
-  float *xt = sma + E * E * xa.rpu;     // BPW * 64
-  float2 *qbuf = reinterpret_cast<float2 *>(xt + BPW * 64);  // NL * W
+  float2 *sst = reinterpret_cast<float2 *>(sma + xa.soff);  // P * W * spu: a group's statistics
+  float *xt = sma + xa.xoff;            // BPW * kXtPitch
   __shared__ float s_red[BPW][W][2];
   __shared__ int s_deg[BPW][W][2];
   __shared__ float s_f[BPW][2];
@@ -1224,10 +1328,14 @@ __global__ void __launch_bounds__(32 * NW, kXWarpsPerSM / NW)
   const int lane = threadIdx.x;
   const int k = lane / W, x = lane - k * W;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
-  if (lane == 0) mbar_init(&s_bar, 1);
+  if (lane == 0) {
+    mbar_init(&s_bar, 1);
+    mbar_init(&s_sbar, 1);
+  }
   __syncthreads();
-  unsigned int phase = 0;
-  const unsigned int win_bytes = (unsigned int)(E * E * xa.rpu * sizeof(float));
+  unsigned int phase = 0, sphase = 0;
+  const unsigned int win_bytes = (unsigned int)(E * E * rpu * sizeof(float));
+  const unsigned int st_bytes = (unsigned int)(P * W * xa.spu * sizeof(float2));
 
   for (long long tile = blockIdx.x; tile < xa.ntiles; tile += gridDim.x) {
     const long long grow = tile / xa.tpr;
@@ -1241,13 +1349,27 @@ __global__ void __launch_bounds__(32 * NW, kXWarpsPerSM / NW)
     const int ox0 = a.stx + bx0 * a.G - R;
     const int ox = ox0 + k * a.G;
     const int xu = ox0 & ~3;             // union origin, rounded down to 16 bytes
+    const int xs = ox0 & ~1;             // the statistics', likewise
+    // every global read of the set-up is issued before the first is used: the
+    // block's record, flags, and the tile's base blocks (lane v loads voxel v
+    // of each block)
+    static_assert(NL == 64, "one lane per voxel of a base block");
+    const BlockStat st = a.bstat[b];
+    const bool sel = !a.selected || a.selected[b], window_in = xa.wand[b] != 0;
+    float xv[BPW];
+    double mv[BPW];
+    {
+      const float *q = a.base + lin(a, ox0 + R + (lane & 3), oy + R + ((lane >> 2) & 3),
+                                    oz + R + (lane >> 4));
+#pragma unroll
+      for (int i = 0; i < BPW; ++i) {
+        xv[i] = i < nbt ? __ldg(q + i * a.G) : 0.f;
+        mv[i] = a.bstat[brow + bx0 + (i < nbt ? i : 0)].mean;
+      }
+    }
     // ---- routing ----------------------------------------------------------
     int state = 0;
-    BlockStat st;
-    st.mean = 0.0; st.sxx = 0.f; st.sxt = 0.f; st.mmode = 0; st.c = 0.f;
     if (mine) {
-      st = a.bstat[b];
-      const bool sel = !a.selected || a.selected[b];
       if (!sel) {
         if (x == 0) {
           write_final(a, b, -3.f, -3.f, lin(a, ox + R, oy + R, oz + R), 0);
@@ -1268,13 +1390,9 @@ __global__ void __launch_bounds__(32 * NW, kXWarpsPerSM / NW)
     // ---- window inside the search mask? -----------------------------------
     const int px = ox + x;
     const bool xok = px >= 0 && px <= nx - 4;
-    unsigned yok = 0;
-#pragma unroll
-    for (int cy = 0; cy < W; ++cy)
-      if (oy + cy >= 0 && oy + cy <= ny - 4) yok |= 1u << cy;
     // a partly masked window sends the block (all of its lanes read the same
     // flag) to the masked kernel
-    if (state && !xa.wand[b]) {
+    if (state && !window_in) {
       if (x == 0) {
         unsigned int p = atomicAdd(&a.ctl[4], 1u);
         a.gen_list[a.nblocks + 1 + p] = (int)b;
@@ -1284,149 +1402,148 @@ __global__ void __launch_bounds__(32 * NW, kXWarpsPerSM / NW)
     if (!__syncthreads_or(state)) continue;
     // ---- staging: the union window by one tensor copy (zero outside the
     // volume), the base blocks (x~) by the lanes meanwhile --------------------
-    const int rpu = xa.rpu;
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // earlier reads of win
     __syncthreads();
     if (lane == 0) {
       mbar_expect_tx(&s_bar, win_bytes);
       tma_load_3d(win, &tmap, xu, oy, oz, &s_bar);
+      mbar_expect_tx(&s_sbar, st_bytes);
+      tma_load_3d(reinterpret_cast<float *>(sst), &smap, xs, oy, oz, &s_sbar);
     }
-    for (int i = lane; i < nbt * 64; i += NL) {
-      const int kk = i >> 6, v = i & 63;
-      const int vx = v & 3, vy = (v >> 2) & 3, vz = v >> 4;
-      const long long q = ((long long)(oz + R + vz) * ny + (oy + R + vy)) * nx +
-                          (ox0 + kk * a.G + R + vx);
-      const double mk = a.bstat[brow + bx0 + kk].mean;
-      xt[i] = (float)__dsub_rn((double)__ldg(&a.base[q]), mk);
-    }
-    // the give-up decision is the CTA's, so no thread is left at a barrier
-    const bool landed = mbar_wait(&s_bar, phase, 1 << 22);
-    if (__syncthreads_or(!landed)) {
-      if (lane == 0) atomicExch(&a.ctl[5], 1u);
-      return;
-    }
+#pragma unroll
+    for (int i = 0; i < BPW; ++i)
+      xt[i * kXtPitch + lane] = (float)__dsub_rn((double)xv[i], mv[i]);
+    // a wait that gives up is the CTA's decision, taken at a barrier, so no
+    // thread is left at one
+    bool gave_up = !mbar_wait(&s_bar, phase, 1 << 22);
     phase ^= 1u;
     __syncthreads();
     // ---- FP32 scores ---------------------------------------------------------
     float l1 = -3.f, l2 = -3.f;
-    int d1 = -1, d2 = -1;
     const int E_rpu = E * rpu;
     {
       // every thread runs the plane loop (it holds CTA barriers); a lane
       // without a block computes on its own placeholder data and writes nothing
       const bool real = state != 0;
-      float t[64];
-      const float4 *tp = reinterpret_cast<const float4 *>(xt + (real ? k : 0) * 64);
+      f32x2 t[32];
+      const float4 *tp = reinterpret_cast<const float4 *>(xt + (real ? k : 0) * kXtPitch);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float4 q = tp[i];
-        t[4 * i] = q.x; t[4 * i + 1] = q.y; t[4 * i + 2] = q.z; t[4 * i + 3] = q.w;
+        t[2 * i] = pack2(q.x, q.y);
+        t[2 * i + 1] = pack2(q.z, q.w);
       }
       const float c = st.c, sxt = st.sxt, sxx = st.sxx;
-      const float rsxx = sxx > 0.f ? 1.f / sxx : 0.f;
-      float2 *qb = qbuf + lane * W;
-      const float2 *st0 = a.stats + (((long long)oz * ny + oy) * nx + px);
+      const f32x2 mc = pack2(-c, -c);
+      // (finite for a sum below the normal range: its candidates then tie at 0 and
+      // the block is re-scored in FP64)
+      const float rsxx = sxx > 0.f ? fminf(1.f / sxx, FLT_MAX) : 0.f;
       const float *rp = win + (real ? ox - xu : 0) + x;
-      // acc[j]: candidate plane cz = wz - 3 + j.  Window plane wz feeds the
-      // planes wz - 3 .. wz (j = 3 - vz); planes outside 0 .. W-1, fed at the
-      // first and last three window planes, are never scored.
-      float acc[4][W];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int cy = 0; cy < W; ++cy) acc[j][cy] = 0.f;
+      const float2 *sl = sst + (real ? ox - xs : 0) + x;
+      float *scp = win + lane * W;
+      const bool live = real && xok, flat = sxx <= 0.f;
 #pragma unroll 1
-      for (int wz = 0; wz < E; ++wz) {
-        const int cz = wz - 3;
-        const bool zok = real && cz >= 0 && xok && oz + cz >= 0 && oz + cz <= nz - 4;
-        if (zok) {
-          // statistics of the plane completed below, fetched meanwhile
+      for (int g = 0; g < Groups::N; ++g) {
+        const int cz0 = Groups::first(g), ns = Groups::scored(g);
+        f32x2 acc[P][W];
 #pragma unroll
-          for (int cy = 0; cy < W; ++cy)
-            if ((yok >> cy) & 1u) cp_async8(qb + cy, st0 + ((long long)cz * ny + cy) * nx);
-          asm volatile("cp.async.commit_group;\n" ::: "memory");
-        }
+        for (int j = 0; j < P; ++j)
 #pragma unroll
-        for (int wy = 0; wy < E; ++wy) {
-          float r[4];
+          for (int cy = 0; cy < W; ++cy) acc[j][cy] = 0ULL;
+        const float *gp = rp + cz0 * E_rpu;
+        float nx4[4] = {gp[0], gp[1], gp[2], gp[3]};
+        xlane_group<W, P>(acc, t, gp, rpu, mc, nx4);
+        __syncthreads();  // window planes cz0 .. cz0 + ns - 1 are read by every warp
+        if (gave_up || !mbar_wait(&s_sbar, sphase, 1 << 22)) gave_up = true;
+        sphase ^= 1u;
 #pragma unroll
-          for (int vx = 0; vx < 4; ++vx) r[vx] = rp[vx] - c;
-          rp += rpu;
-#pragma unroll
-          for (int vx = 0; vx < 4; ++vx)
-#pragma unroll
-            for (int vz = 0; vz < 4; ++vz)
-#pragma unroll
-              for (int vy = 0; vy < 4; ++vy) {
-                const int cy = wy - vy;
-                if (cy < 0 || cy >= W) continue;
-                acc[3 - vz][cy] = fmaf(t[(vz * 4 + vy) * 4 + vx], r[vx], acc[3 - vz][cy]);
+        for (int j = 0; j < P; ++j) {
+          const int cz = cz0 + j;
+          if (j < ns && live && (unsigned)(oz + cz) <= (unsigned)(nz - 4)) {
+            float *sc = scp + cz * E_rpu;
+            const float2 *sj = sl + j * W * xa.spu;
+            if (flat) {  // every candidate of the block is degenerate
+#pragma unroll 1
+              for (int cy = 0; cy < W; ++cy) {
+                const float s = (unsigned)(oy + cy) <= (unsigned)(ny - 4) ? -2.f : -FLT_MAX;
+                top2_push(l1, l2, s);
+                sc[cy] = s;
               }
-        }
-        if (cz >= 0) {
-          // window plane cz was read three planes ago by every warp: its rows
-          // now hold the scores of candidate plane cz (lane-major, W per lane)
-          __syncthreads();
-          if (zok) {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            float *sc = win + cz * E_rpu + lane * W;
-            const long long prow = ((long long)(oz + cz) * ny + oy) * nx + px;
+              continue;
+            }
 #pragma unroll
             for (int cy = 0; cy < W; ++cy) {
-              if (!((yok >> cy) & 1u)) continue;
-              const float2 q = qb[cy];
-              const float sxy = acc[0][cy] - (q.x - c) * sxt;
-              const float s = (sxx <= 0.f || q.y <= 0.f) ? -2.f : __fdividef(sxy * sxy * rsxx, q.y);
+              const float2 q = sj[cy * xa.spu];
+              const float sxy = sum2(acc[j][cy]) - (q.x - c) * sxt;
+              // NaN (not a candidate: a row outside the volume) ranks lowest
+              float s = fmaxf(sxy * sxy * rsxx * q.y, -FLT_MAX);
+              if (q.y <= 0.f) s = -2.f;
               top2_push(l1, l2, s);
-              if (s == -2.f) push_deg(d1, d2, (int)(prow + (long long)cy * nx));
               sc[cy] = s;
             }
           }
         }
-        // rotate: plane wz - 3 is done, plane wz + 1 starts
-#pragma unroll
-        for (int cy = 0; cy < W; ++cy) {
-          acc[0][cy] = acc[1][cy];
-          acc[1][cy] = acc[2][cy];
-          acc[2][cy] = acc[3][cy];
-          acc[3][cy] = 0.f;
+        if (g + 1 < Groups::N) {
+          __syncthreads();  // the statistics are read
+          if (lane == 0) {
+            mbar_expect_tx(&s_sbar, st_bytes);
+            tma_load_3d(reinterpret_cast<float *>(sst), &smap, xs, oy, oz + Groups::first(g + 1),
+                        &s_sbar);
+          }
         }
       }
     }
     // ---- block-level reduction and refinement list --------------------------
     if (state) {
-      s_red[k][x][0] = l1; s_red[k][x][1] = l2;
-      s_deg[k][x][0] = d1; s_deg[k][x][1] = d2;
+      s_red[k][x][0] = l1;
+      s_red[k][x][1] = l2;
     }
-    __syncthreads();
+    if (__syncthreads_or(gave_up)) {
+      if (lane == 0) atomicExch(&a.ctl[5], 1u);
+      return;
+    }
     if (state && x == 0) {
       float f1 = -3.f, f2 = -3.f;
-      int e1 = -1, e2 = -1;
-      for (int j = 0; j < W; ++j) {
-        top2_merge(f1, f2, s_red[k][j][0], s_red[k][j][1]);
-        min2_merge(e1, e2, s_deg[k][j][0], s_deg[k][j][1]);
-      }
-      s_f[k][0] = f1; s_f[k][1] = f2;
-      s_deg[k][0][0] = e1; s_deg[k][0][1] = e2;
+#pragma unroll
+      for (int j = 0; j < W; ++j) top2_merge(f1, f2, s_red[k][j][0], s_red[k][j][1]);
+      s_f[k][0] = f1;
+      s_f[k][1] = f2;
     }
     __syncthreads();
     if (state && xok) {
-      // candidates within 2 delta of the block's FP32 second-best
-      const float T2 = s_f[k][1] - 2.f * kDelta;
+      // candidates within 2 delta of the block's FP32 second-best (a plane's
+      // largest score first: few planes hold one)
+      const float f2 = s_f[k][1];
+      const float T2 = fmaxf(f2 - 2.f * kDelta, -1.999999f);
+      // fewer than two candidates are not degenerate (rare): the lane's first
+      // two degenerate ones in raster order
+      int d1 = -1, d2 = -1;
       for (int cz = 0; cz < W; ++cz) {
-        if (oz + cz < 0 || oz + cz > nz - 4) continue;
+        if ((unsigned)(oz + cz) > (unsigned)(nz - 4)) continue;
         const float *sc = win + cz * E_rpu + lane * W;
-        const long long prow = ((long long)(oz + cz) * ny + oy) * nx + px;
+        float v[W], m = -FLT_MAX;
 #pragma unroll
         for (int cy = 0; cy < W; ++cy) {
-          if (!((yok >> cy) & 1u)) continue;
-          const float sv = sc[cy];
-          if (sv > -2.f && sv >= T2) {
-            const int pos = atomicAdd(&s_cnt[k], 1);
-            if (pos < kK) s_list[k][pos] = (int)(prow + (long long)cy * nx);
-          }
+          v[cy] = sc[cy];
+          m = fmaxf(m, v[cy]);
+        }
+        const long long prow = ((long long)(oz + cz) * ny + oy) * nx + px;
+        if (f2 <= -2.f) {
+#pragma unroll
+          for (int cy = 0; cy < W; ++cy)
+            if (v[cy] == -2.f) push_deg(d1, d2, (int)(prow + (long long)cy * nx));
+        }
+        if (m >= T2) {
+#pragma unroll
+          for (int cy = 0; cy < W; ++cy)
+            if (v[cy] >= T2) {
+              const int pos = atomicAdd(&s_cnt[k], 1);
+              if (pos < kK) s_list[k][pos] = (int)(prow + (long long)cy * nx);
+            }
         }
       }
+      s_deg[k][x][0] = d1;
+      s_deg[k][x][1] = d2;
     }
     __syncthreads();
     if (state && x == 0) {
@@ -1438,8 +1555,14 @@ __global__ void __launch_bounds__(32 * NW, kXWarpsPerSM / NW)
       if (cnt <= kK) {
         for (int j = 0; j < cnt; ++j) rc.p[j] = s_list[k][j];
         if (f2 <= -2.f) {
-          if (s_deg[k][0][0] >= 0) rc.p[cnt++] = s_deg[k][0][0];
-          if (s_deg[k][0][1] >= 0) rc.p[cnt++] = s_deg[k][0][1];
+          int e1 = -1, e2 = -1;
+          for (int j = 0; j < W; ++j) {
+            // (lanes outside the volume took no part)
+            if ((unsigned)(ox + j) <= (unsigned)(nx - 4))
+              min2_merge(e1, e2, s_deg[k][j][0], s_deg[k][j][1]);
+          }
+          if (e1 >= 0) rc.p[cnt++] = e1;
+          if (e2 >= 0) rc.p[cnt++] = e2;
         }
       }
       rc.cnt = cnt;
@@ -1555,10 +1678,10 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
           }
           continue;
         }
-        float2 st = __ldg(&a.stats[p]);
+        float2 st = __ldg(&a.stats[sidx(a, px, py, pz)]);
         const float mu = st.x;
         const int woff = ((cz * a.g) * w.ey + cy * a.g) * w.ex + cx * a.g;
-        float sxy = 0.f, sxx, syy;
+        float sxy = 0.f, sxx, syy = 1.f, rsyy = 1.f;
         if (fast) {
           float acc = 0.f;
 #pragma unroll
@@ -1570,7 +1693,7 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
                 acc = fmaf(xt[(vz * BW + vy) * BW + vx], yw[woff + (vz * w.ey + vy) * w.ex + vx], acc);
           sxy = acc - mu * bst.sxt;
           sxx = bst.sxx;
-          syy = syy_of(st.y);
+          rsyy = rsyy_of(st.y);
         } else {
           float ax = 0.f, ay = 0.f;
 #pragma unroll
@@ -1590,9 +1713,11 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
                 }
               }
           sxx = ax;
-          syy = bst.mmode == 1 ? syy_of(st.y) : ay;
+          if (bst.mmode == 1) rsyy = rsyy_of(st.y);
+          else syy = ay;
         }
-        float s = (sxx <= 0.f || syy <= 0.f) ? -2.f : (sxy * sxy) / sxx / syy;
+        float s = (sxx <= 0.f || syy <= 0.f || rsyy <= 0.f) ? -2.f
+                                                              : (sxy * sxy) / sxx / syy * rsyy;
         top2_merge(l1, l2, s, -3.f);
         if (s == -2.f) push_deg(d1, d2, (int)p);
         scs[c] = s;
@@ -1910,25 +2035,51 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-template <int W, class CM>
+// 3D tensor map of nx x ny x nz elements with rows of `pitch` elements, and
+// boxes of bx x by x bz, filled as `fill` says beyond the extents.
+mirorr_status encode_map3(CUtensorMap *map, CUtensorMapDataType type, int elem, const void *p,
+                          int nx, int ny, int nz, int pitch, int bx, int by, int bz,
+                          CUtensorMapFloatOOBfill fill) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled is not available from the driver");
+    return MIRORR_ECUDA;
+  }
+  const cuuint64_t gdim[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
+  const cuuint64_t gstride[2] = {(cuuint64_t)pitch * elem, (cuuint64_t)pitch * ny * elem};
+  const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, type, 3, const_cast<void *>(p), gdim, gstride, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, fill);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return MIRORR_ECUDA;
+  }
+  return MIRORR_OK;
+}
+
+template <int W, int P, int RPU, class CM>
 mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
                            cudaEvent_t *kev) {
   constexpr int E = W + 3, NL = 32 * kXWarps, BPW = NL / W;
   done = false;
   const long long u = (long long)(BPW - 1) * a.G + E;   // union row length
   XArgs xa;
-  xa.nch = (int)((u + 6) / 4);
-  xa.rpu = 4 * xa.nch;
+  xa.rpu = 4 * (int)((u + 6) / 4);
   // each window plane must hold one plane of scores (W per lane) once read
   const int min_rpu = ((BPW * W * W + E - 1) / E + 3) & ~3;
-  if (xa.rpu < min_rpu) {
-    xa.rpu = min_rpu;
-    xa.nch = min_rpu / 4;
-  }
+  if (xa.rpu < min_rpu) xa.rpu = min_rpu;
+  const bool fixed = xa.rpu <= RPU;  // block spacings up to 4
+  if (fixed) xa.rpu = RPU;
+  xa.spu = (int)(((long long)(BPW - 1) * a.G + W + 2) & ~1LL);
+  xa.soff = (E * E * xa.rpu + 31) & ~31;
+  xa.xoff = xa.soff + 2 * P * W * xa.spu;
   xa.tpr = (a.nbx + BPW - 1) / BPW;
   xa.ntiles = (long long)xa.tpr * a.nby * a.nbz;
-  const size_t smem = sizeof(float) * ((size_t)E * E * xa.rpu + BPW * 64 + 2 * NL * W) + 128;
-  if (xa.rpu > 256 || smem > 64 * 1024) return MIRORR_OK;  // tensor box limit
+  const size_t smem = sizeof(float) * ((size_t)xa.xoff + BPW * kXtPitch) + 128;
+  // tensor box limit
+  if (xa.rpu > 256 || xa.spu > 256 || smem > 64 * 1024) return MIRORR_OK;
   // rows of the search image must start on 16 bytes for the 16-byte copies
   a.search_al = a.search;
   a.spitch = a.nx;
@@ -1946,7 +2097,7 @@ mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
     MB2_TRY(w.ncc_wand.ensure(n1 + n2 + (size_t)a.nblocks));
     uint8_t *b1 = w.ncc_wand.as<uint8_t>(), *b2 = b1 + n1, *b3 = b2 + n2;
     const unsigned g = (unsigned)sm_count() * 8;
-    wand_x_kernel<<<g, 256, 0, s>>>(a.stats, b1, a.nx, a.ny, a.nz, a.nbx, a.stx, a.G, W, 4);
+    wand_x_kernel<<<g, 256, 0, s>>>(a.stats, a.sp, b1, a.nx, a.ny, a.nz, a.nbx, a.stx, a.G, W, 4);
     MB2_LAUNCH_CHECK();
     wand_axis_kernel<<<g, 256, 0, s>>>(b1, b2, a.nbx, a.ny, a.nz, a.nby, a.sty, a.G, W);
     MB2_LAUNCH_CHECK();
@@ -1955,33 +2106,19 @@ mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
     MB2_LAUNCH_CHECK();
     xa.wand = b3;
   }
-  // tensor map of the search image: x extent nx (zero beyond), rows of spitch floats
-  CUtensorMap tmap;
-  {
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) {
-      set_error("cuTensorMapEncodeTiled is not available from the driver");
-      return MIRORR_ECUDA;
-    }
-    const cuuint64_t gdim[3] = {(cuuint64_t)a.nx, (cuuint64_t)a.ny, (cuuint64_t)a.nz};
-    const cuuint64_t gstride[2] = {(cuuint64_t)a.spitch * sizeof(float),
-                                   (cuuint64_t)a.spitch * a.ny * sizeof(float)};
-    const cuuint32_t box[3] = {(cuuint32_t)xa.rpu, (cuuint32_t)E, (cuuint32_t)E};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(a.search_al),
-                     gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-      set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
-      return MIRORR_ECUDA;
-    }
-  }
-  MB2_TRY(set_smem(ncc_xlane_kernel<W, kXWarps>, smem));
-  const long long kCtas = (long long)sm_count() * (kXWarpsPerSM / kXWarps);
+  // tensor maps of the search image and of the statistics: x extent nx (zero
+  // beyond), rows of spitch floats and of sp float2
+  CUtensorMap tmap, smap;
+  MB2_TRY(encode_map3(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.search_al, a.nx, a.ny, a.nz,
+                      a.spitch, xa.rpu, E, E, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+  MB2_TRY(encode_map3(&smap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, a.stats, a.nx, a.ny, a.nz, a.sp,
+                      xa.spu, W, P, CU_TENSOR_MAP_FLOAT_OOB_FILL_NAN_REQUEST_ZERO_FMA));
+  auto kernel = fixed ? ncc_xlane_kernel<W, P, kXWarps, RPU> : ncc_xlane_kernel<W, P, kXWarps, 0>;
+  MB2_TRY(set_smem(kernel, smem));
+  const long long kCtas = (long long)sm_count() * kXCtasPerSM;
   const long long grid = xa.ntiles < kCtas ? xa.ntiles : kCtas;
   if (kev) MB2_CUDA_TRY(cudaEventRecord(kev[0], s));
-  ncc_xlane_kernel<W, kXWarps><<<(unsigned)grid, NL, smem, s>>>(a, xa, tmap);
+  kernel<<<(unsigned)grid, NL, smem, s>>>(a, xa, tmap, smap);
   MB2_LAUNCH_CHECK();
   if (kev) MB2_CUDA_TRY(cudaEventRecord(kev[1], s));
   MB2_TRY((launch_masked<CM>(a, s)));
@@ -1997,7 +2134,7 @@ bool run_fast(NccArgs &a, BmWork &w, cudaStream_t s, mirorr_status &st, cudaEven
   if ((long long)a.nx * a.ny * a.nz >= (1LL << 31)) return false;
   if (a.bw == 4 && a.W == 9) {
     bool done = false;
-    st = launch_xlane<9, FastCfg<4, 9, 1, 3>>(a, w, s, done, kev);
+    st = launch_xlane<9, 3, 48, FastCfg<4, 9, 1, 3>>(a, w, s, done, kev);
     xl_ran = done;
     if (st != MIRORR_OK || done) return true;
     st = launch_fast<WarpCfg<4, 9, 3, 1, 5, 3>, FastCfg<4, 9, 1, 3>>(a, s);
@@ -2005,11 +2142,17 @@ bool run_fast(NccArgs &a, BmWork &w, cudaStream_t s, mirorr_status &st, cudaEven
   }
   if (a.bw == 4 && a.W == 7) {
     bool done = false;
-    st = launch_xlane<7, FastCfg<4, 7, 1, 5>>(a, w, s, done, kev);
+    st = launch_xlane<7, 4, 48, FastCfg<4, 7, 1, 5>>(a, w, s, done, kev);
     xl_ran = done;
     if (st != MIRORR_OK || done) return true;
     st = launch_fast<WarpCfg<4, 7, 4, 2, 4, 3>, FastCfg<4, 7, 1, 5>>(a, s);
     return true;
+  }
+  if (a.bw == 4 && a.W == 5) {
+    bool done = false;
+    st = launch_xlane<5, 5, 56, FastCfg<4, 5, 1, 10>>(a, w, s, done, kev);
+    xl_ran = done;
+    return st != MIRORR_OK || done;
   }
   if (a.bw == 5 && a.W == 11) {
     st = launch_fast<WarpCfg<5, 11, 6, 1, 4, 2>, FastCfg<5, 11, 1, 2>>(a, s);
@@ -2040,6 +2183,7 @@ mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmas
                                sizeof(unsigned int) * (w.ncc_ctl.ptr == ctl_before ? 5 : 8), s));
   NccArgs a;
   a.base = base; a.bmask = bmask; a.search = search; a.smask = smask; a.stats = stats;
+  a.sp = stats_pitch(g.size[0]);
   a.selected = selected;
   a.bstat = w.ncc_bstat.as<BlockStat>();
   a.nx = g.size[0]; a.ny = g.size[1]; a.nz = g.size[2];
@@ -2083,24 +2227,6 @@ mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmas
       set_error("block width %d not supported (1..8)", g.bw);
       return MIRORR_EINVAL;
   }
-}
-
-mirorr_status launch_window_and(const BmGeom &g, const float2 *stats, DevBuf &buf,
-                                const uint8_t **wand, cudaStream_t s) {
-  const int nx = g.size[0], ny = g.size[1], nz = g.size[2];
-  const size_t n1 = (size_t)g.nb[0] * ny * nz, n2 = (size_t)g.nb[0] * g.nb[1] * nz;
-  MB2_TRY(buf.ensure(n1 + n2 + (size_t)g.nblocks));
-  uint8_t *b1 = buf.as<uint8_t>(), *b2 = b1 + n1, *b3 = b2 + n2;
-  const unsigned grid = (unsigned)sm_count() * 8;
-  wand_x_kernel<<<grid, 256, 0, s>>>(stats, b1, nx, ny, nz, g.nb[0], g.st[0], g.ngap, g.nw, g.bw);
-  MB2_LAUNCH_CHECK();
-  wand_axis_kernel<<<grid, 256, 0, s>>>(b1, b2, g.nb[0], ny, nz, g.nb[1], g.st[1], g.ngap, g.nw);
-  MB2_LAUNCH_CHECK();
-  wand_axis_kernel<<<grid, 256, 0, s>>>(b2, b3, (long long)g.nb[0] * g.nb[1], nz, 1, g.nb[2],
-                                        g.st[2], g.ngap, g.nw);
-  MB2_LAUNCH_CHECK();
-  *wand = b3;
-  return MIRORR_OK;
 }
 
 const unsigned int *ncc_timeout_flag(const BmWork &w) {
