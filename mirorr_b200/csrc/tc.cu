@@ -157,39 +157,6 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 }
 
-// Running best / second over a multiset of (score, raster index): best is
-// the largest score, ties to the smallest index; second the largest of the
-// rest.  Equal to the reference's sequential strict update in raster order.
-struct Top2 {
-  float b1, b2;
-  long long i1;
-};
-__device__ __forceinline__ void top2_add(Top2 &t, float s, long long i) {
-  if (s > t.b1 || (s == t.b1 && i < t.i1)) {
-    t.b2 = t.b1;
-    t.b1 = s;
-    t.i1 = i;
-  } else {
-    t.b2 = fmaxf(t.b2, s);
-  }
-}
-__device__ __forceinline__ void top2_merge(Top2 &t, const Top2 &u) {
-  if (u.b1 > t.b1 || (u.b1 == t.b1 && u.i1 < t.i1)) {
-    t.b2 = fmaxf(t.b1, fmaxf(t.b2, u.b2));
-    t.b1 = u.b1;
-    t.i1 = u.i1;
-  } else {
-    t.b2 = fmaxf(t.b2, fmaxf(u.b1, u.b2));
-  }
-}
-__device__ __forceinline__ Top2 top2_shfl_xor(const Top2 &t, int m) {
-  Top2 u;
-  u.b1 = __shfl_xor_sync(0xffffffffu, t.b1, m);
-  u.b2 = __shfl_xor_sync(0xffffffffu, t.b2, m);
-  u.i1 = __shfl_xor_sync(0xffffffffu, t.i1, m);
-  return u;
-}
-
 __device__ __forceinline__ void write_out(const Args16 &a, long long b, float best, float second,
                                           long long match, uint8_t status) {
   a.best[b] = best;
@@ -496,8 +463,8 @@ __global__ void __launch_bounds__(256) prep16_kernel(const Args16 *calls) {
 
 // Base-block preparation for other block widths (no tensor form): one warp
 // per block, lane l < BW^2 holds base row (vz, vy) = (l / BW, l % BW); the
-// FP32 mean, the masked sums of x~ and x~^2, the base-mask mode and the
-// block's route (culled, or the direct search's list).  grid.y = call.
+// FP32 mean, the masked sums of x~ and x~^2 and the base-mask mode of every
+// block that is searched (each goes to the direct search's list).  grid.y = call.
 template <typename T, int BW>
 __global__ void __launch_bounds__(256) prep16w_kernel(const Args16 *calls) {
   static_assert(BW * BW <= 32, "one warp per block");
@@ -509,62 +476,77 @@ __global__ void __launch_bounds__(256) prep16w_kernel(const Args16 *calls) {
   const int nx = a.nx, ny = a.ny;
   const int lane = threadIdx.x & 31;
   const bool row = lane < BW * BW;
+  constexpr unsigned rows_mask = (BW * BW == 32) ? 0xffffffffu : ((1u << (BW * BW)) - 1u);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long b = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); b < a.nblocks;
-       b += nwarps) {
-    int bx, by, bz;
-    split3(b, a.nbx, a.nby, bx, by, bz);
-    const int ox = a.stx + bx * a.G, oy = a.sty + by * a.G, oz = a.stz + bz * a.G;
-    float v[BW];
-    unsigned mbits = 0;
-    float sum = 0.f;
-    if (row) {
-      const long long q = ((long long)(oz + lane / BW) * ny + (oy + lane % BW)) * nx + ox;
-#pragma unroll
-      for (int i = 0; i < BW; ++i) {
-        v[i] = S16<T>::f(x[q + i]);
-        mbits |= (mb[q + i] != 0 ? 1u : 0u) << i;
-        sum += v[i];
-      }
+  // a warp takes 32 consecutive blocks: the culled ones are written by a lane
+  // each, and the others are listed with one addition to the list's counter
+  // (one per block made that counter the bound: 2.65 ms for 0.7 of 2.4 million
+  // blocks, 0.76 ms now)
+  for (long long b0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+       b0 < a.nblocks; b0 += nwarps * 32) {
+    const bool live = b0 + lane < a.nblocks;
+    const bool sel = live && (!a.selected || a.selected[b0 + lane]);
+    if (live && !sel) {
+      int bx, by, bz;
+      split3(b0 + lane, a.nbx, a.nby, bx, by, bz);
+      write_out(a, b0 + lane, -3.f, -3.f,
+                ((long long)(a.stz + bz * a.G) * ny + (a.sty + by * a.G)) * nx + (a.stx + bx * a.G), 0);
     }
+    const unsigned todo = __ballot_sync(0xffffffffu, sel);
+    if (!todo) continue;
+    unsigned int at = 0;
+    if (lane == 0) at = atomicAdd(&a.ctl[1], (unsigned)__popc(todo));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (sel) a.fb_list[at + __popc(todo & ((1u << lane) - 1u))] = (int)(b0 + lane);
+    for (unsigned left = todo; left; left &= left - 1) {
+      const long long b = b0 + (__ffs(left) - 1);
+      int bx, by, bz;
+      split3(b, a.nbx, a.nby, bx, by, bz);
+      const int ox = a.stx + bx * a.G, oy = a.sty + by * a.G, oz = a.stz + bz * a.G;
+      float v[BW];
+      unsigned mbits = 0;
+      float sum = 0.f;
+      if (row) {
+        const long long q = ((long long)(oz + lane / BW) * ny + (oy + lane % BW)) * nx + ox;
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float mu = sum * (1.0f / NB);
-    float sxx = 0.f, sxt = 0.f;
-    if (row) {
-#pragma unroll
-      for (int i = 0; i < BW; ++i) {
-        const float d = v[i] - mu;
-        if ((mbits >> i) & 1u) {
-          sxx = fmaf(d, d, sxx);
-          sxt += d;
+        for (int i = 0; i < BW; ++i) {
+          v[i] = S16<T>::f(x[q + i]);
+          mbits |= (mb[q + i] != 0 ? 1u : 0u) << i;
+          sum += v[i];
         }
       }
-    }
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      sxx += __shfl_xor_sync(0xffffffffu, sxx, o);
-      sxt += __shfl_xor_sync(0xffffffffu, sxt, o);
-    }
-    constexpr unsigned rows_mask = (BW * BW == 32) ? 0xffffffffu : ((1u << (BW * BW)) - 1u);
-    const unsigned full = __ballot_sync(0xffffffffu, row && mbits == (1u << BW) - 1u) & rows_mask;
-    const unsigned none = __ballot_sync(0xffffffffu, row && mbits == 0u) & rows_mask;
-    if (lane == 0) {
-      Prep16 pp;
-      pp.mu = mu;
-      pp.sxx = sxx;
-      pp.sxt = sxt;
-      pp.sxt_tc = 0.f;
-      pp.mmode = full == rows_mask ? 1 : (none == rows_mask ? 2 : 0);
-      pp.route = 0;
-      pp.pad[0] = pp.pad[1] = 0;
-      if (a.selected && !a.selected[b]) {
-        write_out(a, b, -3.f, -3.f, ((long long)oz * ny + oy) * nx + ox, 0);
-      } else {
-        const unsigned int k = atomicAdd(&a.ctl[1], 1u);
-        a.fb_list[k] = (int)b;
+      for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      const float mu = sum * (1.0f / NB);
+      float sxx = 0.f, sxt = 0.f;
+      if (row) {
+#pragma unroll
+        for (int i = 0; i < BW; ++i) {
+          const float d = v[i] - mu;
+          if ((mbits >> i) & 1u) {
+            sxx = fmaf(d, d, sxx);
+            sxt += d;
+          }
+        }
       }
-      a.prep[b] = pp;
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) {
+        sxx += __shfl_xor_sync(0xffffffffu, sxx, o);
+        sxt += __shfl_xor_sync(0xffffffffu, sxt, o);
+      }
+      const unsigned full = __ballot_sync(0xffffffffu, row && mbits == (1u << BW) - 1u) & rows_mask;
+      const unsigned none = __ballot_sync(0xffffffffu, row && mbits == 0u) & rows_mask;
+      if (lane == 0) {
+        Prep16 pp;
+        pp.mu = mu;
+        pp.sxx = sxx;
+        pp.sxt = sxt;
+        pp.sxt_tc = 0.f;
+        pp.mmode = full == rows_mask ? 1 : (none == rows_mask ? 2 : 0);
+        pp.route = 0;
+        pp.pad[0] = pp.pad[1] = 0;
+        a.prep[b] = pp;
+      }
     }
   }
 }
@@ -631,7 +613,9 @@ __device__ __forceinline__ TilePos tile_pos(const Args16 *calls, int ncalls, lon
 
 // Top two over a thread's or a block's candidates with a 32-bit raster key
 // (tile-local: (dz * 8 + py) * 8 + x shift; raster order of the candidates
-// of one block), same rule as Top2.
+// of one block): best is the largest score, ties to the smallest key; second
+// the largest of the rest.  Equal to the reference's sequential strict update
+// in raster order.
 struct Top2k {
   float b1, b2;
   int k1;
@@ -1145,39 +1129,76 @@ __global__ void __launch_bounds__(kWsThreads, 1)
 
 // ---------------------------------------------------------------------------
 // Direct FP32 search for the blocks the tensor form does not take (each
-// call's fb_list; block width 5 takes every block here): one CTA per block.
-// The window (at most 16^3 values) and the base block are staged in shared
-// memory; window rows are 18 floats apart and planes 16 x 18 + 6, so the
-// rows the threads of a warp read (11 strips per plane at window 11) start on
-// distinct bank pairs and a row is read with 8-byte loads.  Thread t owns the x strip of candidates at
-// (py, pz) = (t % ncy, t / ncy): per base row (vy, vz) it reads the window row
-// once and updates all its candidates' cross terms from registers, in the
-// raster order of the base block, so each candidate's sum is the one a
-// per-candidate loop forms (windows of more than 128 strips deal them
-// round-robin).  A candidate whose footprint lies inside the
-// search mask with the base block inside its mask is scored from that cross
-// term and the box statistics (Syy); any other candidate is re-summed with
-// the masked sums of the reference formula.  grid.y = call.
+// call's fb_list; block width 5 takes every block here): one CTA per block,
+// grid.y = call.
+//
+// The window and the centred base block are staged in shared memory.  Thread t
+// owns the x strip of candidates at (py, pz) = (t % ncy, t / ncy): per base row
+// (vy, vz) it reads the window row once and updates all its candidates' cross
+// terms from registers, in the raster order of the base block, so each
+// candidate's sum is the one a per-candidate loop forms.  A candidate whose
+// footprint lies inside the search mask with the base block inside its mask is
+// scored from that cross term and the box statistics (Syy).  The others (their
+// footprint straddles the mask's edge, or the base block is partly masked) are
+// listed, and the CTA's threads share the list: per candidate the masked sums
+// over the voxels that both masks keep, found from a word of mask bits per
+// window row and per base row.
+//
+// What bounds it is instruction issue beside the latency of a block's staging,
+// so the strip is as long as the launch's windows (NCX = 7 or 11; else the
+// longest), a CTA has about as many threads as a block has strips, a block
+// wholly inside both masks stages no mask, and a block whose every candidate is
+// degenerate is written at once.  Measured: block 5, window
+// 11 (512 x 512 x 256 FP16, 0.73 M blocks) 20.0 -> 12.6 ms (19.3 TFLOP/s of
+// cross terms); block 4, window 7 on the partly masked blocks of eight
+// registrations' calls 2.84 -> 0.98 ms.
+//
+// Window rows are RS floats apart and planes PS, RS / 4 odd and PS equal to ncy
+// rows modulo the banks, so the rows that eight consecutive threads read start
+// on distinct 16-byte bank groups and are read with 16-byte loads; base rows are
+// padded to 16 bytes as well.
 // ---------------------------------------------------------------------------
-template <typename T, int BW>
-__global__ void __launch_bounds__(128, 8) ncc_fb16_kernel(const Args16 *calls) {
-  constexpr int NT = 128;
-  constexpr int NB = BW * BW * BW;
-  constexpr int RS = 18;             // window row stride (floats)
-  constexpr int PS = 16 * RS + 6;    // window plane stride (floats)
-  constexpr int NCX = 16 - BW + 1;   // longest x strip (window extent <= 16)
-  __shared__ float s_xt[NB], s_mb[NB];
-  __shared__ __align__(16) float s_y[16 * PS];
-  __shared__ uint8_t s_m[16 * PS];
-  __shared__ Top2 s_red[NT / 32];
+__device__ __forceinline__ uint8_t ld_global(const uint8_t *p) { return __ldg(p); }
+__device__ __forceinline__ __half ld_global(const __half *p) { return __ldg(p); }
+__device__ __forceinline__ __nv_bfloat16 ld_global(const __nv_bfloat16 *p) { return __ldg(p); }
+
+template <int BW_, int NCX_>
+struct FbCfg {
+  static constexpr int BW = BW_, NCX = NCX_;      // block width, longest x strip
+  static constexpr int NB = BW * BW * BW;
+  static constexpr int EX = NCX + BW - 1;         // window extent
+  static constexpr int NT = NCX <= 7 ? 64 : 128;  // threads
+  static constexpr int NV = (EX + 3) / 4 * 4;     // values read of a row
+  static constexpr int RS = NV % 8 == 4 ? NV : NV + 4;
+  static constexpr int XR = (BW + 3) / 4 * 4;     // floats per base row
+  static constexpr int PS = EX * RS + ((NCX - EX) * RS % 32 + 32) % 32;
+  static constexpr int CPS = NT == 64 ? 12 : 7;   // CTAs per SM aimed for
+  static_assert(NT / 16 <= EX, "a step crosses one plane at most");
+  static_assert(RS % 8 == 4 && PS % 4 == 0 && (PS - NCX * RS) % 32 == 0, "bank layout");
+};
+
+template <typename T, class C>
+__global__ void __launch_bounds__(C::NT, C::CPS) ncc_fb16_kernel(const Args16 *calls) {
+  constexpr int NT = C::NT, BW = C::BW, NB = C::NB, NCX = C::NCX, EX = C::EX, NV = C::NV;
+  constexpr int RS = C::RS, PS = C::PS, XR = C::XR, NGRP = NT / 16;
+  __shared__ __align__(16) float s_xt[BW * BW * XR];
+  __shared__ __align__(16) float s_y[EX * PS];
+  __shared__ uint16_t s_bits[EX * EX];   // search-mask bits of the window rows
+  __shared__ uint8_t s_mb[BW * BW];      // base-mask bits of the base rows
+  __shared__ uint16_t s_list[NCX * NCX * NCX];  // pz << 8 | py << 4 | px
+  __shared__ int s_n;
+  __shared__ Top2k s_red[NT / 32];
   const Args16 &a = calls[blockIdx.y];
   if (!a.active) return;
   const int tid = threadIdx.x;
   const T *base = static_cast<const T *>(a.base);
   const T *search = static_cast<const T *>(a.search);
   const unsigned int nlist = *(volatile unsigned int *)&a.ctl[1];
+  long long b_next = blockIdx.x < nlist ? a.fb_list[blockIdx.x] : 0;
+  unsigned long long scored = 0;  // candidates of this CTA's blocks
   for (unsigned int li = blockIdx.x; li < nlist; li += gridDim.x) {
-    const long long b = a.fb_list[li];
+    const long long b = b_next;
+    if (li + gridDim.x < nlist) b_next = a.fb_list[li + gridDim.x];
     int bx, by, bz;
     split3(b, a.nbx, a.nby, bx, by, bz);
     const int ox = a.stx + bx * a.G, oy = a.sty + by * a.G, oz = a.stz + bz * a.G;
@@ -1187,130 +1208,197 @@ __global__ void __launch_bounds__(128, 8) ncc_fb16_kernel(const Args16 *calls) {
     cand_range(oz, a.nz, a.W, BW, zlo, zhi);
     const int ncx = xhi - xlo + 1, ncy = yhi - ylo + 1, ncz = zhi - zlo + 1;
     const int ex = ncx + BW - 1, ey = ncy + BW - 1, ez = ncz + BW - 1;
+    const int nc = ncx > 0 && ncy > 0 && ncz > 0 ? ncx * ncy * ncz : 0;
     const Prep16 pp = a.prep[b];
-    __syncthreads();
+    const bool full = pp.mmode == 1 && wand_of(a)[b] != 0;
+    if (nc == 0 || pp.mmode == 2 || (pp.mmode == 1 && pp.sxx <= 0.f)) {
+      // no candidate, or Sxx = 0 for every one of them (all degenerate)
+      if (tid == 0) {
+        if (nc == 0) write_out(a, b, -3.f, -3.f, ((long long)oz * a.ny + oy) * a.nx + ox, 1);
+        else
+          write_out(a, b, -2.f, nc > 1 ? -2.f : -3.f,
+                    ((long long)zlo * a.ny + ylo) * a.nx + xlo, 1);
+      }
+      scored += nc;
+      continue;
+    }
+    __syncthreads();  // the previous block's shared state is read
+    if (tid == 0) s_n = 0;
     for (int t = tid; t < NB; t += NT) {
       const int vx = t % BW, vy = (t / BW) % BW, vz = t / (BW * BW);
-      const long long qq = ((long long)(oz + vz) * a.ny + (oy + vy)) * a.nx + (ox + vx);
-      const float mv = a.bmask[qq] != 0 ? 1.f : 0.f;
-      s_xt[t] = S16<T>::f(base[qq]) - pp.mu;
-      s_mb[t] = mv;
+      s_xt[(t / BW) * XR + vx] = S16<T>::f(base[((long long)(oz + vz) * a.ny + (oy + vy)) * a.nx + (ox + vx)]) - pp.mu;
+    }
+    if (!full && tid < BW * BW) {
+      const uint8_t *m = a.bmask + ((long long)(oz + tid / BW) * a.ny + (oy + tid % BW)) * a.nx + ox;
+      unsigned k = 0;
+#pragma unroll
+      for (int vx = 0; vx < BW; ++vx) k |= (m[vx] != 0 ? 1u : 0u) << vx;
+      s_mb[tid] = (uint8_t)k;
     }
     {
-      // a 16-lane group per window row (ex <= 16); the group's row (wy, wz)
-      // advances by NT / 16 rows without a division
-      const int wx = tid & 15;
-      int wy = tid >> 4, wz = ncx > 0 && ncy > 0 && ncz > 0 ? 0 : ez;  // empty window: none
-      while (wz < ez && wy >= ey) {
-        wy -= ey;
-        ++wz;
-      }
-      // four rows per pass, all of their loads issued before the stores
-      while (wz < ez) {
-        T yv[4];
-        uint8_t mv[4];
-        int so[4];
+      // a 16-lane group per window row, SR rows per pass with all of their
+      // loads issued before the stores.  Rows are numbered EX to a plane, a
+      // group takes every NGRP-th, and moves to the next by fixed steps.
+      constexpr int SR = 8;
+      const int wx = tid & 15, nrow = ez * EX;
+      int r = tid >> 4, wy = r, so = r * RS + wx;
+      long long q = ((long long)zlo * a.ny + ylo + wy) * a.nx + xlo + wx;
+      const long long dq = (long long)NGRP * a.nx, dqz = dq + (long long)(a.ny - EX) * a.nx;
+      const bool xin = wx < ex;
+      for (int r0 = 0; r0 < nrow; r0 += SR * NGRP) {
+        T yv[SR];
+        uint8_t mv[SR];
+        int sv[SR];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          so[j] = -1;
-          if (wz < ez && wx < ex) {
-            const long long qq = ((long long)(zlo + wz) * a.ny + (ylo + wy)) * a.nx + (xlo + wx);
-            yv[j] = search[qq];
-            mv[j] = a.smask[qq];
-            so[j] = wz * PS + wy * RS + wx;
+        for (int j = 0; j < SR; ++j) {
+          sv[j] = -1;
+          if (xin && r < nrow && wy < ey) {
+            sv[j] = so;
+            yv[j] = ld_global(search + q);
+            if (!full) mv[j] = ld_global(a.smask + q);
           }
-          wy += NT / 16;
-          while (wz < ez && wy >= ey) {
-            wy -= ey;
-            ++wz;
+          r += NGRP;
+          wy += NGRP;
+          so += NGRP * RS;
+          const bool wrap = wy >= EX;
+          q += wrap ? dqz : dq;
+          if (wrap) {
+            wy -= EX;
+            so += PS - EX * RS;
           }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (so[j] >= 0) {
-            s_y[so[j]] = S16<T>::f(yv[j]);
-            s_m[so[j]] = mv[j] != 0 ? 1 : 0;
+        for (int j = 0; j < SR; ++j)
+          if (sv[j] >= 0) s_y[sv[j]] = S16<T>::f(yv[j]);
+        if (!full) {
+#pragma unroll
+          for (int j = 0; j < SR; ++j) {
+            const unsigned bal = __ballot_sync(0xffffffffu, sv[j] >= 0 && mv[j] != 0);
+            const int rj = r - (SR - j) * NGRP;
+            if (wx == 0 && rj < nrow) s_bits[rj] = (uint16_t)(bal >> (tid & 16));
           }
+        }
       }
     }
     __syncthreads();
-    Top2 tp;
+    Top2k tp;
     tp.b1 = -3.f;
     tp.b2 = -3.f;
-    tp.i1 = 0x7fffffffffffffffLL;
-    const int nc = ncx * ncy * ncz;
-    for (int strip = tid; strip < ncy * ncz; strip += NT) {
-      const int py = strip % ncy, pz = strip / ncy;
-      const int cy = ylo + py, cz = zlo + pz;
-      // the strip's cross terms (base block inside its mask only)
-      float acc[NCX];
+    tp.k1 = 0x7fffffff;
+    auto add = [&](float sc, int key) {
+      if (sc > tp.b1 || (sc == tp.b1 && key < tp.k1)) {
+        tp.b2 = tp.b1;
+        tp.b1 = sc;
+        tp.k1 = key;
+      } else {
+        tp.b2 = fmaxf(tp.b2, sc);
+      }
+    };
+    if (pp.mmode == 1) {
+      for (int strip = tid; strip < ncy * ncz; strip += NT) {
+        const int pz = strip / ncy, py = strip - pz * ncy;
+        float acc[NCX];
 #pragma unroll
-      for (int px = 0; px < NCX; ++px) acc[px] = 0.f;
-      if (pp.mmode == 1) {
+        for (int px = 0; px < NCX; ++px) acc[px] = 0.f;
         for (int vz = 0; vz < BW; ++vz)
 #pragma unroll
           for (int vy = 0; vy < BW; ++vy) {
             // values past the window's extent only feed strip positions
             // px >= ncx, which are not scored
-            const float2 *row = reinterpret_cast<const float2 *>(s_y + (pz + vz) * PS + (py + vy) * RS);
-            float r[16];
+            const float4 *row = reinterpret_cast<const float4 *>(s_y + (pz + vz) * PS + (py + vy) * RS);
+            const float4 *xrow = reinterpret_cast<const float4 *>(s_xt + (vz * BW + vy) * XR);
+            float r[NV], t[XR];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float2 q = row[k];
-              r[2 * k] = q.x;
-              r[2 * k + 1] = q.y;
+            for (int k = 0; k < XR / 4; ++k) {
+              const float4 q = xrow[k];
+              t[4 * k] = q.x; t[4 * k + 1] = q.y; t[4 * k + 2] = q.z; t[4 * k + 3] = q.w;
             }
-            float t[BW];
 #pragma unroll
-            for (int vx = 0; vx < BW; ++vx) t[vx] = s_xt[(vz * BW + vy) * BW + vx];
+            for (int k = 0; k < NV / 4; ++k) {
+              const float4 q = row[k];
+              r[4 * k] = q.x; r[4 * k + 1] = q.y; r[4 * k + 2] = q.z; r[4 * k + 3] = q.w;
+            }
 #pragma unroll
             for (int px = 0; px < NCX; ++px)
 #pragma unroll
               for (int vx = 0; vx < BW; ++vx) acc[px] = fmaf(t[vx], r[px + vx], acc[px]);
           }
-      }
+        const float2 *st = a.stats + ((long long)(zlo + pz) * a.ny + (ylo + py)) * a.sp + xlo;
+        const int key = (pz << 8) | (py << 4);
 #pragma unroll
-      for (int px = 0; px < NCX; ++px) {
-        if (px >= ncx) break;
-        const int cx = xlo + px;
-        const long long idx = ((long long)cz * a.ny + cy) * a.nx + cx;
-        const float2 st = __ldg(a.stats + ((long long)cz * a.ny + cy) * a.sp + cx);
-        const float muy = st.x;
-        float sxy = 0.f, sxx = 0.f, syy = 0.f;
-        if (pp.mmode == 1 && !signbit(st.y)) {
-          // footprint and base block wholly inside their masks
-          sxy = acc[px] - muy * pp.sxt;
-          sxx = pp.sxx;
-          syy = st.y;
-        } else {
-#pragma unroll 5
-          for (int i = 0; i < NB; ++i) {
-            const int vx = i % BW, vy = (i / BW) % BW, vz = i / (BW * BW);
-            const int w = (pz + vz) * PS + (py + vy) * RS + px + vx;
-            const float mk = s_mb[i] * (float)s_m[w];
-            const float dy = s_y[w] - muy;
-            const float xm = mk * s_xt[i];
-            sxy = fmaf(xm, dy, sxy);
-            sxx = fmaf(xm, s_xt[i], sxx);
-            syy = fmaf(mk * dy, dy, syy);
+        for (int px = 0; px < NCX; ++px) {
+          if (px >= ncx) break;
+          const float2 q = __ldg(st + px);
+          if (full || !signbit(q.y)) {
+            // footprint and base block wholly inside their masks; a thread's
+            // keys grow, so an equal score never replaces
+            const float sxy = acc[px] - q.x * pp.sxt;
+            const float sc = q.y <= 0.f ? -2.f : __fdividef(sxy * sxy, pp.sxx * q.y);
+            const bool up = sc > tp.b1;
+            tp.b2 = up ? tp.b1 : fmaxf(tp.b2, sc);
+            tp.b1 = up ? sc : tp.b1;
+            tp.k1 = up ? key + px : tp.k1;
+          } else {
+            s_list[atomicAdd(&s_n, 1)] = (uint16_t)(key + px);
           }
         }
-        const float sc = (sxx <= 0.f || syy <= 0.f) ? -2.f : __fdividef(sxy * sxy, sxx * syy);
-        top2_add(tp, sc, idx);
+      }
+    }
+    if (!full) {
+      __syncthreads();
+      const bool listed = pp.mmode == 1;
+      const int n = listed ? s_n : nc;
+      for (int i = tid; i < n; i += NT) {
+        int px, py, pz;
+        if (listed) {
+          const int k = s_list[i];
+          px = k & 15;
+          py = (k >> 4) & 15;
+          pz = k >> 8;
+        } else {
+          const int k = i / ncx;
+          px = i - k * ncx;
+          pz = k / ncy;
+          py = k - pz * ncy;
+        }
+        const float muy = __ldg(a.stats + ((long long)(zlo + pz) * a.ny + (ylo + py)) * a.sp + xlo + px).x;
+        float sxy = 0.f, sxx = 0.f, syy = 0.f;
+        for (int vz = 0; vz < BW; ++vz)
+#pragma unroll
+          for (int vy = 0; vy < BW; ++vy) {
+            const unsigned pat = ((unsigned)s_bits[(pz + vz) * EX + py + vy] >> px) & s_mb[vz * BW + vy];
+            if (pat == 0) continue;
+            const float *yr = s_y + (pz + vz) * PS + (py + vy) * RS + px;
+            const float *xr = s_xt + (vz * BW + vy) * XR;
+#pragma unroll
+            for (int vx = 0; vx < BW; ++vx) {
+              const bool in = (pat >> vx) & 1u;
+              const float x = in ? xr[vx] : 0.f, dy = in ? yr[vx] - muy : 0.f;
+              sxy = fmaf(x, dy, sxy);
+              sxx = fmaf(x, x, sxx);
+              syy = fmaf(dy, dy, syy);
+            }
+          }
+        add((sxx <= 0.f || syy <= 0.f) ? -2.f : __fdividef(sxy * sxy, sxx * syy),
+            (pz << 8) | (py << 4) | px);
       }
     }
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) top2_merge(tp, top2_shfl_xor(tp, o));
+    for (int o = 1; o < 32; o <<= 1) top2k_merge(tp, top2k_shfl_xor(tp, o));
     if ((tid & 31) == 0) s_red[tid >> 5] = tp;
     __syncthreads();
     if (tid == 0) {
-      for (int w = 1; w < NT / 32; ++w) top2_merge(tp, s_red[w]);
-      const long long orig = ((long long)oz * a.ny + oy) * a.nx + ox;
-      if (nc > 0) write_out(a, b, tp.b1, tp.b2, tp.i1, 1);
-      else write_out(a, b, -3.f, -3.f, orig, 1);
-      if (a.ncc_count) atomicAdd(a.ncc_count, (unsigned long long)nc);
+      for (int w = 1; w < NT / 32; ++w) top2k_merge(tp, s_red[w]);
+      const int k = tp.k1;
+      write_out(a, b, tp.b1, tp.b2,
+                k == 0x7fffffff ? -1  // every score is NaN
+                                : ((long long)(zlo + (k >> 8)) * a.ny + (ylo + ((k >> 4) & 15))) * a.nx +
+                                      xlo + (k & 15),
+                1);
     }
+    scored += nc;
   }
+  if (tid == 0 && scored && a.ncc_count) atomicAdd(a.ncc_count, scored);
 }
 
 // ---------------------------------------------------------------------------
@@ -1446,7 +1534,7 @@ mirorr_status run16(int ncalls, Match16Call *host_calls, DevBuf &calls_dev, cuda
   MB2_TRY(match16_prepare_copies(S16<T>::kFmt == 1 ? MIRORR_DTYPE_BF16 : MIRORR_DTYPE_F16, host_calls,
                                  ncalls));
   long long max_vox = 0, max_blocks = 0, max_chunks = 0;
-  int W = 0, G = 0, BWc = 0;
+  int W = 0, G = 0, BWc = 0, max_w = 0;
   bool any_tensor = false;
   for (int i = 0; i < ncalls; ++i) {
     const Match16Call &c = host_calls[i];
@@ -1467,6 +1555,7 @@ mirorr_status run16(int ncalls, Match16Call *host_calls, DevBuf &calls_dev, cuda
       G = c.G;
     }
     if (!c.active) continue;
+    max_w = std::max(max_w, c.W);
     max_vox = std::max(max_vox, (long long)c.nx * c.ny * c.nz);
     max_blocks = std::max(max_blocks, c.nblocks);
     max_chunks = std::max(max_chunks, (long long)c.nxc * c.nz * c.ny);
@@ -1523,8 +1612,20 @@ mirorr_status run16(int ncalls, Match16Call *host_calls, DevBuf &calls_dev, cuda
       MB2_LAUNCH_CHECK();
     }
   }
-  if (BWc == 5) ncc_fb16_kernel<T, 5><<<dim3((unsigned)SM * 8, (unsigned)ncalls), 128, 0, s>>>(dc);
-  else ncc_fb16_kernel<T, 4><<<dim3((unsigned)SM * 8, (unsigned)ncalls), 128, 0, s>>>(dc);
+  {
+    auto direct = [&](auto cfg) {
+      using C = decltype(cfg);
+      ncc_fb16_kernel<T, C><<<dim3((unsigned)(SM * C::CPS), (unsigned)ncalls), C::NT, 0, s>>>(dc);
+    };
+    // the strip length by the launch's largest window
+    if (BWc == 5) {
+      if (max_w <= 11) direct(FbCfg<5, 11>{});
+      else direct(FbCfg<5, 12>{});
+    } else {
+      if (max_w <= 7) direct(FbCfg<4, 7>{});
+      else direct(FbCfg<4, 13>{});
+    }
+  }
   MB2_LAUNCH_CHECK();
   return MIRORR_OK;
 }
