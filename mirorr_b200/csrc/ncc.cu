@@ -1793,6 +1793,7 @@ __device__ double exact_score(const NccArgs &a, const float *x, const uint8_t *m
 template <int BW>
 __global__ void __launch_bounds__(128) ncc_refine_kernel(NccArgs a) {
   constexpr int B = BW * BW * BW;
+  unsigned int scored = 0, refined = 0;  // this thread's candidates
   for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < a.nblocks;
        b += (long long)gridDim.x * blockDim.x) {
     NccRec rc = a.rec[b];
@@ -1890,21 +1891,48 @@ __global__ void __launch_bounds__(128) ncc_refine_kernel(NccArgs a) {
       for (int i = 0; i < n; ++i) r.push(exact_score<BW>(a, x, mb, mean_b, rc.p[i]), rc.p[i]);
     }
     write_final(a, b, r.best, r.second, r.arg < 0 ? lin(a, w.sx, w.sy, w.sz) : r.arg, 1);
-    if (a.ncc_count) atomicAdd(a.ncc_count, (unsigned long long)w.nc);
-    atomicAdd(&a.ctl[2], (unsigned int)n);
+    scored += w.nc;
+    refined += n;
+  }
+  // one addition per warp: one per block, all to one address, was a bound
+  scored = __reduce_add_sync(0xffffffffu, scored);
+  refined = __reduce_add_sync(0xffffffffu, refined);
+  if ((threadIdx.x & 31) == 0 && refined) {
+    if (a.ncc_count) atomicAdd(a.ncc_count, (unsigned long long)scored);
+    atomicAdd(&a.ctl[2], refined);
   }
 }
 
 // ---------------------------------------------------------------------------
-// Fallback: every candidate of an overflowed block re-scored in FP64.
+// Fallback: every candidate of an overflowed block re-scored in FP64, one CTA
+// per block.  Overflow is the lot of blocks with few voxels inside both masks
+// (every candidate scores nearly 1) and of near-constant regions, so a masked
+// call has thousands of them.  STAGED: the window is held in shared memory (it
+// is read once per candidate and voxel otherwise) with its mask as one word of
+// bits per row; windows beyond 21 a side are read from global memory.
+// Measured (219 x 203 x 107, W = 7, both masks, 5,362 blocks): 1.44 ms with one
+// CTA per SM, candidates read from global memory and the sequential update in
+// one thread; 0.16 ms now.
 // ---------------------------------------------------------------------------
-template <int BW>
+constexpr int kFbStageMax = 21;
+constexpr int kFbCtasPerSM = 8;
+
+size_t fallback_smem(int emax, size_t cmax, int B, bool staged) {
+  return sizeof(double) * (cmax + B) +
+         (staged ? sizeof(float) * emax * emax * emax + sizeof(unsigned) * emax * emax : 0) + 16;
+}
+
+template <int BW, bool STAGED>
 __global__ void __launch_bounds__(128) ncc_fallback_kernel(NccArgs a) {
   constexpr int B = BW * BW * BW;
   extern __shared__ __align__(16) unsigned char smem[];
   double *ex = reinterpret_cast<double *>(smem);  // W^3
+  double *xb = ex + a.W * a.W * a.W;              // B: x - mean
+  float *yw = reinterpret_cast<float *>(xb + B);  // window
+  unsigned *yb = reinterpret_cast<unsigned *>(yw + a.emax * a.emax * a.emax);  // mask bits of its rows
   __shared__ float xs[B];
   __shared__ uint8_t mbs[B];
+  __shared__ unsigned s_mrow[BW * BW];            // base-mask bits per base row
   __shared__ double s_mean;
   const int tid = threadIdx.x;
   const unsigned int n = *(volatile unsigned int *)&a.ctl[1];
@@ -1920,26 +1948,95 @@ __global__ void __launch_bounds__(128) ncc_fallback_kernel(NccArgs a) {
       xs[v] = __ldg(&a.base[q]);
       mbs[v] = __ldg(&a.bmask[q]);
     }
+    if constexpr (STAGED) {
+      const long long wo = lin(a, w.sx, w.sy, w.sz);
+      const int rows = w.ey * w.ez, lane = tid & 31;
+      for (int r = tid >> 5; r < rows; r += 4) {
+        const int wz = r / w.ey, wy = r - wz * w.ey;
+        const long long q = wo + ((long long)wz * a.ny + wy) * a.nx + lane;
+        bool m = false;
+        if (lane < w.ex) {
+          yw[(wz * a.emax + wy) * a.emax + lane] = __ldg(&a.search[q]);
+          m = __ldg(&a.smask[q]) != 0;
+        }
+        const unsigned bits = __ballot_sync(0xffffffffu, m);
+        if (lane == 0) yb[wz * a.emax + wy] = bits;
+      }
+    }
     __syncthreads();
     if (tid == 0) {
       double sum = 0.0;
+#pragma unroll
       for (int v = 0; v < B; ++v) sum = __dadd_rn(sum, (double)xs[v]);
       s_mean = __ddiv_rn(sum, (double)B);
     }
-    __syncthreads();
-    for (int c = tid; c < w.nc; c += blockDim.x) {
-      int cx = c % w.nx, cy = (c / w.nx) % w.ny, cz = c / (w.nx * w.ny);
-      ex[c] = exact_score<BW>(a, xs, mbs, s_mean,
-                              lin(a, w.sx + cx * a.g, w.sy + cy * a.g, w.sz + cz * a.g));
+    if (STAGED && tid >= 32 && tid < 32 + BW * BW) {
+      unsigned m = 0;
+      for (int vx = 0; vx < BW; ++vx) m |= (mbs[(tid - 32) * BW + vx] ? 1u : 0u) << vx;
+      s_mrow[tid - 32] = m;
     }
     __syncthreads();
-    if (tid == 0) {
-      SeqTop2 r;
-      for (int c = 0; c < w.nc; ++c) r.push(ex[c], c);
-      int c = r.arg < 0 ? 0 : r.arg;
+    if constexpr (STAGED) {
+      for (int v = tid; v < B; v += blockDim.x) xb[v] = __dsub_rn((double)xs[v], s_mean);
+      __syncthreads();
+    }
+    for (int c = tid; c < w.nc; c += blockDim.x) {
       int cx = c % w.nx, cy = (c / w.nx) % w.ny, cz = c / (w.nx * w.ny);
-      write_final(a, b, r.best, r.second, lin(a, w.sx + cx * a.g, w.sy + cy * a.g, w.sz + cz * a.g), 1);
-      if (a.ncc_count) atomicAdd(a.ncc_count, (unsigned long long)w.nc);
+      if constexpr (STAGED) {
+        // exact_score's sums in its order; a voxel outside the masks adds nothing
+        const int wo = (cz * a.g * a.emax + cy * a.g) * a.emax + cx * a.g;
+        double ms = 0.0;
+        for (int vz = 0; vz < BW; ++vz)
+#pragma unroll
+          for (int vy = 0; vy < BW; ++vy)
+#pragma unroll
+            for (int vx = 0; vx < BW; ++vx)
+              ms = __dadd_rn(ms, (double)yw[wo + (vz * a.emax + vy) * a.emax + vx]);
+        ms = __ddiv_rn(ms, (double)B);
+        double prod = 0.0, bss = 0.0, sss = 0.0;
+        for (int vz = 0; vz < BW; ++vz)
+#pragma unroll
+          for (int vy = 0; vy < BW; ++vy) {
+            const unsigned m = (yb[(cz * a.g + vz) * a.emax + cy * a.g + vy] >> (cx * a.g)) &
+                               s_mrow[vz * BW + vy];
+            if (!m) continue;
+#pragma unroll
+            for (int vx = 0; vx < BW; ++vx)
+              if ((m >> vx) & 1u) {
+                const double bb = xb[(vz * BW + vy) * BW + vx];
+                const double sb = __dsub_rn((double)yw[wo + (vz * a.emax + vy) * a.emax + vx], ms);
+                prod = __dadd_rn(prod, __dmul_rn(bb, sb));
+                bss = __dadd_rn(bss, __dmul_rn(bb, bb));
+                sss = __dadd_rn(sss, __dmul_rn(sb, sb));
+              }
+          }
+        ex[c] = (bss <= 0.0 || sss <= 0.0)
+                    ? -2.0 : __ddiv_rn(__ddiv_rn(__dmul_rn(prod, prod), bss), sss);
+      } else {
+        ex[c] = exact_score<BW>(a, xs, mbs, s_mean,
+                                lin(a, w.sx + cx * a.g, w.sy + cy * a.g, w.sz + cz * a.g));
+      }
+    }
+    __syncthreads();
+    if (tid < 32) {
+      // the sequential update, by one warp: best and second only grow (and
+      // second <= best), so of 32 candidates only those above the second at
+      // hand can change them, and those are taken in order
+      SeqTop2 r;
+      for (int c0 = 0; c0 < w.nc; c0 += 32) {
+        const double m = c0 + tid < w.nc ? ex[c0 + tid] : -4.0;
+        for (unsigned hot = __ballot_sync(0xffffffffu, (double)r.second < m); hot; hot &= hot - 1) {
+          const int l = __ffs(hot) - 1;
+          r.push(__shfl_sync(0xffffffffu, m, l), c0 + l);
+        }
+      }
+      if (tid == 0) {
+        int c = r.arg < 0 ? 0 : r.arg;
+        int cx = c % w.nx, cy = (c / w.nx) % w.ny, cz = c / (w.nx * w.ny);
+        write_final(a, b, r.best, r.second,
+                    lin(a, w.sx + cx * a.g, w.sy + cy * a.g, w.sz + cz * a.g), 1);
+        if (a.ncc_count) atomicAdd(a.ncc_count, (unsigned long long)w.nc);
+      }
     }
   }
 }
@@ -1991,14 +2088,16 @@ mirorr_status launch_rest(const NccArgs &a, bool all_general, cudaStream_t s) {
   constexpr int B = BW * BW * BW;
   const size_t e3 = (size_t)a.emax * a.emax * a.emax, cmax = (size_t)a.W * a.W * a.W;
   size_t smem_g = sizeof(float) * (B + e3 + cmax) + B + e3 + 16;
-  size_t smem_f = sizeof(double) * cmax + 16;
+  const bool staged = a.emax <= kFbStageMax;
+  const size_t smem_f = fallback_smem(a.emax, cmax, B, staged);
   if (smem_g > 200 * 1024 || smem_f > 200 * 1024) {
     set_error("search window too large for shared memory (window %d^3, %d candidates)",
               a.emax, (int)cmax);
     return MIRORR_EINVAL;
   }
   MB2_TRY(set_smem(ncc_general_kernel<BW>, smem_g));
-  MB2_TRY(set_smem(ncc_fallback_kernel<BW>, smem_f));
+  auto fallback = staged ? ncc_fallback_kernel<BW, true> : ncc_fallback_kernel<BW, false>;
+  MB2_TRY(set_smem(fallback, smem_f));
   if (all_general) {
     // no register-blocked kernels for this geometry: every block here
     long long grid = a.nblocks < (long long)sm_count() * 16 ? a.nblocks : (long long)sm_count() * 16;
@@ -2008,7 +2107,7 @@ mirorr_status launch_rest(const NccArgs &a, bool all_general, cudaStream_t s) {
   long long rgrid = (a.nblocks + 127) / 128;
   ncc_refine_kernel<BW><<<(unsigned)rgrid, 128, 0, s>>>(a);
   MB2_LAUNCH_CHECK();
-  ncc_fallback_kernel<BW><<<(unsigned)sm_count(), 128, smem_f, s>>>(a);
+  fallback<<<(unsigned)(sm_count() * kFbCtasPerSM), 128, smem_f, s>>>(a);
   MB2_LAUNCH_CHECK();
   return MIRORR_OK;
 }
