@@ -357,17 +357,27 @@ struct FastCfg {
   static constexpr int TPB = W * NYG;                  // threads per block
   static constexpr int NT = ((BPC * TPB + 31) / 32) * 32;
   static constexpr int NC = W * W * W;                 // candidates per block
-  static constexpr int NROW = E * EY;                  // window rows per block
-  static constexpr int NPAT = 1 << BW;                 // mask patterns of one base row
-  static constexpr int NTAB = BW * BW * NPAT;          // table entries per block
-  // dynamic shared memory, in floats: windows, base blocks, row bits, tables
-  static constexpr int OFF_XT = BPC * WIN;
-  static constexpr int OFF_BITS = OFF_XT + ((BPC * B + 3) & ~3);
-  static constexpr int OFF_TAB = OFF_BITS + ((BPC * NROW + 3) & ~3);
-  static constexpr int SMEM_FLOATS = OFF_TAB + 2 * BPC * NTAB;
   static_assert(WIN % 4 == 0 && EXP % 4 == 0 && PS % 4 == 0 && B > 0, "alignment");
   static_assert(2 * NC <= WIN, "scores and straddler list reuse the window");
-  static_assert(E <= 16 && EY <= NT / 16 && NT % 32 == 0, "a window plane fits the CTA");
+  static_assert(E <= 16 && NT % 32 == 0, "a window row fits 16 lanes");
+};
+
+// The masked-window kernel's tile.  One block per CTA: its nine barriers a tile
+// then wait for two or three warps, not eight (397 -> 303 us with the staging
+// of stage_rows at 219 x 203 x 107, W = 7, masks; 5 or 3 blocks per CTA 325 us).
+template <int BW_, int W_>
+struct MaskedCfg : FastCfg<BW_, W_, 1, 1> {
+  using F = FastCfg<BW_, W_, 1, 1>;
+  static constexpr int NROW = F::E * F::EY;            // window rows per block
+  static constexpr int NPAT = 1 << BW_;                // mask patterns of one base row
+  static constexpr int NTAB = BW_ * BW_ * NPAT;        // table entries per block
+  // dynamic shared memory, in floats: windows, base blocks, row bits, tables
+  static constexpr int OFF_XT = F::BPC * F::WIN;
+  static constexpr int OFF_BITS = OFF_XT + ((F::BPC * F::B + 3) & ~3);
+  static constexpr int OFF_TAB = OFF_BITS + ((F::BPC * NROW + 3) & ~3);
+  static constexpr int SMEM_FLOATS = OFF_TAB + 2 * F::BPC * NTAB;
+  // resident CTAs per SM aimed for (64 registers a thread)
+  static constexpr int MINB = F::NT <= 64 ? 16 : (F::NT <= 96 ? 10 : 8);
 };
 
 // Shared state of the per-block reduction that ends a CTA tile.
@@ -409,18 +419,21 @@ __device__ void finish_tile(const NccArgs &a, TileTail<C::BPC, C::TPB> &tt, cons
       if (!s_state[wp]) continue;
       float f1 = -3.f, f2 = -3.f;
       int e1 = -1, e2 = -1;
-      for (int k = ln; k < TPB; k += 32) {
-        top2_merge(f1, f2, tt.red[wp][k][0], tt.red[wp][k][1]);
-        min2_merge(e1, e2, tt.deg[wp][k][0], tt.deg[wp][k][1]);
-      }
+      for (int k = ln; k < TPB; k += 32) top2_merge(f1, f2, tt.red[wp][k][0], tt.red[wp][k][1]);
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
-        const float o1 = __shfl_down_sync(0xffffffffu, f1, off);
-        const float o2 = __shfl_down_sync(0xffffffffu, f2, off);
-        const int g1 = __shfl_down_sync(0xffffffffu, e1, off);
-        const int g2 = __shfl_down_sync(0xffffffffu, e2, off);
+        const float o1 = __shfl_xor_sync(0xffffffffu, f1, off);
+        const float o2 = __shfl_xor_sync(0xffffffffu, f2, off);
         top2_merge(f1, f2, o1, o2);
-        min2_merge(e1, e2, g1, g2);
+      }
+      if (f2 <= -2.f) {
+        // fewer than two candidates are not degenerate: the first two that are
+        for (int k = ln; k < TPB; k += 32) min2_merge(e1, e2, tt.deg[wp][k][0], tt.deg[wp][k][1]);
+        for (int off = 16; off > 0; off >>= 1) {
+          const int g1 = __shfl_xor_sync(0xffffffffu, e1, off);
+          const int g2 = __shfl_xor_sync(0xffffffffu, e2, off);
+          min2_merge(e1, e2, g1, g2);
+        }
       }
       if (ln == 0) {
         tt.f[wp][0] = f1;
@@ -468,9 +481,49 @@ __device__ void finish_tile(const NccArgs &a, TileTail<C::BPC, C::TPB> &tt, cons
   }
 }
 
+// The windows of a CTA's blocks, row by row: a 16-lane group takes a (block,
+// row y) and walks its E planes, all of whose loads are issued before the first
+// is used; x and y are tested and addressed once per row and the planes by one
+// addition each (with rows dealt singly, that arithmetic was nine tenths of the
+// kernels' instructions).  put(block, z, y, x, value, inside the mask, the
+// row's mask bits) for every lane; values outside the image come with ms false.
+template <class C, class Put>
+__device__ __forceinline__ void stage_rows(const NccArgs &a, const int *s_state,
+                                           const int (*s_o)[3], Put put) {
+  constexpr int E = C::E, EY = C::EY, BPC = C::BPC, NGRP = C::NT / 16;
+  constexpr int ZC = E > 10 ? (E + 1) / 2 : E;  // planes in flight per thread
+  const int xl = threadIdx.x & 15, half = threadIdx.x & 16;
+  const unsigned lanes = 0xFFFFu << half;
+  const long long plane = (long long)a.nx * a.ny;
+  for (int item = threadIdx.x >> 4; item < BPC * EY; item += NGRP) {
+    const int s = item / EY, yl = item - s * EY;
+    if (!s_state[s]) continue;
+    const int gx = s_o[s][0] + xl, gy = s_o[s][1] + yl, gz0 = s_o[s][2];
+    const bool in = xl < E && yl < E && (unsigned)gx < (unsigned)a.nx && (unsigned)gy < (unsigned)a.ny;
+    long long q = gz0 * plane + (long long)gy * a.nx + gx;
+#pragma unroll 1
+    for (int z0 = 0; z0 < E; z0 += ZC) {
+      float yv[ZC];
+      bool ms[ZC];
+#pragma unroll
+      for (int i = 0; i < ZC; ++i) {
+        const bool ok = in && z0 + i < E && (unsigned)(gz0 + z0 + i) < (unsigned)a.nz;
+        yv[i] = ok ? __ldg(a.search + q) : 0.f;
+        ms[i] = ok && __ldg(a.smask + q) != 0;
+        q += plane;
+      }
+#pragma unroll
+      for (int i = 0; i < ZC; ++i) {
+        const unsigned bal = __ballot_sync(lanes, ms[i]) >> half;
+        if (z0 + i < E) put(s, z0 + i, yl, xl, yv[i], ms[i], bal & 0xFFFFu);
+      }
+    }
+  }
+}
+
 template <class C>
-__global__ void __launch_bounds__(C::NT, 4) ncc_masked_kernel(NccArgs a) {
-  constexpr int BW = C::BW, W = C::W, TY = C::TY, BPC = C::BPC, B = C::B, R = C::R, E = C::E;
+__global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
+  constexpr int BW = C::BW, W = C::W, TY = C::TY, BPC = C::BPC, B = C::B, R = C::R;
   constexpr int EY = C::EY, EXP = C::EXP, PS = C::PS, WIN = C::WIN, TPB = C::TPB, NYG = C::NYG;
   constexpr int NC = C::NC, NROW = C::NROW, NPAT = C::NPAT, NTAB = C::NTAB;
   extern __shared__ __align__(16) float sm[];
@@ -530,46 +583,12 @@ __global__ void __launch_bounds__(C::NT, 4) ncc_masked_kernel(NccArgs a) {
     }
     if (tid < BPC) s_nstr[tid] = 0;
     __syncthreads();
-    // stage the windows, a 16-lane group per window row (consecutive x): the
-    // E EY rows of a window (plane-major) are dealt round-robin to the CTA's
-    // groups, and a group issues the loads of up to CH rows before it stores:
-    // (y - c) ms, zero outside the image and in the padding, and the row's
-    // mask bits (warp ballot); the base blocks as x - mu
-    {
-      constexpr int LPR = 16, NGRP = C::NT / LPR, RPG = (NROW + NGRP - 1) / NGRP;
-      constexpr int CH = RPG < 6 ? RPG : 6;  // rows in flight per thread (registers)
-      const int xl = tid & (LPR - 1), grp = tid / LPR;
-      for (int s = 0; s < BPC; ++s) {
-        if (!s_state[s]) continue;
-        const int gx = s_o[s][0] + xl;
-        const bool xin = xl < E && gx >= 0 && gx < nx;
-        const float c = s_c[s];
-#pragma unroll 1
-        for (int i0 = 0; i0 < RPG; i0 += CH) {
-          float yv[CH];
-          bool msv[CH];
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            const int rr = grp + (i0 + i) * NGRP, z = rr / EY, yl = rr - z * EY;
-            const int gy = s_o[s][1] + yl, gz = s_o[s][2] + z;
-            const bool in =
-                rr < NROW && xin && yl < E && gy >= 0 && gy < ny && gz >= 0 && gz < nz;
-            const long long q = ((long long)gz * ny + gy) * nx + gx;
-            yv[i] = in ? __ldg(&a.search[q]) : 0.f;
-            msv[i] = in && __ldg(&a.smask[q]) != 0;
-          }
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            const int rr = grp + (i0 + i) * NGRP, z = rr / EY, yl = rr - z * EY;
-            const unsigned int bal = __ballot_sync(0xffffffffu, msv[i]);
-            if (rr < NROW) {
-              if (xl < EXP) win[s * WIN + z * PS + yl * EXP + xl] = msv[i] ? yv[i] - c : 0.f;
-              if (xl == 0) bits[s * NROW + rr] = (bal >> (tid & LPR)) & 0xFFFFu;
-            }
-          }
-        }
-      }
-    }
+    // stage the windows: (y - c) ms, zero outside the image and in the padding,
+    // and the rows' mask bits
+    stage_rows<C>(a, s_state, s_o, [&](int s, int z, int yl, int xl, float yv, bool ms, unsigned bal) {
+      if (xl < EXP) win[s * WIN + z * PS + yl * EXP + xl] = ms ? yv - s_c[s] : 0.f;
+      if (xl == 0) bits[s * NROW + z * EY + yl] = bal;
+    });
     for (int i = tid; i < BPC * B; i += blockDim.x) {
       const int s = i / B;
       if (!s_state[s]) continue;
@@ -726,9 +745,10 @@ __global__ void __launch_bounds__(C::NT, 4) ncc_masked_kernel(NccArgs a) {
 // ---------------------------------------------------------------------------
 template <class C>
 __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
-  constexpr int BW = C::BW, W = C::W, TY = C::TY, BPC = C::BPC, B = C::B, R = C::R, E = C::E;
-  constexpr int EY = C::EY, EXP = C::EXP, PS = C::PS, WIN = C::WIN, TPB = C::TPB, NYG = C::NYG;
-  constexpr int NC = C::NC;
+  static_assert(C::EY <= C::NT / 16, "a window plane fits the CTA");
+  constexpr int BW = C::BW, W = C::W, TY = C::TY, BPC = C::BPC, B = C::B, R = C::R;
+  constexpr int E = C::E, EY = C::EY, EXP = C::EXP, PS = C::PS, WIN = C::WIN, TPB = C::TPB;
+  constexpr int NYG = C::NYG, NC = C::NC;
   extern __shared__ __align__(16) float sm[];
   float *win = sm;                                               // BPC * WIN: y ms
   float *mwin = sm + BPC * WIN;                                  // BPC * WIN: ms
@@ -739,6 +759,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
   __shared__ int s_b[BPC];
   __shared__ int s_o[BPC][3];
   __shared__ double s_mean[BPC];
+  __shared__ unsigned int s_rows[BPC];   // base rows with a voxel inside the mask
   const int tid = threadIdx.x;
   const int slot = tid / TPB;
   const int lt = tid - slot * TPB;
@@ -754,6 +775,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
       long long i = base + tid;
       int state = 0;
       tt.cnt[tid] = 0;
+      s_rows[tid] = 0;
       if (i < nlist) {
         const int b = a.gen_list[i];
         s_b[tid] = b;
@@ -808,6 +830,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
                           (s_o[s][0] + R + vx);
       const float xv = (float)__dsub_rn((double)__ldg(&a.base[q]), s_mean[s]);
       const float mb = __ldg(&a.bmask[q]) ? 1.f : 0.f;
+      if (mb != 0.f) atomicOr(&s_rows[s], 1u << (vz * BW + vy));
       xb[i] = make_float4(mb * xv, mb * (xv * xv), mb, 0.f);
     }
     __syncthreads();
@@ -833,6 +856,9 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
       for (int vz = 0; vz < BW; ++vz) {
 #pragma unroll
         for (int j = 0; j < TY + BW - 1; ++j) {
+          // (one candidate row per thread: window row j meets base row vy = j
+          // only, and a base row outside its mask adds nothing)
+          if (TY == 1 && !((s_rows[slot] >> (vz * BW + j)) & 1u)) continue;
           float r[EXP], m[EXP];
           const float4 *rp = reinterpret_cast<const float4 *>(win + wo + vz * PS + j * EXP);
           const float4 *mp = reinterpret_cast<const float4 *>(mwin + wo + vz * PS + j * EXP);
@@ -2047,20 +2073,22 @@ mirorr_status set_smem(K kernel, size_t smem) {
   return MIRORR_OK;
 }
 
-template <class C>
+// CM: the masked-window kernel's configuration, CB: the base-mask kernel's.
+template <class CM, class CB>
 mirorr_status launch_masked(const NccArgs &a, cudaStream_t s) {
-  size_t smem = sizeof(float) * (size_t)C::SMEM_FLOATS;
-  MB2_TRY(set_smem(ncc_masked_kernel<C>, smem));
-  long long need = (a.nblocks + C::BPC - 1) / C::BPC;
-  long long grid = need < (long long)sm_count() * 8 ? need : (long long)sm_count() * 8;
-  ncc_masked_kernel<C><<<(unsigned)grid, C::NT, smem, s>>>(a);
+  size_t smem = sizeof(float) * (size_t)CM::SMEM_FLOATS;
+  MB2_TRY(set_smem(ncc_masked_kernel<CM>, smem));
+  long long need = (a.nblocks + CM::BPC - 1) / CM::BPC;
+  const long long cap = (long long)sm_count() * 2 * CM::MINB;
+  ncc_masked_kernel<CM><<<(unsigned)(need < cap ? need : cap), CM::NT, smem, s>>>(a);
   MB2_LAUNCH_CHECK();
   // then the blocks with a partly masked base block (the list grows in both
   // kernels above)
-  const size_t smem_b = sizeof(float) * (size_t)C::BPC * (2 * C::WIN + 4 * C::B);
-  MB2_TRY(set_smem(ncc_basemask_kernel<C>, smem_b));
+  const size_t smem_b = sizeof(float) * (size_t)CB::BPC * (2 * CB::WIN + 4 * CB::B);
+  MB2_TRY(set_smem(ncc_basemask_kernel<CB>, smem_b));
+  need = (a.nblocks + CB::BPC - 1) / CB::BPC;
   const long long grid_b = need < (long long)sm_count() * 4 ? need : (long long)sm_count() * 4;
-  ncc_basemask_kernel<C><<<(unsigned)grid_b, C::NT, smem_b, s>>>(a);
+  ncc_basemask_kernel<CB><<<(unsigned)grid_b, CB::NT, smem_b, s>>>(a);
   MB2_LAUNCH_CHECK();
   return MIRORR_OK;
 }
@@ -2076,10 +2104,10 @@ mirorr_status launch_warp(const NccArgs &a, cudaStream_t s) {
   return MIRORR_OK;
 }
 
-template <class CW, class CM>
+template <class CW, class CM, class CB>
 mirorr_status launch_fast(const NccArgs &a, cudaStream_t s) {
   MB2_TRY((launch_warp<CW>(a, s)));
-  MB2_TRY((launch_masked<CM>(a, s)));
+  MB2_TRY((launch_masked<CM, CB>(a, s)));
   return MIRORR_OK;
 }
 
@@ -2158,7 +2186,7 @@ mirorr_status encode_map3(CUtensorMap *map, CUtensorMapDataType type, int elem, 
   return MIRORR_OK;
 }
 
-template <int W, int P, int RPU, class CM>
+template <int W, int P, int RPU, class CM, class CB>
 mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
                            cudaEvent_t *kev) {
   constexpr int E = W + 3, NL = 32 * kXWarps, BPW = NL / W;
@@ -2220,7 +2248,7 @@ mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
   kernel<<<(unsigned)grid, NL, smem, s>>>(a, xa, tmap, smap);
   MB2_LAUNCH_CHECK();
   if (kev) MB2_CUDA_TRY(cudaEventRecord(kev[1], s));
-  MB2_TRY((launch_masked<CM>(a, s)));
+  MB2_TRY((launch_masked<CM, CB>(a, s)));
   done = true;
   return MIRORR_OK;
 }
@@ -2233,28 +2261,28 @@ bool run_fast(NccArgs &a, BmWork &w, cudaStream_t s, mirorr_status &st, cudaEven
   if ((long long)a.nx * a.ny * a.nz >= (1LL << 31)) return false;
   if (a.bw == 4 && a.W == 9) {
     bool done = false;
-    st = launch_xlane<9, 3, 48, FastCfg<4, 9, 1, 3>>(a, w, s, done, kev);
+    st = launch_xlane<9, 3, 48, MaskedCfg<4, 9>, FastCfg<4, 9, 1, 3>>(a, w, s, done, kev);
     xl_ran = done;
     if (st != MIRORR_OK || done) return true;
-    st = launch_fast<WarpCfg<4, 9, 3, 1, 5, 3>, FastCfg<4, 9, 1, 3>>(a, s);
+    st = launch_fast<WarpCfg<4, 9, 3, 1, 5, 3>, MaskedCfg<4, 9>, FastCfg<4, 9, 1, 3>>(a, s);
     return true;
   }
   if (a.bw == 4 && a.W == 7) {
     bool done = false;
-    st = launch_xlane<7, 4, 48, FastCfg<4, 7, 1, 5>>(a, w, s, done, kev);
+    st = launch_xlane<7, 4, 48, MaskedCfg<4, 7>, FastCfg<4, 7, 1, 5>>(a, w, s, done, kev);
     xl_ran = done;
     if (st != MIRORR_OK || done) return true;
-    st = launch_fast<WarpCfg<4, 7, 4, 2, 4, 3>, FastCfg<4, 7, 1, 5>>(a, s);
+    st = launch_fast<WarpCfg<4, 7, 4, 2, 4, 3>, MaskedCfg<4, 7>, FastCfg<4, 7, 1, 5>>(a, s);
     return true;
   }
   if (a.bw == 4 && a.W == 5) {
     bool done = false;
-    st = launch_xlane<5, 5, 56, FastCfg<4, 5, 1, 10>>(a, w, s, done, kev);
+    st = launch_xlane<5, 5, 56, MaskedCfg<4, 5>, FastCfg<4, 5, 1, 10>>(a, w, s, done, kev);
     xl_ran = done;
     return st != MIRORR_OK || done;
   }
   if (a.bw == 5 && a.W == 11) {
-    st = launch_fast<WarpCfg<5, 11, 6, 1, 4, 2>, FastCfg<5, 11, 1, 2>>(a, s);
+    st = launch_fast<WarpCfg<5, 11, 6, 1, 4, 2>, MaskedCfg<5, 11>, FastCfg<5, 11, 1, 2>>(a, s);
     return true;
   }
   return false;
