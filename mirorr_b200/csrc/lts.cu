@@ -22,8 +22,8 @@
 // which meet at a software grid barrier whose wait is bounded (about one
 // second; a timeout raises an error flag and every CTA returns).  Per inner
 // iteration of a rigid fit: 84K cycles with a software barrier over 2 to 16
-// CTAs and the matrices of the solve in local memory, 39K now at 7,300 pairs;
-// of a symmetric affine one at 590,000 pairs 150K, now 81K.
+// CTAs and the matrices of the solve in local memory, 36K now at 7,300 pairs;
+// of a symmetric affine one at 590,000 pairs 150K, now 80K.
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -45,9 +45,14 @@ constexpr int kPartial = 32;  // doubles per CTA partial
 constexpr int kSums = 28;     // count, 6 first and 21 second moments
 constexpr int kClusterCtas = 8;  // CTAs of a cluster (the portable limit)
 // Pairs up to which one cluster is faster than a CTA per SM: an iteration
-// (rigid) takes 28K + 1.2 n cycles on a cluster (39K at 7,500 pairs, 59K at
-// 25,600, 67K at 47,500) and about 46K on the whole GPU.
+// (rigid) takes 36K cycles on a cluster at 7,500 pairs, 51K at 25,600 and 64K
+// at 47,500, and about 46K on the whole GPU.
 constexpr long long kClusterPairs = 16384;
+// Pairs up to which one CTA of the cluster runs the fit alone, with the
+// histogram, the residuals and the state in its shared memory and no global
+// round trips (an iteration at 1,000 pairs 25K cycles against 35K on the
+// cluster; equal at about 4,500).
+constexpr long long kSinglePairs = 4096;
 // The first histogram's keys: 64 bins per octave over [2^-12, 2^20) mm^2 (a
 // residual's bit pattern above kKeyLo in steps of 2^46), one bin below and one
 // above.
@@ -80,6 +85,7 @@ struct LtsArgs {
 // at cluster scope and cannot time out (its CTAs are resident together and
 // none leaves early).
 struct GridSync {
+  static constexpr bool single = false;
   LtsCtl *ctl;
   long long spin_limit;
   unsigned int nctas;
@@ -87,9 +93,18 @@ struct GridSync {
   __device__ bool operator()() { return grid_barrier(&ctl->bar, round++, spin_limit, nctas); }
 };
 struct ClusterSync {
+  static constexpr bool single = false;
   __device__ bool operator()() {
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::
                      : "memory");
+    return true;
+  }
+};
+
+struct SingleSync {
+  static constexpr bool single = true;
+  __device__ bool operator()() {
+    __syncthreads();
     return true;
   }
 };
@@ -163,17 +178,31 @@ __device__ inline void grid_partial_sums(const double *part, double *out, int nc
   __syncthreads();
 }
 
-__device__ inline double residual(const LtsState &s, const double *x, const double *y) {
+// Squared distance of the transformed initial point f(x) (matrix f[0..9),
+// offset f[9..12)) from y, or from b(y) in the symmetric fit (tfm_apply's
+// order of operations).
+__device__ inline void apply_rows(const double (&f)[12], const double *x, double *o) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double v = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) v += f[3 * i + j] * x[j];
+    o[i] = v + f[9 + i];
+  }
+}
+__device__ inline double residual(const double (&f)[12], const double (&b)[12], bool symmetric,
+                                  const double *x, const double *y) {
   double p[3], q[3];
-  tfm_apply(s.fin, x, p);
-  if (s.symmetric) {
-    tfm_apply(s.finb, y, q);
+  apply_rows(f, x, p);
+  if (symmetric) {
+    apply_rows(b, y, q);
   } else {
     q[0] = y[0]; q[1] = y[1]; q[2] = y[2];
   }
   double r = 0.0;
+#pragma unroll
   for (int i = 0; i < 3; ++i) {
-    double d = p[i] - q[i];
+    const double d = p[i] - q[i];
     r += d * d;
   }
   return r;
@@ -193,6 +222,22 @@ __device__ inline void first_range(int bin, unsigned long long &lo, unsigned lon
   } else {
     lo = kKeyLo + ((unsigned long long)(bin - 1) << kKeyShift);
     hi = bin == kBins - 1 ? ~0ULL : lo + ((1ULL << kKeyShift) - 1);
+  }
+}
+
+// f(key) for this thread's residuals' bit patterns, four loads in flight.
+template <class F>
+__device__ __forceinline__ void for_keys(const double *resid, long long n, long long first,
+                                         long long stride, F f) {
+  constexpr int U = 4;
+  for (long long i0 = first; i0 < n; i0 += U * stride) {
+    unsigned long long k[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      k[u] = (unsigned long long)__double_as_longlong(resid[i0 + u * stride < n ? i0 + u * stride : i0]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * stride < n) f(k[u]);
   }
 }
 
@@ -271,8 +316,11 @@ __device__ __noinline__ void solve_symmetric(LtsState &s, const Subset &m) {
 }
 
 // The LTS loop run by `ncta` CTAs (index `cta` among them) that meet at `sync`.
+// resid: one double per pair (global scratch; shared memory when one CTA runs
+// the fit).
 template <class Sync>
-__device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
+__device__ void lts_body(const LtsArgs &a, Sync sync, double *resid, int cta, int ncta) {
+  constexpr bool kSingle = Sync::single;
   __shared__ __align__(16) LtsState s;
   __shared__ unsigned int h[kBins];
   __shared__ unsigned long long ck[kCandMax];
@@ -281,21 +329,35 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
   __shared__ Subset sub;
   __shared__ double s_nth;
   __shared__ unsigned long long s_key;
+  __shared__ unsigned int s_left;  // keys gathered for the final rank
   __shared__ unsigned long long s_pair[2];
   const long long n = __ldcg(&a.n_dev[0]) + __ldcg(&a.n_dev[1]);
   const long long gstride = (long long)ncta * kThreads;
   const long long gtid = (long long)cta * kThreads + threadIdx.x;
 
   for (int guard = 0; guard < 200; ++guard) {
-    load_cg(&s, a.state, sizeof(LtsState));
+    if (!kSingle || guard == 0) load_cg(&s, a.state, sizeof(LtsState));
     for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
-    if (cta == 0)
+    if (kSingle && threadIdx.x == 0) {
+      s_key = 0;
+      s_left = 0;
+    }
+    if (!kSingle && cta == 0)
       for (int i = threadIdx.x; i < kBins; i += kThreads) a.hist[kBins + i] = 0;  // next pass's
     __syncthreads();
     if (!s.running || n <= 0) break;
     const bool first = s.fraction > 0.99999;
     // ---- residuals (+ max or first histogram) ----------------------------
     unsigned long long kmax = 0;
+    // the transforms in registers (in shared memory they would be read again
+    // for every pair)
+    double ft[12], bt[12];
+    const bool symmetric = s.symmetric != 0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+      ft[i] = i < 9 ? s.fin.M[i < 9 ? i : 0] : s.fin.off[i < 9 ? 0 : i - 9];
+      bt[i] = i < 9 ? s.finb.M[i < 9 ? i : 0] : s.finb.off[i < 9 ? 0 : i - 9];
+    }
     for (long long i0 = gtid; i0 < n; i0 += kUnroll * gstride) {
       // kUnroll pairs' loads are issued before the first is used
       double x[kUnroll][3], y[kUnroll][3];
@@ -311,13 +373,13 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         if (i0 + u * gstride >= n) break;
-        const double r = residual(s, x[u], y[u]);
-        a.resid[i0 + u * gstride] = r;
+        const double r = residual(ft, bt, symmetric, x[u], y[u]);
+        resid[i0 + u * gstride] = r;
         const unsigned long long key = (unsigned long long)__double_as_longlong(r);
         if (first) {
           if (key > kmax) kmax = key;
         } else {
-          hist_add(h, first_bin(key));
+          atomicAdd(&h[first_bin(key)], 1u);
         }
       }
     }
@@ -326,8 +388,8 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
         unsigned long long o = __shfl_down_sync(0xffffffffu, kmax, off);
         if (o > kmax) kmax = o;
       }
-      if ((threadIdx.x & 31) == 0 && kmax) atomicMax(&a.ctl->maxkey, kmax);
-    } else {
+      if ((threadIdx.x & 31) == 0 && kmax) atomicMax(kSingle ? &s_key : &a.ctl->maxkey, kmax);
+    } else if (!kSingle) {
       __syncthreads();
       for (int i = threadIdx.x; i < kBins; i += kThreads)
         if (h[i]) atomicAdd(&a.hist[i], h[i]);
@@ -335,8 +397,10 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
     if (!sync()) return;
     double nth;
     if (first) {
-      if (threadIdx.x == 0) s_key = __ldcg(&a.ctl->maxkey);
-      __syncthreads();
+      if (!kSingle) {
+        if (threadIdx.x == 0) s_key = __ldcg(&a.ctl->maxkey);
+        __syncthreads();
+      }
       nth = __longlong_as_double((long long)s_key);
     } else {
       // ---- radix select of rank k ------------------------------------------
@@ -345,11 +409,13 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
       unsigned long long lo = 0, hi = 0;  // the keys left lie in [lo, hi]
       int shift = 0, pass = 0;
       while (true) {
-        // every CTA scans the global histogram of this pass identically
-        const unsigned int *gh = a.hist + (pass % 3) * kBins;
-        __syncthreads();
-        for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = __ldcg(&gh[i]);
-        __syncthreads();
+        if (!kSingle) {
+          // every CTA scans the global histogram of this pass identically
+          const unsigned int *gh = a.hist + (pass % 3) * kBins;
+          __syncthreads();
+          for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = __ldcg(&gh[i]);
+          __syncthreads();
+        }
         int d = 0;
         unsigned long long cum = 0;
         find_bucket<kBins, kThreads>(h, k, kBins, s_pair, &d, &cum);
@@ -370,36 +436,46 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
         ++pass;
         shift = 0;
         while (((hi - lo) >> shift) >= (unsigned long long)kBins) ++shift;
-        if (cta == 0) {
+        if (!kSingle && cta == 0) {
           unsigned int *zb = a.hist + ((pass + 1) % 3) * kBins;
           for (int i = threadIdx.x; i < kBins; i += kThreads) zb[i] = 0;
         }
         for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
         __syncthreads();
-        for (long long i = gtid; i < n; i += gstride) {
-          const unsigned long long key = (unsigned long long)__double_as_longlong(a.resid[i]);
-          if (key >= lo && key <= hi) hist_add(h, (unsigned int)((key - lo) >> shift));
+        for_keys(resid, n, gtid, gstride, [&](unsigned long long key) {
+          if (key >= lo && key <= hi) atomicAdd(&h[(key - lo) >> shift], 1u);
+        });
+        if (!kSingle) {
+          __syncthreads();
+          unsigned int *gh2 = a.hist + (pass % 3) * kBins;
+          for (int i = threadIdx.x; i < kBins; i += kThreads)
+            if (h[i]) atomicAdd(&gh2[i], h[i]);
         }
-        __syncthreads();
-        unsigned int *gh2 = a.hist + (pass % 3) * kBins;
-        for (int i = threadIdx.x; i < kBins; i += kThreads)
-          if (h[i]) atomicAdd(&gh2[i], h[i]);
         if (!sync()) return;
       }
       if (lo == hi) {
         nth = __longlong_as_double((long long)lo);  // the keys left are equal
       } else {
         // ---- gather the keys left (at most one per thread) and rank them
-        for (long long i = gtid; i < n; i += gstride) {
-          const unsigned long long key = (unsigned long long)__double_as_longlong(a.resid[i]);
+        for_keys(resid, n, gtid, gstride, [&](unsigned long long key) {
           if (key >= lo && key <= hi) {
-            const unsigned long long pos = atomicAdd(&a.ctl->ncand, 1ULL);
-            if (pos < (unsigned long long)kCandMax) a.cand[pos] = key;
+            if (kSingle) {
+              ck[atomicAdd(&s_left, 1u)] = key;  // the bucket holds at most kCandMax
+            } else {
+              const unsigned long long pos = atomicAdd(&a.ctl->ncand, 1ULL);
+              if (pos < (unsigned long long)kCandMax) a.cand[pos] = key;
+            }
           }
-        }
+        });
         if (!sync()) return;
-        if (threadIdx.x == 0) s_key = __ldcg(&a.ctl->ncand);
-        unsigned long long mine = __ldcg(&a.cand[threadIdx.x]);
+        unsigned long long mine;
+        if (kSingle) {
+          mine = ck[threadIdx.x];
+          if (threadIdx.x == 0) s_key = s_left;
+        } else {
+          if (threadIdx.x == 0) s_key = __ldcg(&a.ctl->ncand);
+          mine = __ldcg(&a.cand[threadIdx.x]);
+        }
         __syncthreads();
         int nc = (int)(s_key < (unsigned long long)kCandMax ? s_key : kCandMax);
         bool have = threadIdx.x < nc;
@@ -458,7 +534,7 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         const long long i = i0 + u * gstride < n ? i0 + u * gstride : i0;
-        r[u] = a.resid[i];
+        r[u] = resid[i];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           z[u][c] = __ldcg(&a.init[3 * i + c]);
@@ -482,10 +558,12 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
       }
     }
     block_sums(acc, red, s_out);
-    if (threadIdx.x < kSums) a.partial[(long long)threadIdx.x * ncta + cta] = s_out[threadIdx.x];
-    if (!sync()) return;
+    if (!kSingle) {
+      if (threadIdx.x < kSums) a.partial[(long long)threadIdx.x * ncta + cta] = s_out[threadIdx.x];
+      if (!sync()) return;
+    }
     if (cta == 0) {
-      grid_partial_sums(a.partial, s_out, ncta);
+      if (!kSingle) grid_partial_sums(a.partial, s_out, ncta);
       if (threadIdx.x < 32) {
         const int l = threadIdx.x;
         const double cnt = s_out[0];
@@ -507,7 +585,12 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
           sub.mean[l - 21] =
               (l < 24 ? __ldg(&a.init[l - 21]) : __ldg(&a.moved[l - 24])) + s_out[1 + l - 21] / cnt;
         }
-        __syncwarp();
+      }
+      // (a CTA barrier, after which the solving warp is whole again: run by its
+      // lane groups one after another, a solve took three times as long)
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        const int l = threadIdx.x;
         if (s.symmetric) solve_symmetric(s, sub);
         else solve_classic(s, sub);
         __syncwarp();
@@ -516,15 +599,16 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
           s.iter += 1;
           s.running = lts_continue(s) ? 1 : 0;
           if (s.iter > 101) s.running = 0;
-          // reset select scratch for the next iteration
-          a.ctl->maxkey = 0;
-          a.ctl->ncand = 0;
+          if (!kSingle) {  // reset select scratch for the next iteration
+            a.ctl->maxkey = 0;
+            a.ctl->ncand = 0;
+          }
         }
         __syncwarp();
         const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&s);
         unsigned long long *dst = reinterpret_cast<unsigned long long *>(a.state);
         for (int i = l; i < (int)(sizeof(LtsState) / 8); i += 32) dst[i] = src[i];
-      } else {
+      } else if (!kSingle) {
         for (int i = threadIdx.x - 32; i < kBins; i += kThreads - 32) a.hist[i] = 0;
       }
     }
@@ -533,13 +617,24 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, int cta, int ncta) {
 }
 
 __global__ void __launch_bounds__(kThreads) lts_kernel(LtsArgs a) {
-  lts_body(a, GridSync{a.ctl, a.spin_limit, gridDim.x, 0u}, blockIdx.x, gridDim.x);
+  lts_body(a, GridSync{a.ctl, a.spin_limit, gridDim.x, 0u}, a.resid, blockIdx.x, gridDim.x);
 }
 
-// One fit by one cluster.
+// A fit by a cluster, or by its first CTA alone.
+__device__ void lts_cluster_body(const LtsArgs &a, int cta) {
+  extern __shared__ double s_resid[];  // kSinglePairs
+  const long long n = __ldcg(&a.n_dev[0]) + __ldcg(&a.n_dev[1]);
+  if (n <= kSinglePairs) {
+    if (cta == 0) lts_body(a, SingleSync{}, s_resid, 0, 1);
+    return;
+  }
+  lts_body(a, ClusterSync{}, a.resid, cta, kClusterCtas);
+}
+constexpr size_t kClusterSmem = sizeof(double) * kSinglePairs;
+
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
     lts_cluster_kernel(LtsArgs a) {
-  lts_body(a, ClusterSync{}, blockIdx.x, kClusterCtas);
+  lts_cluster_body(a, blockIdx.x);
 }
 
 // Several independent fits in one launch, a cluster each: fit f runs on CTAs
@@ -547,7 +642,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
     lts_batch_kernel(const LtsArgs *args) {
   const LtsArgs a = args[blockIdx.x / kClusterCtas];
-  lts_body(a, ClusterSync{}, blockIdx.x % kClusterCtas, kClusterCtas);
+  lts_cluster_body(a, blockIdx.x % kClusterCtas);
 }
 
 // Zeroes each fit's barrier, select control and histograms (CTA f: fit f) so
@@ -567,7 +662,9 @@ int fit_ctas(long long n, int max_ctas) {
 
 mirorr_status launch_fit(LtsArgs &a, long long n, int ctas, cudaStream_t st) {
   if (n <= kClusterPairs) {
-    lts_cluster_kernel<<<kClusterCtas, kThreads, 0, st>>>(a);
+    MB2_CUDA_TRY(cudaFuncSetAttribute(lts_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kClusterSmem));
+    lts_cluster_kernel<<<kClusterCtas, kThreads, kClusterSmem, st>>>(a);
     MB2_LAUNCH_CHECK();
     return MIRORR_OK;
   }
@@ -729,7 +826,9 @@ mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, DevBuf &args_dev,
   const size_t zbytes = up(sizeof(LtsCtl)) + up(sizeof(unsigned int) * 3 * kBins);
   lts_batch_zero_kernel<<<nfits, 256, 0, st>>>(dargs, (unsigned long long)(zbytes / 16));
   MB2_LAUNCH_CHECK();
-  lts_batch_kernel<<<nfits * kClusterCtas, kThreads, 0, st>>>(dargs);
+  MB2_CUDA_TRY(cudaFuncSetAttribute(lts_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kClusterSmem));
+  lts_batch_kernel<<<nfits * kClusterCtas, kThreads, kClusterSmem, st>>>(dargs);
   MB2_LAUNCH_CHECK();
   return MIRORR_OK;
 }

@@ -1,7 +1,7 @@
 """The LTS fit where its launch and its selection change form, against the oracle.
 
-* pair counts around one cluster's limit (16,384 pairs) and around a cluster's
-  thread and candidate counts, down to a handful;
+* pair counts around one CTA's limit (4,096 pairs), one cluster's (16,384) and
+  a CTA's thread and candidate counts, down to a handful;
 * residuals below, inside and above the first histogram's range
   ([2^-12, 2^20) mm^2), so the cut-off falls into its open end bins;
 * more equal residuals than the final ranking holds.
@@ -44,7 +44,7 @@ def _fit_both(ctx, kind, x, y, symmetric):
 
 @pytest.mark.parametrize("symmetric", [False, True])
 @pytest.mark.parametrize("kind", ["rigid", "affine"])
-@pytest.mark.parametrize("n", [40, 511, 4097, 16384, 16385, 33000])
+@pytest.mark.parametrize("n", [40, 511, 4096, 4097, 16384, 16385, 33000])
 def test_pair_counts(ctx, n, kind, symmetric):
     rng = np.random.default_rng(n)
     x = rng.uniform(-60, 60, size=(n, 3))
