@@ -2275,7 +2275,12 @@ bool run_fast(NccArgs &a, BmWork &w, cudaStream_t s, mirorr_status &st, cudaEven
     st = launch_fast<WarpCfg<4, 7, 4, 2, 4, 3>, MaskedCfg<4, 7>, FastCfg<4, 7, 1, 5>>(a, s);
     return true;
   }
-  if (a.bw == 4 && a.W == 5) {
+  // window 5: 125 candidates a block are little work, and a call of few blocks
+  // is shorter as one general launch than as the window-AND, the per-x-lane and
+  // the two masked kernels in a row (6,600 blocks 242 us against 234, with masks
+  // 256 against 274; 13,500 blocks 315 and 349 against 258 and 299)
+  constexpr long long kXlane5Blocks = 10000;
+  if (a.bw == 4 && a.W == 5 && a.nblocks >= kXlane5Blocks) {
     bool done = false;
     st = launch_xlane<5, 5, 56, MaskedCfg<4, 5>, FastCfg<4, 5, 1, 10>>(a, w, s, done, kev);
     xl_ran = done;

@@ -478,13 +478,15 @@ __global__ void __launch_bounds__(256) prep16w_kernel(const Args16 *calls) {
   const bool row = lane < BW * BW;
   constexpr unsigned rows_mask = (BW * BW == 32) ? 0xffffffffu : ((1u << (BW * BW)) - 1u);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  // a warp takes 32 consecutive blocks: the culled ones are written by a lane
-  // each, and the others are listed with one addition to the list's counter
-  // (one per block made that counter the bound: 2.65 ms for 0.7 of 2.4 million
-  // blocks, 0.76 ms now)
-  for (long long b0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
-       b0 < a.nblocks; b0 += nwarps * 32) {
-    const bool live = b0 + lane < a.nblocks;
+  // a warp takes `per` consecutive blocks (32 once every warp has that many):
+  // the culled ones are written by a lane each, and the others are listed with
+  // one addition to the list's counter (one per block made that counter the
+  // bound: 2.65 ms for 0.7 of 2.4 million blocks, 0.76 ms now)
+  int per = 1;
+  while (per < 32 && per * nwarps < a.nblocks) per *= 2;
+  for (long long b0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * per;
+       b0 < a.nblocks; b0 += nwarps * per) {
+    const bool live = lane < per && b0 + lane < a.nblocks;
     const bool sel = live && (!a.selected || a.selected[b0 + lane]);
     if (live && !sel) {
       int bx, by, bz;

@@ -1,8 +1,8 @@
 """The per-x-lane search over its windows, spacings and volume edges.
 
-Block width 4 with windows 5, 7 and 9 takes the per-x-lane kernel at every
-block spacing whose union window fits; spacings above 4 use the run-time row
-pitch.  Odd and even volumes (statistics rows padded to an even pitch), volumes
+Block width 4 with windows 7 and 9, and 5 from 10,000 blocks on, takes the
+per-x-lane kernel at every block spacing whose union window fits; spacings above
+4 use the run-time row pitch.  Odd and even volumes (statistics rows padded to an even pitch), volumes
 smaller than a window, flat regions (degenerate candidates) and fewer blocks
 than one tile are where its tiles end.  Best, second, argmax and points equal
 the FP64 oracle's exactly, as for every other search kernel.
@@ -63,3 +63,17 @@ def test_wide_value_ranges(ctx, nw):
     a, b = rng.random((2, 10, 14, 30)).astype(np.float32)
     _check(ctx, a + np.float32(4000.0), b + np.float32(4000.0), nw, 3)
     _check(ctx, a * np.float32(1e-20), b * np.float32(1e-20), nw, 3)
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("shape,gap", [((24, 30, 41), 1), ((43, 44, 62), 2), ((27, 25, 30), 1)])
+def test_window_5_on_both_sides_of_its_limit(ctx, shape, gap, flat):
+    # 20,000 to 22,000 blocks, and 13,700; the smaller volumes above stay below
+    _check(ctx, _volume(shape, 1, flat), _volume(shape, 2, flat), 5, gap)
+
+
+def test_window_5_wide_value_ranges(ctx):
+    rng = np.random.default_rng(5)
+    a, b = rng.random((2, 24, 30, 41)).astype(np.float32)
+    _check(ctx, a + np.float32(4000.0), b + np.float32(4000.0), 5, 1)
+    _check(ctx, a * np.float32(1e-20), b * np.float32(1e-20), 5, 1)
