@@ -95,7 +95,8 @@ __device__ __noinline__ double box_ss64(const float *__restrict__ y,
   return ss;
 }
 
-template <int BW>
+// MASK false: no search mask (every voxel counts, none is read).
+template <int BW, bool MASK>
 __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict__ y,
                                                         const uint8_t *__restrict__ ms, int nx,
                                                         int ny, int nz, int sp,
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict_
 #pragma unroll
           for (int vx = 0; vx < BW; ++vx) {
             v[vx] = __ldg(y + q + vx);
-            m[vx] = __ldg(ms + q + vx) != 0;
+            m[vx] = !MASK || __ldg(ms + q + vx) != 0;
             rall = rall && m[vx];
             rany = rany || m[vx];
           }
@@ -203,14 +204,19 @@ __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict_
 }
 
 mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8_t *smask,
-                               float2 *stats, cudaStream_t s) {
+                               float2 *stats, cudaStream_t s, bool no_masks) {
   long long n = (long long)g.size[0] * g.size[1] * ((g.size[2] + kBoxPZ - 1) / kBoxPZ);
   int threads = 256;
   long long blocks = (n + threads - 1) / threads;
   if (blocks > (long long)sm_count() * 64) blocks = (long long)sm_count() * 64;
   switch (g.bw) {
-#define CASE(B) \
-  case B: box_stats_kernel<B><<<(unsigned)blocks, threads, 0, s>>>(search, smask, g.size[0], g.size[1], g.size[2], stats_pitch(g.size[0]), stats); break;
+#define CASE(B)                                                                            \
+  case B: {                                                                                \
+    auto k = no_masks ? box_stats_kernel<B, false> : box_stats_kernel<B, true>;            \
+    k<<<(unsigned)blocks, threads, 0, s>>>(search, smask, g.size[0], g.size[1], g.size[2], \
+                                           stats_pitch(g.size[0]), stats);                 \
+    break;                                                                                 \
+  }
     CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
 #undef CASE
     default:

@@ -318,6 +318,7 @@ struct MatchCall {
   const uint8_t *bmask, *smask;
   int size[3];
   mirorr_geometry point_geom;  // base image geometry (blockPositionToPoint)
+  bool no_masks = false;       // no mask was given: both are 255 everywhere
 };
 
 mirorr_status run_match(mirorr_ctx c, const mirorr_bm_params &p, const MatchCall &mc,
@@ -350,13 +351,13 @@ mirorr_status run_match(mirorr_ctx c, const mirorr_bm_params &p, const MatchCall
                                       give_up, c->ltsw.spin_limit));
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[2], s));
     MB2_TRY(launch_match16(mc.dtype, g, mc.base, mc.bmask, mc.search, mc.smask, sel, out, c->bm16,
-                           c->ncc_count.as<unsigned long long>(), s));
+                           c->ncc_count.as<unsigned long long>(), s, mc.no_masks));
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[3], s));
     if (xl_ran) *xl_ran = false;
   } else {
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[0], s));
     MB2_TRY(launch_box_stats(g, static_cast<const float *>(mc.search), mc.smask,
-                             c->bmw.stats.as<float2>(), s));
+                             c->bmw.stats.as<float2>(), s, mc.no_masks));
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[1], s));
     const uint8_t *sel = nullptr;
     unsigned int *give_up = nullptr;
@@ -366,8 +367,8 @@ mirorr_status run_match(mirorr_ctx c, const mirorr_bm_params &p, const MatchCall
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[2], s));
     MB2_TRY(launch_ncc(g, static_cast<const float *>(mc.base), mc.bmask,
                        static_cast<const float *>(mc.search), mc.smask, c->bmw.stats.as<float2>(),
-                       sel, out, c->bmw, c->ncc_count.as<unsigned long long>(), s, kev, xl_count,
-                       xl_ran));
+                       sel, out, c->bmw, c->ncc_count.as<unsigned long long>(), s, mc.no_masks, kev,
+                       xl_count, xl_ran));
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[3], s));
   }
   PointGeom pg;
@@ -1495,7 +1496,7 @@ mirorr_status mirorr_bm_get_offsets(mirorr_matcher m, size_t capacity, double *b
   MB2_CUDA_TRY(cudaMemsetAsync(c->counts.ptr, 0, 4 * sizeof(long long), c->stream));
   MatchCall mc{m->base.img, m->search.img, m->storage, bmask, smask,
                {m->base.geom.size[0], m->base.geom.size[1], m->base.geom.size[2]},
-               m->base.geom};
+               m->base.geom, !m->base.has_mask && !m->search.has_mask};
   MB2_TRY(run_match(c, m->p, mc, g, m->best, m->second, m->match, m->status,
                     m->pts_b.as<double>(), m->pts_m.as<double>(), c->counts.as<long long>(),
                     nullptr, m->ev));

@@ -57,8 +57,11 @@ inline int stats_pitch(int nx) { return (nx + 1) & ~1; }
 // stats: (mean, 1 / masked sum of squares) per candidate origin; the second is
 // 0 when the sum is, NaN where the footprint leaves the volume, and its sign
 // bit is set when some voxel of the footprint is outside the search mask.
+// no_masks (here and in launch_ncc, launch_match16): the caller set no mask, so
+// the mask buffers hold 255 everywhere; what masks decide is not launched and
+// most kernels do not read them.
 mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8_t *smask,
-                               float2 *stats, cudaStream_t s);
+                               float2 *stats, cudaStream_t s, bool no_masks);
 // base: float32, or 16-bit when dtype is MIRORR_DTYPE_BF16 / _F16.
 // Work-area sizes of one selection: BmWork::var and BmWork::select_state.
 size_t selection_var_bytes(long long nblocks);
@@ -78,7 +81,7 @@ mirorr_status launch_variance_selection(const BmGeom &g, const void *base, doubl
 mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmask,
                          const float *search, const uint8_t *smask, const float2 *stats,
                          const uint8_t *selected, const BmOut &out, BmWork &w,
-                         unsigned long long *ncc_count, cudaStream_t s,
+                         unsigned long long *ncc_count, cudaStream_t s, bool no_masks,
                          cudaEvent_t *kev = nullptr, unsigned long long *xl_count = nullptr,
                          bool *xl_ran = nullptr);
 // True when a bounded device wait of the NCC stage gave up since the last
@@ -143,6 +146,7 @@ struct alignas(64) Match16Call {
   int tiles_x;
   int chunk_x0, nxc;      // x of the copy's first 8-wide chunk, chunks per row
   int tensor;             // the call takes the tensor form
+  int no_masks;           // no mask was given: masks are 255 everywhere and not read
   int active;             // 0: the launch skips the call
   long long ntiles;
   long long tile0;        // first tile of the call in the launch (set by the launcher)
@@ -183,7 +187,7 @@ mirorr_status launch_match16_batch(int dtype, int ncalls, Match16Call *host_call
 mirorr_status launch_match16(int dtype, const BmGeom &g, const void *base, const uint8_t *bmask,
                              const void *search, const uint8_t *smask, const uint8_t *selected,
                              const BmOut &out, Bm16Work &w, unsigned long long *ncc_count,
-                             cudaStream_t s);
+                             cudaStream_t s, bool no_masks);
 // True when a bounded wait of the 16-bit search gave up (synchronises).
 mirorr_status match16_take_timeout(Bm16Work &w, cudaStream_t s, bool *timed_out);
 // Blocks of the last 16-bit search taken by [0] the tensor form, [1] the

@@ -71,6 +71,7 @@ struct NccArgs {
   const uint8_t *smask;
   const float2 *stats;  // box_stats, rows of sp
   int sp;
+  int no_masks;         // both masks are 255 everywhere
   const uint8_t *selected;
   const BlockStat *bstat;
   int nx, ny, nz;
@@ -279,7 +280,7 @@ __device__ inline void finish_unmasked_block(const NccArgs &a, long long b) {
 // ---------------------------------------------------------------------------
 // BW > 0: the block width known at compile time (the block's loads are all
 // issued before the sums); BW = 0: a.bw at run time.  Same arithmetic order.
-template <int BW>
+template <int BW, bool MASK>
 __global__ void block_stat_kernel(NccArgs a) {
   for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < a.nblocks;
        b += (long long)gridDim.x * blockDim.x) {
@@ -296,7 +297,7 @@ __global__ void block_stat_kernel(NccArgs a) {
         for (int x = 0; x < bw; ++x) {
           long long q = o + ((long long)z * a.ny + y) * a.nx + x;
           sum = __dadd_rn(sum, (double)__ldg(&a.base[q]));
-          if (__ldg(&a.bmask[q])) ++nin;
+          if (!MASK || __ldg(&a.bmask[q])) ++nin;
         }
     double mean = __ddiv_rn(sum, (double)(bw * bw * bw));
     double sxx = 0.0, sxt = 0.0;
@@ -307,7 +308,7 @@ __global__ void block_stat_kernel(NccArgs a) {
 #pragma unroll
         for (int x = 0; x < bw; ++x) {
           long long q = o + ((long long)z * a.ny + y) * a.nx + x;
-          if (__ldg(&a.bmask[q])) {
+          if (!MASK || __ldg(&a.bmask[q])) {
             double d = __dsub_rn((double)__ldg(&a.base[q]), mean);
             sxx = __dadd_rn(sxx, __dmul_rn(d, d));
             sxt = __dadd_rn(sxt, d);
@@ -1276,7 +1277,7 @@ constexpr int kXtPitch = 68;      // floats per staged base block (the blocks' b
 constexpr int kXCtasPerSM = 6;    // resident CTAs per SM aimed for
 
 struct XArgs {
-  const uint8_t *wand;  // per block: window wholly inside the search mask
+  const uint8_t *wand;  // per block: window wholly inside the search mask (null: every one is)
   int rpu;              // union row pitch in floats (multiple of 4, the box's x extent)
   int spu;              // x extent of the statistics box (even)
   int soff, xoff;       // where the statistics and the base blocks lie in shared memory (floats)
@@ -1381,7 +1382,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     // of each block)
     static_assert(NL == 64, "one lane per voxel of a base block");
     const BlockStat st = a.bstat[b];
-    const bool sel = !a.selected || a.selected[b], window_in = xa.wand[b] != 0;
+    const bool sel = !a.selected || a.selected[b], window_in = !xa.wand || xa.wand[b] != 0;
     float xv[BPW];
     double mv[BPW];
     {
@@ -1763,7 +1764,7 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
         }
       }
       rc.cnt = cnt;
-      rc.full = 0;
+      rc.full = fast ? 1 : 0;
     }
   }
 }
@@ -2107,7 +2108,7 @@ mirorr_status launch_warp(const NccArgs &a, cudaStream_t s) {
 template <class CW, class CM, class CB>
 mirorr_status launch_fast(const NccArgs &a, cudaStream_t s) {
   MB2_TRY((launch_warp<CW>(a, s)));
-  MB2_TRY((launch_masked<CM, CB>(a, s)));
+  if (!a.no_masks) MB2_TRY((launch_masked<CM, CB>(a, s)));
   return MIRORR_OK;
 }
 
@@ -2219,7 +2220,8 @@ mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
     a.search_al = w.ncc_pad.as<float>();
   }
   // window-AND of the footprint flags per block, one pass per axis
-  {
+  xa.wand = nullptr;
+  if (!a.no_masks) {
     const size_t n1 = (size_t)a.nbx * a.ny * a.nz, n2 = (size_t)a.nbx * a.nby * a.nz;
     MB2_TRY(w.ncc_wand.ensure(n1 + n2 + (size_t)a.nblocks));
     uint8_t *b1 = w.ncc_wand.as<uint8_t>(), *b2 = b1 + n1, *b3 = b2 + n2;
@@ -2248,7 +2250,7 @@ mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
   kernel<<<(unsigned)grid, NL, smem, s>>>(a, xa, tmap, smap);
   MB2_LAUNCH_CHECK();
   if (kev) MB2_CUDA_TRY(cudaEventRecord(kev[1], s));
-  MB2_TRY((launch_masked<CM, CB>(a, s)));
+  if (!a.no_masks) MB2_TRY((launch_masked<CM, CB>(a, s)));
   done = true;
   return MIRORR_OK;
 }
@@ -2298,8 +2300,8 @@ bool run_fast(NccArgs &a, BmWork &w, cudaStream_t s, mirorr_status &st, cudaEven
 mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmask,
                          const float *search, const uint8_t *smask, const float2 *stats,
                          const uint8_t *selected, const BmOut &out, BmWork &w,
-                         unsigned long long *ncc_count, cudaStream_t s, cudaEvent_t *kev,
-                         unsigned long long *xl_count, bool *xl_ran) {
+                         unsigned long long *ncc_count, cudaStream_t s, bool no_masks,
+                         cudaEvent_t *kev, unsigned long long *xl_count, bool *xl_ran) {
   if (g.nblocks > 0x7fffffffLL) {
     set_error("too many blocks (%lld)", g.nblocks);
     return MIRORR_EINVAL;
@@ -2316,6 +2318,7 @@ mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmas
   NccArgs a;
   a.base = base; a.bmask = bmask; a.search = search; a.smask = smask; a.stats = stats;
   a.sp = stats_pitch(g.size[0]);
+  a.no_masks = no_masks ? 1 : 0;
   a.selected = selected;
   a.bstat = w.ncc_bstat.as<BlockStat>();
   a.nx = g.size[0]; a.ny = g.size[1]; a.nz = g.size[2];
@@ -2336,9 +2339,10 @@ mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmas
   {
     long long grid = (g.nblocks + 127) / 128;
     if (grid > (long long)sm_count() * 16) grid = (long long)sm_count() * 16;
-    if (a.bw == 4) block_stat_kernel<4><<<(unsigned)grid, 128, 0, s>>>(a);
-    else if (a.bw == 5) block_stat_kernel<5><<<(unsigned)grid, 128, 0, s>>>(a);
-    else block_stat_kernel<0><<<(unsigned)grid, 128, 0, s>>>(a);
+    auto k = a.bw == 4   ? (no_masks ? block_stat_kernel<4, false> : block_stat_kernel<4, true>)
+             : a.bw == 5 ? (no_masks ? block_stat_kernel<5, false> : block_stat_kernel<5, true>)
+                         : (no_masks ? block_stat_kernel<0, false> : block_stat_kernel<0, true>);
+    k<<<(unsigned)grid, 128, 0, s>>>(a);
     MB2_LAUNCH_CHECK();
   }
   mirorr_status st = MIRORR_OK;

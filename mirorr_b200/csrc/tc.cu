@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(256) box_stats16_kernel(const Args16 *calls) {
   const long long ntiles = stats_tiles(a, BW, ntx, nty);
   const T *__restrict__ y = static_cast<const T *>(a.search);
   const uint8_t *__restrict__ ms = a.smask;
+  const bool no_masks = a.no_masks != 0;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const int tid = threadIdx.x, lx = tid & 31, ly = tid >> 5;
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(256) box_stats16_kernel(const Args16 *calls) {
         if (gx < nx && gy < ny) {
           const long long q = (plane + gy) * nx + gx;
           v = S16<T>::f(y[q]);
-          m = ms[q] != 0 ? 1 : 0;
+          m = no_masks || ms[q] != 0 ? 1 : 0;
         }
         s_v[hy][hx] = v;
         s_m[hy][hx] = m;
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(256) prep16_kernel(const Args16 *calls) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         v[i] = S16<T>::f(x[q + i]);
-        mbits |= (mb[q + i] != 0 ? 1u : 0u) << i;
+        mbits |= (a.no_masks || mb[q + i] != 0 ? 1u : 0u) << i;
       }
     }
     const float mu = half_sum((v[0] + v[1]) + (v[2] + v[3])) * (1.0f / kB);
@@ -449,7 +450,7 @@ __global__ void __launch_bounds__(256) prep16_kernel(const Args16 *calls) {
           split3(b, a.nbx, a.nby, bx, by, bz);
           write_out(a, b, -3.f, -3.f,
                     ((long long)(a.stz + bz * a.G) * ny + (a.sty + by * a.G)) * nx + (a.stx + bx * a.G), 0);
-        } else if (a.tensor && pp.mmode == 1 && wand_of(a)[b] && sxx > 0.f) {
+        } else if (a.tensor && pp.mmode == 1 && (a.no_masks || wand_of(a)[b]) && sxx > 0.f) {
           pp.route = 1;
         } else {
           const unsigned int k = atomicAdd(&a.ctl[1], 1u);
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(256) prep16w_kernel(const Args16 *calls) {
 #pragma unroll
         for (int i = 0; i < BW; ++i) {
           v[i] = S16<T>::f(x[q + i]);
-          mbits |= (mb[q + i] != 0 ? 1u : 0u) << i;
+          mbits |= (a.no_masks || mb[q + i] != 0 ? 1u : 0u) << i;
           sum += v[i];
         }
       }
@@ -1212,7 +1213,7 @@ __global__ void __launch_bounds__(C::NT, C::CPS) ncc_fb16_kernel(const Args16 *c
     const int ex = ncx + BW - 1, ey = ncy + BW - 1, ez = ncz + BW - 1;
     const int nc = ncx > 0 && ncy > 0 && ncz > 0 ? ncx * ncy * ncz : 0;
     const Prep16 pp = a.prep[b];
-    const bool full = pp.mmode == 1 && wand_of(a)[b] != 0;
+    const bool full = pp.mmode == 1 && (a.no_masks || wand_of(a)[b] != 0);
     if (nc == 0 || pp.mmode == 2 || (pp.mmode == 1 && pp.sxx <= 0.f)) {
       // no candidate, or Sxx = 0 for every one of them (all degenerate)
       if (tid == 0) {
@@ -1587,12 +1588,16 @@ mirorr_status run16(int ncalls, Match16Call *host_calls, DevBuf &calls_dev, cuda
     else box_stats16_kernel<T, 4><<<dim3((unsigned)gx, (unsigned)ncalls), 256, 0, s>>>(dc);
   }
   MB2_LAUNCH_CHECK();
-  wand_x16_kernel<<<grid_for(max_vox / 2 + 1), 256, 0, s>>>(dc);
-  MB2_LAUNCH_CHECK();
-  wand_y16_kernel<<<grid_for(max_vox / 4 + 1), 256, 0, s>>>(dc);
-  MB2_LAUNCH_CHECK();
-  wand_z16_kernel<<<grid_for(max_blocks), 256, 0, s>>>(dc);
-  MB2_LAUNCH_CHECK();
+  bool masks = every_stage;
+  for (int i = 0; i < ncalls; ++i) masks = masks || (host_calls[i].active && !host_calls[i].no_masks);
+  if (masks) {
+    wand_x16_kernel<<<grid_for(max_vox / 2 + 1), 256, 0, s>>>(dc);
+    MB2_LAUNCH_CHECK();
+    wand_y16_kernel<<<grid_for(max_vox / 4 + 1), 256, 0, s>>>(dc);
+    MB2_LAUNCH_CHECK();
+    wand_z16_kernel<<<grid_for(max_blocks), 256, 0, s>>>(dc);
+    MB2_LAUNCH_CHECK();
+  }
   if (BWc == 5) prep16w_kernel<T, 5><<<grid_for(max_blocks * 32), 256, 0, s>>>(dc);
   else prep16_kernel<T><<<grid_for(max_blocks * 16), 256, 0, s>>>(dc);
   MB2_LAUNCH_CHECK();
@@ -1647,7 +1652,7 @@ mirorr_status launch_match16_batch(int dtype, int ncalls, Match16Call *host_call
 mirorr_status launch_match16(int dtype, const BmGeom &g, const void *base, const uint8_t *bmask,
                              const void *search, const uint8_t *smask, const uint8_t *selected,
                              const BmOut &out, Bm16Work &w, unsigned long long *ncc_count,
-                             cudaStream_t s) {
+                             cudaStream_t s, bool no_masks) {
   if (g.bw != 4 && g.bw != 5) {
     set_error("the 16-bit search supports block widths 4 and 5 (got %d)", g.bw);
     return MIRORR_EINVAL;
@@ -1676,6 +1681,7 @@ mirorr_status launch_match16(int dtype, const BmGeom &g, const void *base, const
   c.bmask = bmask;
   c.search = search;
   c.smask = smask;
+  c.no_masks = no_masks ? 1 : 0;
   c.selected = selected;
   c.stats = w.stats.as<float2>();
   c.wand = w.wand.as<uint8_t>();
