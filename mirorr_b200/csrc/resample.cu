@@ -60,110 +60,136 @@ __device__ inline double dlerp(double a, double b, double t) {
   return __dadd_rn(a, __dmul_rn(__dsub_rn(b, a), t));
 }
 
-// Linear or nearest resampling of one output voxel (i, j, k); cj, ck hold
-// C[r][1] * j and C[r][2] * k (products the whole x-run shares).  Writes the
-// image value to *v and the mask value to *m when the respective input exists.
-template <bool IMG, bool MSK, typename TI, typename TO>
-__device__ __forceinline__ void resample_voxel(const ResampleArgs &a, int i, const double cj[3],
-                                               const double ck[3], TO *v, uint8_t *m) {
-  const TI *in = static_cast<const TI *>(a.in);
+// Continuous input index of output voxel (i, j, k); cj, ck hold C[r][1] * j and
+// C[r][2] * k (products the whole x-run shares).
+__device__ __forceinline__ void index_of(const ResampleArgs &a, int i, const double cj[3],
+                                         const double ck[3], double c[3]) {
   const double di = (double)i;
-  double c[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r)
     c[r] = __dadd_rn(__dadd_rn(__dadd_rn(a.e[r], __dmul_rn(a.C[3 * r], di)), cj[r]), ck[r]);
+}
+__device__ __forceinline__ bool inside_of(const ResampleArgs &a, const double c[3]) {
+  return c[0] >= -0.5 && c[0] < (double)a.inx - 0.5 && c[1] >= -0.5 && c[1] < (double)a.iny - 0.5 &&
+         c[2] >= -0.5 && c[2] < (double)a.inz - 0.5;
+}
+
+// Nearest-neighbour resampling of one voxel.
+template <bool IMG, bool MSK, typename TI, typename TO>
+__device__ __forceinline__ void nearest_voxel(const ResampleArgs &a, const double c[3], bool inside,
+                                              TO *v, uint8_t *m) {
+  if (!inside) {
+    if (IMG) st_copy(*v, 0.0f);
+    if (MSK) *m = 0;
+    return;
+  }
   const int nn[3] = {a.inx, a.iny, a.inz};
-  bool inside = true;
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-    if (!(c[r] >= -0.5 && c[r] < (double)nn[r] - 0.5)) inside = false;
-  const bool mread = MSK && !a.mask_ones;
-  if (a.nearest) {
-    if (!inside) {
-      if (IMG) st_copy(*v, 0.0f);
-      if (MSK) *m = 0;
-      return;
-    }
-    if (MSK && a.mask_ones) *m = 255;
-    // NearestNeighborInterpolateImageFunction: index = floor(c + 0.5)
-    long long q = 0, stride = 1;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      int b = (int)floor(__dadd_rn(c[r], 0.5));
-      if (b < 0) b = 0;
-      if (b > nn[r] - 1) b = nn[r] - 1;
-      q += (long long)b * stride;
-      stride *= nn[r];
-    }
-    if (IMG) st_copy(*v, ld_f(in, q));
-    if (mread) *m = __ldg(a.inm + q);
-    return;
-  }
-  if (!IMG && !mread) {
-    if (MSK) *m = inside ? 255 : 0;
-    return;
-  }
-  // Linear: every voxel is evaluated, with its neighbours clamped into the
-  // image (straight-line code, so the voxels of a run overlap), and the
-  // inside test selects the result.  Inside the image the clamps change
-  // nothing: floor(c) lies in [-1, n - 1].
-  int i0[3], i1[3];
-  double t[3];
+  // NearestNeighborInterpolateImageFunction: index = floor(c + 0.5)
+  long long q = 0, stride = 1;
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    const double cc = fmin(fmax(c[r], -1.0), (double)nn[r]);  // NaN -> -1
-    int b = (int)floor(cc);
-    b = b < 0 ? 0 : (b > nn[r] - 1 ? nn[r] - 1 : b);
-    double d = __dsub_rn(c[r], (double)b);
-    if (d <= 0.0) d = 0.0;
-    i0[r] = b;
-    i1[r] = (b + 1 > nn[r] - 1) ? b : b + 1;
-    t[r] = d;
+    int b = (int)floor(__dadd_rn(c[r], 0.5));
+    if (b < 0) b = 0;
+    if (b > nn[r] - 1) b = nn[r] - 1;
+    q += (long long)b * stride;
+    stride *= nn[r];
   }
-  // the eight neighbours: a base pointer and 32-bit deltas (a slice holds
-  // fewer than 2^31 voxels, checked by the launcher)
-  const int sy = a.inx, sz = a.inx * a.iny;
-  const long long q000 = (long long)i0[2] * sz + (long long)(i0[1] * sy + i0[0]);
-  const int dx = i1[0] - i0[0], dy = (i1[1] - i0[1]) * sy, dz = (i1[2] - i0[2]) * sz;
+  if (IMG) st_copy(*v, ld_f(static_cast<const TI *>(a.in), q));
+  if (MSK) *m = a.mask_ones ? 255 : __ldg(a.inm + q);
+}
+
+// Where a voxel's eight neighbours lie and the lerp parameters.  Neighbours are
+// clamped into the image, so every voxel is evaluated and the inside test
+// selects the result (straight-line code: the voxels of a run overlap); inside
+// the image the clamps change nothing, as floor(c) lies in [-1, n - 1].  The
+// floor is one saturating conversion (NaN gives 0) and the clamps are integer
+// ones; t <= 0 becomes 0 by its sign bit (c >= 0 has t >= 0).
+struct Cell {
+  long long q;     // the base neighbour's index
+  int dx, dy, dz;  // to the others (a slice holds fewer than 2^31 voxels,
+                   // checked by the launcher)
+  double t[3];
+};
+__device__ __forceinline__ void cell_of(const ResampleArgs &a, const double c[3], Cell &o) {
+  const int nn[3] = {a.inx, a.iny, a.inz};
+  const int step[3] = {1, a.inx, a.inx * a.iny};
+  int b[3], d[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    b[r] = max(0, min(__double2int_rd(c[r]), nn[r] - 1));
+    d[r] = b[r] < nn[r] - 1 ? step[r] : 0;
+    const double t = __dsub_rn(c[r], (double)b[r]);
+    const int keep = ~(__double2hiint(t) >> 31);
+    o.t[r] = __hiloint2double(__double2hiint(t) & keep, __double2loint(t) & keep);
+  }
+  o.q = (long long)b[2] * step[2] + (b[1] * step[1] + b[0]);
+  o.dx = d[0];
+  o.dy = d[1];
+  o.dz = d[2];
+}
+
+__device__ __forceinline__ double lerp3(const double v[8], const double t[3]) {
+  const double x00 = dlerp(v[0], v[1], t[0]), x10 = dlerp(v[2], v[3], t[0]);
+  const double x01 = dlerp(v[4], v[5], t[0]), x11 = dlerp(v[6], v[7], t[0]);
+  return dlerp(dlerp(x00, x10, t[1]), dlerp(x01, x11, t[1]), t[2]);
+}
+
+// Resampling of output voxel (i, j, k).  Writes the image value to *v; returns
+// the mask value.
+template <bool IMG, bool MSK, typename TI, typename TO>
+__device__ __forceinline__ unsigned int resample_voxel(const ResampleArgs &a, int i,
+                                                       const double cj[3], const double ck[3], TO *v) {
+  double c[3];
+  index_of(a, i, cj, ck, c);
+  const bool inside = inside_of(a, c);
+  if (a.nearest) {
+    uint8_t m = 0;
+    nearest_voxel<IMG, MSK, TI, TO>(a, c, inside, v, &m);
+    return m;
+  }
+  const bool mread = MSK && !a.mask_ones;
+  if (!IMG && !mread) return inside ? 255u : 0u;
+  Cell e;
+  cell_of(a, c, e);
   if (IMG) {
-    const TI *p = in + q000;
-    const double x00 = dlerp((double)ld_f(p, 0), (double)ld_f(p, dx), t[0]);
-    const double x10 = dlerp((double)ld_f(p, dy), (double)ld_f(p, dy + dx), t[0]);
-    const double x01 = dlerp((double)ld_f(p, dz), (double)ld_f(p, dz + dx), t[0]);
-    const double x11 = dlerp((double)ld_f(p, dz + dy), (double)ld_f(p, dz + dy + dx), t[0]);
-    const double val = dlerp(dlerp(x00, x10, t[1]), dlerp(x01, x11, t[1]), t[2]);
+    const TI *p = static_cast<const TI *>(a.in) + e.q;
+    const double n8[8] = {(double)ld_f(p, 0),           (double)ld_f(p, e.dx),
+                          (double)ld_f(p, e.dy),        (double)ld_f(p, e.dy + e.dx),
+                          (double)ld_f(p, e.dz),        (double)ld_f(p, e.dz + e.dx),
+                          (double)ld_f(p, e.dz + e.dy), (double)ld_f(p, e.dz + e.dy + e.dx)};
+    const double val = lerp3(n8, e.t);
     st_v(*v, inside ? val : 0.0);
   }
-  if (MSK && !mread) *m = inside ? 255 : 0;
-  if (mread) {
-    const uint8_t *p = a.inm + q000;
-    const uint8_t m000 = __ldg(p), m100 = __ldg(p + dx), m010 = __ldg(p + dy),
-                  m110 = __ldg(p + dy + dx), m001 = __ldg(p + dz), m101 = __ldg(p + dz + dx),
-                  m011 = __ldg(p + dz + dy), m111 = __ldg(p + dz + dy + dx);
-    if (!inside) {
-      *m = 0;
-    } else if (m000 == m100 && m000 == m010 && m000 == m110 && m000 == m001 && m000 == m101 &&
-               m000 == m011 && m000 == m111) {
-      // every lerp of equal values returns that value exactly
-      *m = m000;
-    } else {
-      const double x00 = dlerp((double)m000, (double)m100, t[0]);
-      const double x10 = dlerp((double)m010, (double)m110, t[0]);
-      const double x01 = dlerp((double)m001, (double)m101, t[0]);
-      const double x11 = dlerp((double)m011, (double)m111, t[0]);
-      double w = dlerp(dlerp(x00, x10, t[1]), dlerp(x01, x11, t[1]), t[2]);
-      if (w < 0.0) w = 0.0;
-      if (w > 255.0) w = 255.0;
-      *m = (uint8_t)(int)w;
-    }
-  }
+  if (!MSK) return 0;
+  if (!mread) return inside ? 255u : 0u;
+  const uint8_t *p = a.inm + e.q;
+  const unsigned int m0 = __ldg(p), m1 = __ldg(p + e.dx), m2 = __ldg(p + e.dy),
+                     m3 = __ldg(p + e.dy + e.dx), m4 = __ldg(p + e.dz), m5 = __ldg(p + e.dz + e.dx),
+                     m6 = __ldg(p + e.dz + e.dy), m7 = __ldg(p + e.dz + e.dy + e.dx);
+  const unsigned int any = m0 | m1 | m2 | m3 | m4 | m5 | m6 | m7;
+  const unsigned int all = m0 & m1 & m2 & m3 & m4 & m5 & m6 & m7;
+  if (!inside) return 0u;
+  if (any == all) return m0;  // every lerp of equal values returns that value exactly
+  const double n8[8] = {(double)m0, (double)m1, (double)m2, (double)m3,
+                        (double)m4, (double)m5, (double)m6, (double)m7};
+  double w = lerp3(n8, e.t);
+  if (w < 0.0) w = 0.0;
+  if (w > 255.0) w = 255.0;
+  return (unsigned int)(int)w;
 }
 
 // Each thread produces a run of 4 consecutive output voxels (linear order, so
 // a run may cross a row) and stores them with one 16-byte image store and one
 // 4-byte mask store.  The output buffers are 16-byte aligned (checked by the
 // launcher).  Per voxel the index map is the same FP64 expression as a plain
-// evaluation; only the j and k products are shared along the run.
+// evaluation; only the j and k products are shared along the run.  Instruction
+// issue is the bound: with the floor and the clamps in integers, 64 registers
+// and four CTAs per SM, a 256 x 256 x 128 image + mask pass takes 97 us (101
+// before), with the default mask 60 us a pass of a registration's finest level
+// (it is not read), and the eight registrations' passes of a batch 279 us (334).
+// Interpolating only the mask's edge voxels, after the run, was slower (118 us;
+// 108 with them dealt to the warp's lanes; FP32 first, 101), as was 32-bit
+// addressing in a second copy of the loop.
 template <bool IMG, bool MSK, typename TI, typename TO>
 __device__ __forceinline__ void resample_runs(const ResampleArgs &a, long long g0, long long gstride) {
   TO *const out = static_cast<TO *>(a.out);
@@ -191,18 +217,19 @@ __device__ __forceinline__ void resample_runs(const ResampleArgs &a, long long g
       ck[r] = __dmul_rn(a.C[3 * r + 2], (double)k);
     }
     TO v[4];
-    uint8_t m[4] = {0, 0, 0, 0};
+    unsigned int m32 = 0;  // the run's mask bytes
     const int cnt = n - o0 < 4 ? (int)(n - o0) : 4;
     if (row_runs) {
       // the run lies in one row: four independent voxels
 #pragma unroll
-      for (int u = 0; u < 4; ++u) resample_voxel<IMG, MSK, TI, TO>(a, i + u, cj, ck, &v[u], &m[u]);
+      for (int u = 0; u < 4; ++u)
+        m32 |= resample_voxel<IMG, MSK, TI, TO>(a, i + u, cj, ck, &v[u]) << (8 * u);
     } else {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         st_copy(v[u], 0.0f);
         if (u < cnt) {
-          resample_voxel<IMG, MSK, TI, TO>(a, i, cj, ck, &v[u], &m[u]);
+          m32 |= resample_voxel<IMG, MSK, TI, TO>(a, i, cj, ck, &v[u]) << (8 * u);
           if (++i == a.onx) {
             i = 0;
             if (++j == a.ony) {
@@ -229,15 +256,13 @@ __device__ __forceinline__ void resample_runs(const ResampleArgs &a, long long g
               make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
         }
       }
-      if (MSK)
-        *reinterpret_cast<uint32_t *>(a.outm + o0) =
-            (uint32_t)m[0] | ((uint32_t)m[1] << 8) | ((uint32_t)m[2] << 16) | ((uint32_t)m[3] << 24);
+      if (MSK) *reinterpret_cast<uint32_t *>(a.outm + o0) = m32;
     } else {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (u < cnt) {
           if (IMG) out[o0 + u] = v[u];
-          if (MSK) a.outm[o0 + u] = m[u];
+          if (MSK) a.outm[o0 + u] = (uint8_t)(m32 >> (8 * u));
         }
       }
     }
@@ -246,7 +271,7 @@ __device__ __forceinline__ void resample_runs(const ResampleArgs &a, long long g
 
 // resident CTAs of 256 threads per SM the resampling kernels are compiled for
 #ifndef MB2_RS_MINB
-#define MB2_RS_MINB 3
+#define MB2_RS_MINB 4
 #endif
 
 template <bool IMG, bool MSK, typename TI, typename TO>
