@@ -35,6 +35,7 @@
 //      ncc_fallback_kernel.
 #include <cuda.h>  // CUtensorMap (the encoder is fetched through the runtime)
 
+#include <algorithm>
 #include <cfloat>
 
 #include "kernels.cuh"
@@ -1346,12 +1347,14 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
       sm + ((128u - ((unsigned int)__cvta_generic_to_shared(sm) & 127u)) & 127u) / sizeof(float));
   float *win = sma;                     // E * E * rpu
   float2 *sst = reinterpret_cast<float2 *>(sma + xa.soff);  // P * W * spu: a group's statistics
-  float *xt = sma + xa.xoff;            // BPW * kXtPitch
+  float *xt = sma + xa.xoff;            // BPW * kXtPitch; then NL * W plane maxima
+  // what a tile's last step reads of these, the next tile writes only after its
+  // first barrier, so that a tile's end needs none
   __shared__ float s_red[BPW][W][2];
   __shared__ int s_deg[BPW][W][2];
-  __shared__ float s_f[BPW][2];
   __shared__ int s_cnt[BPW];
   __shared__ int s_list[BPW][kK];
+  unsigned int blocks_done = 0;
   const int lane = threadIdx.x;
   const int k = lane / W, x = lane - k * W;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -1359,6 +1362,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     mbar_init(&s_bar, 1);
     mbar_init(&s_sbar, 1);
   }
+  if (lane < BPW) s_cnt[lane] = 0;
   __syncthreads();
   unsigned int phase = 0, sphase = 0;
   const unsigned int win_bytes = (unsigned int)(E * E * rpu * sizeof(float));
@@ -1413,7 +1417,6 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
         }
       }
     }
-    if (lane < BPW) s_cnt[lane] = 0;
     // ---- window inside the search mask? -----------------------------------
     const int px = ox + x;
     const bool xok = px >= 0 && px <= nx - 4;
@@ -1496,8 +1499,10 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
                 top2_push(l1, l2, s);
                 sc[cy] = s;
               }
+              xt[lane * W + cz] = -2.f;
               continue;
             }
+            float pm = -FLT_MAX;
 #pragma unroll
             for (int cy = 0; cy < W; ++cy) {
               const float2 q = sj[cy * xa.spu];
@@ -1506,8 +1511,10 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
               float s = fmaxf(sxy * sxy * rsxx * q.y, -FLT_MAX);
               if (q.y <= 0.f) s = -2.f;
               top2_push(l1, l2, s);
+              pm = fmaxf(pm, s);
               sc[cy] = s;
             }
+            xt[lane * W + cz] = pm;  // (the base blocks are in registers by now)
           }
         }
         if (g + 1 < Groups::N) {
@@ -1529,54 +1536,53 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
       if (lane == 0) atomicExch(&a.ctl[5], 1u);
       return;
     }
-    if (state && x == 0) {
-      float f1 = -3.f, f2 = -3.f;
+    float f1 = -3.f, f2 = -3.f;
+    if (state) {
 #pragma unroll
       for (int j = 0; j < W; ++j) top2_merge(f1, f2, s_red[k][j][0], s_red[k][j][1]);
-      s_f[k][0] = f1;
-      s_f[k][1] = f2;
     }
-    __syncthreads();
     if (state && xok) {
-      // candidates within 2 delta of the block's FP32 second-best (a plane's
-      // largest score first: few planes hold one)
-      const float f2 = s_f[k][1];
+      // candidates within 2 delta of the block's FP32 second-best, looked for in
+      // the planes whose largest score is one
       const float T2 = fmaxf(f2 - 2.f * kDelta, -1.999999f);
-      // fewer than two candidates are not degenerate (rare): the lane's first
-      // two degenerate ones in raster order
-      int d1 = -1, d2 = -1;
+      unsigned int planes = 0, valid = 0;
+#pragma unroll
       for (int cz = 0; cz < W; ++cz) {
         if ((unsigned)(oz + cz) > (unsigned)(nz - 4)) continue;
-        const float *sc = win + cz * E_rpu + lane * W;
-        float v[W], m = -FLT_MAX;
-#pragma unroll
-        for (int cy = 0; cy < W; ++cy) {
-          v[cy] = sc[cy];
-          m = fmaxf(m, v[cy]);
-        }
-        const long long prow = ((long long)(oz + cz) * ny + oy) * nx + px;
-        if (f2 <= -2.f) {
-#pragma unroll
-          for (int cy = 0; cy < W; ++cy)
-            if (v[cy] == -2.f) push_deg(d1, d2, (int)(prow + (long long)cy * nx));
-        }
-        if (m >= T2) {
-#pragma unroll
-          for (int cy = 0; cy < W; ++cy)
-            if (v[cy] >= T2) {
-              const int pos = atomicAdd(&s_cnt[k], 1);
-              if (pos < kK) s_list[k][pos] = (int)(prow + (long long)cy * nx);
-            }
-        }
+        valid |= 1u << cz;
+        if (xt[lane * W + cz] >= T2) planes |= 1u << cz;
       }
-      s_deg[k][x][0] = d1;
-      s_deg[k][x][1] = d2;
+      for (; planes; planes &= planes - 1) {
+        const int cz = __ffs(planes) - 1;
+        const float *sc = win + cz * E_rpu + lane * W;
+        const long long prow = ((long long)(oz + cz) * ny + oy) * nx + px;
+#pragma unroll
+        for (int cy = 0; cy < W; ++cy)
+          if (sc[cy] >= T2) {
+            const int pos = atomicAdd(&s_cnt[k], 1);
+            if (pos < kK) s_list[k][pos] = (int)(prow + (long long)cy * nx);
+          }
+      }
+      if (f2 <= -2.f) {
+        // fewer than two candidates are not degenerate (rare): the lane's first
+        // two degenerate ones in raster order
+        int d1 = -1, d2 = -1;
+        for (; valid; valid &= valid - 1) {
+          const int cz = __ffs(valid) - 1;
+          const float *sc = win + cz * E_rpu + lane * W;
+          const long long prow = ((long long)(oz + cz) * ny + oy) * nx + px;
+          for (int cy = 0; cy < W; ++cy)
+            if (sc[cy] == -2.f) push_deg(d1, d2, (int)(prow + (long long)cy * nx));
+        }
+        s_deg[k][x][0] = d1;
+        s_deg[k][x][1] = d2;
+      }
     }
     __syncthreads();
     if (state && x == 0) {
       NccRec &rc = a.rec[b];
-      const float f1 = s_f[k][0], f2 = s_f[k][1];
       int cnt = s_cnt[k];
+      s_cnt[k] = 0;
       rc.f1 = f1;
       rc.f2 = f2;
       if (cnt <= kK) {
@@ -1594,7 +1600,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
       }
       rc.cnt = cnt;
       rc.full = 1;
-      atomicAdd(&a.ctl[3], 1u);
+      ++blocks_done;
       if (a.xl_count) {
         // candidates of the clipped window: valid offsets per axis
         auto nval = [](int o, int n) {
@@ -1604,8 +1610,9 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
         atomicAdd(a.xl_count, (unsigned long long)nval(ox, nx) * nval(oy, ny) * nval(oz, nz));
       }
     }
-    __syncthreads();
   }
+  blocks_done = __reduce_add_sync(0xffffffffu, blocks_done);
+  if ((lane & 31) == 0 && blocks_done) atomicAdd(&a.ctl[3], blocks_done);
 }
 
 // ---------------------------------------------------------------------------
@@ -2205,7 +2212,8 @@ mirorr_status launch_xlane(NccArgs &a, BmWork &w, cudaStream_t s, bool &done,
   xa.xoff = xa.soff + 2 * P * W * xa.spu;
   xa.tpr = (a.nbx + BPW - 1) / BPW;
   xa.ntiles = (long long)xa.tpr * a.nby * a.nbz;
-  const size_t smem = sizeof(float) * ((size_t)xa.xoff + BPW * kXtPitch) + 128;
+  const size_t smem =
+      sizeof(float) * ((size_t)xa.xoff + std::max(BPW * kXtPitch, NL * W)) + 128;
   // tensor box limit
   if (xa.rpu > 256 || xa.spu > 256 || smem > 64 * 1024) return MIRORR_OK;
   // rows of the search image must start on 16 bytes for the 16-byte copies
