@@ -16,6 +16,7 @@
 
 #include <cuda.h>
 
+#include "hostcopy.cuh"
 #include "kernels.cuh"
 
 namespace mb2 {
@@ -160,6 +161,7 @@ struct mirorr_ctx_s {
   // pyramid level, kept for the next registration while its key (geometry,
   // parameters, every buffer its launches address) is unchanged
   HostBuf it_jobs, it_lts_in, it_lts_out;
+  HostCopier copier;  // copies of callers' host arrays
   DevBuf it_jobs_d;
   bool graphs = true;
   struct LevelGraph {
@@ -1138,8 +1140,7 @@ mirorr_status register_impl(mirorr_ctx c, const mirorr_geometry *fg, const void 
 
 mirorr_status upload(mirorr_ctx c, DevBuf &b, const void *host, size_t bytes) {
   MB2_TRY(b.ensure(bytes));
-  MB2_CUDA_TRY(cudaMemcpyAsync(b.ptr, host, bytes, cudaMemcpyHostToDevice, c->stream));
-  return MIRORR_OK;
+  return c->copier.to_device(b.ptr, host, bytes, c->stream);
 }
 
 }  // namespace
@@ -1188,6 +1189,7 @@ mirorr_status mirorr_ctx_destroy(mirorr_ctx c) {
   for (DevBuf *b : bufs) b->release();
   HostBuf *hbufs[] = {&c->it_jobs, &c->it_lts_in, &c->it_lts_out, &c->ltsw.out};
   for (HostBuf *b : hbufs) b->release();
+  c->copier.release();
   for (auto &lg : c->lgraph)
     if (lg.exec) cudaGraphExecDestroy(lg.exec);
   c->timer.release();
@@ -1529,9 +1531,9 @@ mirorr_status mirorr_bm_get_offsets(mirorr_matcher m, size_t capacity, double *b
     return MIRORR_ERANGE;
   }
   if (bp)
-    MB2_CUDA_TRY(cudaMemcpy(bp, m->pts_b.ptr, sizeof(double) * 3 * kept, cudaMemcpyDeviceToHost));
+    MB2_TRY(c->copier.to_host(bp, m->pts_b.ptr, sizeof(double) * 3 * kept, c->stream));
   if (mp)
-    MB2_CUDA_TRY(cudaMemcpy(mp, m->pts_m.ptr, sizeof(double) * 3 * kept, cudaMemcpyDeviceToHost));
+    MB2_TRY(c->copier.to_host(mp, m->pts_m.ptr, sizeof(double) * 3 * kept, c->stream));
   return MIRORR_OK;
 }
 
@@ -1546,7 +1548,7 @@ mirorr_status mirorr_bm_block_results(mirorr_matcher m, size_t capacity, int32_t
   MB2_CUDA_TRY(cudaSetDevice(m->ctx->device));
   if (match_index) {
     std::vector<int32_t> lin(n);
-    MB2_CUDA_TRY(cudaMemcpy(lin.data(), m->match.ptr, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
+    MB2_TRY(m->ctx->copier.to_host(lin.data(), m->match.ptr, sizeof(int32_t) * n, m->ctx->stream));
     const int nx = m->last.size[0], ny = m->last.size[1];
     for (long long b = 0; b < n; ++b) {
       int v = lin[b];
@@ -1555,9 +1557,11 @@ mirorr_status mirorr_bm_block_results(mirorr_matcher m, size_t capacity, int32_t
       match_index[3 * b + 2] = v / (nx * ny);
     }
   }
-  if (best) MB2_CUDA_TRY(cudaMemcpy(best, m->best.ptr, sizeof(float) * n, cudaMemcpyDeviceToHost));
-  if (second) MB2_CUDA_TRY(cudaMemcpy(second, m->second.ptr, sizeof(float) * n, cudaMemcpyDeviceToHost));
-  if (status) MB2_CUDA_TRY(cudaMemcpy(status, m->status.ptr, n, cudaMemcpyDeviceToHost));
+  HostCopier &cp = m->ctx->copier;
+  cudaStream_t st = m->ctx->stream;
+  if (best) MB2_TRY(cp.to_host(best, m->best.ptr, sizeof(float) * n, st));
+  if (second) MB2_TRY(cp.to_host(second, m->second.ptr, sizeof(float) * n, st));
+  if (status) MB2_TRY(cp.to_host(status, m->status.ptr, n, st));
   return MIRORR_OK;
 }
 
@@ -1646,12 +1650,9 @@ static mirorr_status resample_common(mirorr_ctx c, const int32_t in_size[3], con
     if ((st = launch_resample(in_size, pi, pm, out_size, m, pi ? oi.as<float>() : nullptr,
                               pm ? om.as<uint8_t>() : nullptr, c->stream, nearest)) != MIRORR_OK)
       goto done;
-    if (pi && cudaMemcpyAsync(out_image, oi.ptr, sizeof(float) * no, cudaMemcpyDeviceToHost,
-                              c->stream) != cudaSuccess) { st = MIRORR_ECUDA; goto done; }
-    if (pm && cudaMemcpyAsync(out_mask, om.ptr, no, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) {
-      st = MIRORR_ECUDA;
+    if (pi && (st = c->copier.to_host(out_image, oi.ptr, sizeof(float) * no, c->stream)) != MIRORR_OK)
       goto done;
-    }
+    if (pm && (st = c->copier.to_host(out_mask, om.ptr, no, c->stream)) != MIRORR_OK) goto done;
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
       set_error("resample failed: %s", cudaGetErrorString(cudaGetLastError()));
       st = MIRORR_ECUDA;
@@ -1704,10 +1705,7 @@ static mirorr_status resample_final(mirorr_ctx c, const int32_t in_size[3], cons
       MB2_TRY(launch_resample_sinc(in_size, di.as<float>(), out_size, m, oi.as<float>(),
                                    c->stream));
     }
-    MB2_CUDA_TRY(cudaMemcpyAsync(out_image, oi.ptr, sizeof(float) * no, cudaMemcpyDeviceToHost,
-                                 c->stream));
-    MB2_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return MIRORR_OK;
+    return c->copier.to_host(out_image, oi.ptr, sizeof(float) * no, c->stream);
   };
   const mirorr_status st = run();
   cudaStreamSynchronize(c->stream);  // nothing in flight uses the buffers below
@@ -1772,8 +1770,8 @@ static mirorr_status lts_common(mirorr_ctx c, mirorr_transform *t, mirorr_transf
   }
   MB2_TRY(ensure_pts(c, (long long)n));
   if (n) {
-    MB2_CUDA_TRY(cudaMemcpyAsync(c->pts_i.ptr, init, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-    MB2_CUDA_TRY(cudaMemcpyAsync(c->pts_m.ptr, moved, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
+    MB2_TRY(c->copier.to_device(c->pts_i.ptr, init, sizeof(double) * 3 * n, c->stream));
+    MB2_TRY(c->copier.to_device(c->pts_m.ptr, moved, sizeof(double) * 3 * n, c->stream));
   }
   long long cnt[4] = {(long long)n, 0, 0, 0};
   MB2_CUDA_TRY(cudaMemcpyAsync(c->counts.ptr, cnt, sizeof(cnt), cudaMemcpyHostToDevice, c->stream));
@@ -1974,8 +1972,7 @@ mirorr_status mirorr_pyramid_level(mirorr_ctx c, const mirorr_geometry *ig, cons
   const void *lp = nullptr;
   int lt = MIRORR_DTYPE_F32;
   MB2_TRY(make_level(c, *ig, c->up_f.ptr, MIRORR_DTYPE_F32, factors, g, c->lvl_f, &lp, &lt));
-  MB2_CUDA_TRY(cudaMemcpyAsync(out, lp, sizeof(float) * vox(g.size), cudaMemcpyDeviceToHost, c->stream));
-  MB2_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  MB2_TRY(c->copier.to_host(out, lp, sizeof(float) * vox(g.size), c->stream));
   *og = g;
   return MIRORR_OK;
 }
