@@ -328,7 +328,7 @@ MIRORR_API mirorr_status mirorr_register_device(mirorr_ctx ctx, const mirorr_geo
  * advances every running request by one block-matching iteration with one
  * launch per stage for all of them (the variance selections, the tensor-core
  * search of every request's blocks in one persistent launch, every LTS fit in
- * one cooperative launch).  The step's launches run from a CUDA graph: replayed
+ * one launch).  The step's launches run from a CUDA graph: replayed
  * while the running set and their levels stay unchanged, otherwise updated in
  * place.  Requests may be submitted between steps (continuous batching): a new
  * request starts at its coarsest level while the others continue.  Each
@@ -439,8 +439,10 @@ MIRORR_API mirorr_status mirorr_ctx_search_kernel_times(mirorr_ctx ctx, double *
 MIRORR_API mirorr_status mirorr_ctx_resample_times(mirorr_ctx ctx, double *ms, int64_t *passes,
                                         int64_t *voxels);
 /* A test aid with no counterpart in the reference: the number of polls a
- * grid-barrier wait of the LTS kernel and of the variance selection makes
- * before it gives up (0 restores the default of 2^23 polls, about 0.84 s).  When a wait gives up, every CTA of the
+ * grid-barrier wait of the LTS fit (of more than 16,384 point pairs; smaller
+ * fits meet at a hardware barrier and have no such wait) and of the variance
+ * selection makes before it gives up (0 restores the default of 2^23 polls,
+ * about 0.84 s).  When a wait gives up, every CTA of the
  * launch returns, the call returns MIRORR_ETIMEOUT, the caller's transforms
  * are left as they were, and the context stays usable.  A tiny limit makes the
  * waits give up on CTAs that are merely late, which is how the tests reach

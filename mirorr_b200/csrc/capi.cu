@@ -1988,8 +1988,8 @@ mirorr_status mirorr_pyramid_level(mirorr_ctx c, const mirorr_geometry *ig, cons
 // of them: the resampling passes, the 16-bit search of every matcher call
 // (box statistics, window-AND, base blocks, the tensor-core search over all
 // calls' tiles in one persistent launch, the direct search), the
-// post-filters and the LTS fits (one cooperative launch, a group of CTAs
-// per request).  The host reads the fit states back once per round and
+// post-filters and the LTS fits (one launch, a cluster of CTAs per
+// request).  The host reads the fit states back once per round and
 // advances each request's iteration, level and convergence as the
 // registration methods do (itkMirorrRegistrationMethod.txx:598-658,
 // itkSymMirorrRegistrationMethod.txx:458-720, itkMirorrPyramidImplement.txx:

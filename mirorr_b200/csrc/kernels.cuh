@@ -275,7 +275,7 @@ struct LtsWork {
   HostBuf out;               // pinned read-back of an uncaptured fit (lts_out_bytes)
 };
 // A fit in two halves, so that a captured sequence can hold the first: lts_issue
-// enqueues the upload of *state_in (after lts_begin), the cooperative launch
+// enqueues the upload of *state_in (after lts_begin), the fit's launch
 // and the read-back of the state, the barrier control and the point counts
 // (and *watch_dev when given) into out_host (lts_out_bytes() bytes of host
 // memory, pinned when captured; null: the work area's own); lts_collect, after

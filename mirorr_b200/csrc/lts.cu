@@ -24,8 +24,6 @@
 // iteration of a rigid fit: 84K cycles with a software barrier over 2 to 16
 // CTAs and the matrices of the solve in local memory, 36K now at 7,300 pairs;
 // of a symmetric affine one at 590,000 pairs 150K, now 80K.
-#include <cooperative_groups.h>
-
 #include <mutex>
 
 #include "gridsel.cuh"
