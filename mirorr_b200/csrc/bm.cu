@@ -6,10 +6,11 @@
 //                   itkBlockMatcher.txx:57-68) and the masked sum of squares
 //                   Syy(p) = sum_{ms != 0} (y - mu)^2, both in FP64 in the
 //                   reference's raster order, stored as the float2
-//                   (mu, 1 / Syy), 0 for Syy = 0: the search multiplies by it
-//                   once per block and candidate (some 27 times a voxel); the
-//                   sign bit of the second is set when a search-mask voxel of
-//                   the footprint is 0.
+//                   (mu, 1 / sqrt(Syy)), 0 for Syy = 0: the search multiplies
+//                   by it once per block and candidate (some 27 times a
+//                   voxel), and the root of any float32 image's Syy is a float
+//                   where 1 / Syy may not be one; the sign bit of the second
+//                   is set when a search-mask voxel of the footprint is 0.
 //   2. selection:   (optional) dead-code variance cut-off of
 //                   itkBlockMatcher.txx:664-719, FP64 per block, exact k-th
 //                   value by a device radix select.
@@ -73,7 +74,9 @@ void point_geom(const double origin[3], const double spacing[3], const double di
 // float, a masked voxel differs from it in FP32 exactly when it does in FP64;
 // otherwise an FP32 sum of at least 1e-30 implies a non-zero FP64 one, and
 // below that the position is recomputed with the FP64 two-pass sum, zero
-// exactly when every masked voxel equals the mean, as in the reference.
+// exactly when every masked voxel equals the mean, as in the reference.  (The
+// squares of differences below 1e-22 leave the floats, so a mean as small as the
+// values that differ so little does not count as a float, unless it is 0.)
 constexpr int kBoxPZ = 8;
 
 // FP64 masked sum of squares about mean of the footprint at linear index o
@@ -95,12 +98,27 @@ __device__ __noinline__ double box_ss64(const float *__restrict__ y,
   return ss;
 }
 
+// 1 / sqrt of a position's sum of squares when it does not follow from the FP32
+// sum fs alone (out of line: few positions, if any); *unusual is raised for an
+// unusual one.  NaN, which never scores, stays.
+template <int BW>
+__device__ __noinline__ float box_root(const float *__restrict__ y,
+                                       const uint8_t *__restrict__ ms, long long o, int nx, int ny,
+                                       double mean, float fs, unsigned int *unusual) {
+  double ss = (double)fs;
+  if (fs < 1e-30f) ss = box_ss64<BW>(y, ms, o, nx, ny, mean);
+  if (ss == 0.0) return 0.f;
+  if (ss < (double)kSquaresLo || ss > (double)kSquaresHi) *unusual = 1u;
+  return (float)(ss > 0.0 ? fmax(fmin(rsqrt(ss), (double)FLT_MAX), (double)FLT_MIN) : ss);
+}
+
 // MASK false: no search mask (every voxel counts, none is read).
 template <int BW, bool MASK>
-__global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict__ y,
+__global__ void __launch_bounds__(256, BW <= 5 ? 3 : 2) box_stats_kernel(const float *__restrict__ y,
                                                         const uint8_t *__restrict__ ms, int nx,
                                                         int ny, int nz, int sp,
-                                                        float2 *__restrict__ out) {
+                                                        float2 *__restrict__ out,
+                                                        unsigned int *__restrict__ unusual) {
   constexpr int PZ = kBoxPZ, NP = PZ + BW - 1;
   const int ngz = (nz + PZ - 1) / PZ;
   const long long n = (long long)nx * ny * ngz;
@@ -188,15 +206,15 @@ __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict_
       // not a candidate (the footprint leaves the volume): NaN
       float2 r = make_float2(0.f, __int_as_float(0x7fc00000));
       if (ok[j]) {
-        double ss = (double)s32[j];
+        const float fs = s32[j], mu = (float)mean[j];
+        float rs = fs > 0.f ? rsqrtf(fs) : 0.f;
         // no masked voxel: zero; with a mean that is a float, v - mean is zero
         // in FP32 exactly when it is in FP64; otherwise a tiny FP32 sum is
         // recomputed in FP64
-        if (any_in[j] && s32[j] < 1e-30f && (double)(float)mean[j] != mean[j])
-          ss = box_ss64<BW>(y, ms, o + j * plane, nx, ny, mean[j]);
-        const float fs = (float)ss;
-        const float rs = fs > 0.f ? fmaxf(fminf(__frcp_rn(fs), FLT_MAX), FLT_MIN) : fs;
-        r = make_float2((float)mean[j], all_in[j] ? rs : -rs);
+        if (!(fs >= 1e-30f && fs <= kSquaresHi) && any_in[j] &&
+            (fs != 0.f || (double)mu != mean[j] || (mu != 0.f && fabsf(mu) < 1e-14f)))
+          rs = box_root<BW>(y, ms, o + j * plane, nx, ny, mean[j], fs, unusual);
+        r = make_float2(mu, all_in[j] ? rs : -rs);
       }
       out[((long long)(z0 + j) * ny + yy) * sp + x] = r;
     }
@@ -204,7 +222,8 @@ __global__ void __launch_bounds__(256) box_stats_kernel(const float *__restrict_
 }
 
 mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8_t *smask,
-                               float2 *stats, cudaStream_t s, bool no_masks) {
+                               float2 *stats, unsigned int *unusual, cudaStream_t s,
+                               bool no_masks) {
   long long n = (long long)g.size[0] * g.size[1] * ((g.size[2] + kBoxPZ - 1) / kBoxPZ);
   int threads = 256;
   long long blocks = (n + threads - 1) / threads;
@@ -214,7 +233,7 @@ mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8
   case B: {                                                                                \
     auto k = no_masks ? box_stats_kernel<B, false> : box_stats_kernel<B, true>;            \
     k<<<(unsigned)blocks, threads, 0, s>>>(search, smask, g.size[0], g.size[1], g.size[2], \
-                                           stats_pitch(g.size[0]), stats);                 \
+                                           stats_pitch(g.size[0]), stats, unusual);        \
     break;                                                                                 \
   }
     CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)

@@ -358,8 +358,10 @@ mirorr_status run_match(mirorr_ctx c, const mirorr_bm_params &p, const MatchCall
     if (xl_ran) *xl_ran = false;
   } else {
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[0], s));
+    unsigned int *unusual = nullptr;
+    MB2_TRY(ncc_begin(c->bmw, s, &unusual));
     MB2_TRY(launch_box_stats(g, static_cast<const float *>(mc.search), mc.smask,
-                             c->bmw.stats.as<float2>(), s, mc.no_masks));
+                             c->bmw.stats.as<float2>(), unusual, s, mc.no_masks));
     if (ev) MB2_CUDA_TRY(cudaEventRecord(ev[1], s));
     const uint8_t *sel = nullptr;
     unsigned int *give_up = nullptr;

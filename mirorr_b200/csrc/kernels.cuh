@@ -28,7 +28,8 @@ struct BmWork {
   DevBuf ncc_lists; // block lists of the NCC stages (general path, fallback)
   DevBuf ncc_ctl;   // NCC counters: [0] general-path blocks, [1] fallback blocks,
                     // [2] FP64-refined candidates, [3] fast-path blocks,
-                    // [4] masked-window blocks
+                    // [4] masked-window blocks, [5] an unusual sum of squares,
+                    // [6] a bounded wait gave up
   DevBuf ncc_rec;   // per-block FP32 stage results
   DevBuf ncc_bstat; // per-block base statistics
   DevBuf ncc_pad;   // search image with 16-byte aligned rows (when its own are not)
@@ -54,14 +55,22 @@ void point_geom(const double origin[3], const double spacing[3], const double di
 // Row pitch of the float32 search's statistics (float2 per candidate origin):
 // rows start on 16 bytes, so that a tensor map can address them.
 inline int stats_pitch(int nx) { return (nx + 1) & ~1; }
-// stats: (mean, 1 / masked sum of squares) per candidate origin; the second is
-// 0 when the sum is, NaN where the footprint leaves the volume, and its sign
-// bit is set when some voxel of the footprint is outside the search mask.
+// Masked sums of squares that the float32 search takes as they come: within this
+// range neither they nor the cross terms of two of them leave the normal floats.
+// Any other, but 0, is unusual, and the search looks at each before it trusts
+// its FP32 score (ncc.cu: unsound_pair).
+constexpr float kSquaresLo = 1e-37f, kSquaresHi = 1e30f;
+// stats: (mean, 1 / square root of the masked sum of squares) per candidate
+// origin; the second is 0 when the sum is, NaN where the footprint leaves the
+// volume, and its sign bit is set when some voxel of the footprint is outside
+// the search mask.  *unusual (the word of ncc_begin) becomes 1 when some sum is
+// unusual.
 // no_masks (here and in launch_ncc, launch_match16): the caller set no mask, so
 // the mask buffers hold 255 everywhere; what masks decide is not launched and
 // most kernels do not read them.
 mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8_t *smask,
-                               float2 *stats, cudaStream_t s, bool no_masks);
+                               float2 *stats, unsigned int *unusual, cudaStream_t s,
+                               bool no_masks);
 // base: float32, or 16-bit when dtype is MIRORR_DTYPE_BF16 / _F16.
 // Work-area sizes of one selection: BmWork::var and BmWork::select_state.
 size_t selection_var_bytes(long long nblocks);
@@ -78,6 +87,8 @@ mirorr_status launch_variance_selection(const BmGeom &g, const void *base, doubl
 // scores evaluated.  Profiling (optional): kev[0], kev[1] are recorded around
 // the per-x-lane search kernel's launch and xl_count adds up the candidates it
 // scores; *xl_ran tells whether that kernel ran.
+// Starts a call's counters and its unusual-sums word, before launch_box_stats.
+mirorr_status ncc_begin(BmWork &w, cudaStream_t s, unsigned int **unusual);
 mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmask,
                          const float *search, const uint8_t *smask, const float2 *stats,
                          const uint8_t *selected, const BmOut &out, BmWork &w,

@@ -17,7 +17,13 @@
 //      block_stats).  Per block the stage records the FP32 best and second
 //      and the list of candidates whose FP32 score lies within 2*delta of the
 //      FP32 second-best (delta bounds |FP32 - FP64|), plus the first two
-//      degenerate candidates when fewer than two are non-degenerate.
+//      degenerate candidates when fewer than two are non-degenerate.  The score
+//      is formed as (Sxy / sqrt(Sxx) / sqrt(Syy))^2 from stored reciprocal
+//      roots, so that no square of a sum is ever formed: for images of any
+//      scale the factors are floats where the sums' squares, or 1 / Syy, need
+//      not be.  Where the sums themselves or the cross term's products leave
+//      the floats (unsound_pair) delta bounds nothing, and the block counts as
+//      one whose list overflowed.
 //        * ncc_xlane_kernel (block width 4, window 5, 7 or 9) and
 //          ncc_warp_kernel (other widths): blocks whose base block and search
 //          window are wholly inside both masks, block gap 1; cross term only,
@@ -31,8 +37,8 @@
 //      and the sequential best/second update is replayed over them in
 //      raster order.  No unlisted candidate can be the best or the second,
 //      so the block's best, second and argmax equal the FP64 reference's.
-//      Blocks whose list overflowed are re-scored entirely by
-//      ncc_fallback_kernel.
+//      Blocks whose list overflowed (or whose sums are out of the FP32 search's
+//      range) are re-scored entirely by ncc_fallback_kernel.
 #include <cuda.h>  // CUtensorMap (the encoder is fetched through the runtime)
 
 #include <algorithm>
@@ -46,6 +52,14 @@ namespace {
 
 constexpr int kK = 8;              // refinement list capacity per block
 constexpr float kDelta = 1e-4f;    // bound on |FP32 score - FP64 score|
+// Words of NccArgs::ctl.
+constexpr int kCtlWords = 8;
+constexpr int kCtlUnusual = 5;     // box statistics met an unusual sum of squares
+constexpr int kCtlGaveUp = 6;      // kept until the host reads it
+// Reciprocal roots of the usual sums of squares (kernels.cuh), and the largest
+// that the search takes one by one: at 1e31 the values' differences are about
+// 1e-32, still floats of full precision.
+constexpr float kRootLo = 1e-15f, kRootUsual = 3.1e18f, kRootHi = 1e31f;
 
 // Per-block result of the FP32 stage.
 struct NccRec {
@@ -59,7 +73,8 @@ struct NccRec {
 // Base-block statistics for the FP32 stage.
 struct BlockStat {
   double mean;
-  float sxx;   // sum over masked voxels of (x - mean)^2
+  float rq;    // 1 / sqrt(sum over masked voxels of (x - mean)^2), 0 for a sum of 0;
+               // negated when it is outside [kRootLo, kRootHi]
   float sxt;   // sum over masked voxels of (x - mean)
   int mmode;   // base mask over the block: 1 every voxel non-zero, 2 every voxel zero, 0 mixed
   float c;     // window shift: mean of the block's own candidate footprint
@@ -92,7 +107,7 @@ struct NccArgs {
   int *ovf_list;    // blocks for the fallback kernel
   unsigned int *ctl;  // [0] base-mask blocks, [1] overflow blocks, [2] refined candidates,
                       // [3] register-blocked blocks, [4] masked-window blocks,
-                      // [5] a bounded wait on a tensor copy gave up
+                      // [kCtlUnusual], [kCtlGaveUp] a bounded wait on a tensor copy gave up
   const float *search_al;  // the search image with rows of spitch floats, 16-byte aligned
   int spitch;
   unsigned long long *xl_count;  // optional: candidates scored by the per-x-lane kernel
@@ -251,10 +266,60 @@ __device__ __forceinline__ float sum2(f32x2 v) {
   return lo + hi;
 }
 
-// box_stats stores 1 / Syy (0 when Syy is) with its sign bit set when some
+// box_stats stores 1 / sqrt(Syy) (0 when Syy is) with its sign bit set when some
 // search-mask voxel of the candidate's footprint is zero.
 __device__ inline bool footprint_in_mask(float field) { return !signbit(field); }
-__device__ inline float rsyy_of(float field) { return fabsf(field); }
+__device__ inline float root_of(float field) { return fabsf(field); }
+
+// (Sxy / sqrt(Sxx) / sqrt(Syy))^2 from the reciprocal roots.
+__device__ inline float score_of(float sxy, float rx, float ry) {
+  const float t = sxy * rx * ry;
+  return t * t;
+}
+
+// 1 / sqrt(x) to 2 units in the last place in one instruction; a usual sum is a
+// normal float.
+__device__ __forceinline__ float root_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The FP32 score of a candidate with reciprocal roots rx > 0 and ry is not
+// within delta of the FP64 one: ry (0: degenerate; NaN: not a candidate) is out
+// of range, or sqrt(Sxx Syy) is below 1e-37, where the cross term's products
+// leave the normal floats (their roundings of 2^-150, 512 of them, are 4e-6 of
+// it there).  No pair of usual sums is unsound.
+__device__ inline bool unsound_pair(float rx, float ry) {
+  return (ry > 0.f && ry < kRootLo) || ry > kRootHi || rx * ry > 1e37f;
+}
+// The same for sums of squares formed in FP32 (0: degenerate, if no square left
+// the floats).
+__device__ inline bool unsound_sum(float ss) {
+  return ss > kSquaresHi || (ss > 0.f && ss < kSquaresLo);
+}
+__device__ inline bool square_leaves(float v) { return v != 0.f && fabsf(v) < 1e-19f; }
+// Not 0 when the call's box statistics hold an unusual sum; if 0, the pairs of a
+// block with rx <= kRootUsual need no look.  (The kernels load it with their
+// other set-up and compare it where it is used.)
+__device__ inline unsigned int met_unusual(const NccArgs &a) { return __ldcg(&a.ctl[kCtlUnusual]); }
+// Some candidate of the W x W column of candidates from st (statistics, rows of
+// sp, planes of sz) on makes an unsound pair with rx > 0 (out of line: few calls
+// meet an unusual sum).
+__device__ __noinline__ bool unsound_column(const float2 *st, int sp, long long sz, int y0, int y1,
+                                            int z0, int z1, float rx) {
+  bool bad = false;
+  for (int z = z0; z < z1; ++z)
+    for (int y = y0; y < y1; ++y)
+      bad = bad || unsound_pair(rx, root_of(__ldg(&st[z * sz + (long long)y * sp].y)));
+  return bad;
+}
+// The same for the column at origin x of the window from (y0, z0) on.
+template <int W>
+__device__ __forceinline__ bool unsound_column(const NccArgs &a, int x, int y0, int z0, float rx) {
+  return unsound_column(a.stats + x, a.sp, (long long)a.sp * a.ny, max(y0, 0),
+                        min(y0 + W, a.ny - a.bw + 1), max(z0, 0), min(z0 + W, a.nz - a.bw + 1), rx);
+}
 
 __device__ inline void push_deg(int &d1, int &d2, int p) {
   if (d1 < 0) d1 = p;
@@ -279,6 +344,15 @@ __device__ inline void finish_unmasked_block(const NccArgs &a, long long b) {
 // ---------------------------------------------------------------------------
 // base-block statistics (one thread per block)
 // ---------------------------------------------------------------------------
+// BlockStat::rq of a sum of squares (NaN stays): in FP32, scaled by 2^200 where
+// the sum is below the usual ones.
+__device__ __forceinline__ float block_root(double sxx) {
+  const bool tiny = sxx < (double)kSquaresLo;
+  const float r = rsqrtf((float)(tiny ? sxx * 0x1p200 : sxx)) * (tiny ? 0x1p100f : 1.f);
+  if (sxx <= 0.0) return 0.f;
+  return r > kRootHi || r < kRootLo ? -fmaxf(fminf(r, FLT_MAX), FLT_MIN) : r;
+}
+
 // BW > 0: the block width known at compile time (the block's loads are all
 // issued before the sums); BW = 0: a.bw at run time.  Same arithmetic order.
 template <int BW, bool MASK>
@@ -317,7 +391,7 @@ __global__ void block_stat_kernel(NccArgs a) {
         }
     BlockStat s;
     s.mean = mean;
-    s.sxx = (float)sxx;
+    s.rq = block_root(sxx);
     s.sxt = (float)sxt;
     s.mmode = nin == bw * bw * bw ? 1 : (nin == 0 ? 2 : 0);
     s.c = __ldg(&a.stats[sidx(a, a.stx + bx * a.G, a.sty + by * a.G, a.stz + bz * a.G)]).x;
@@ -543,7 +617,8 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
   __shared__ int s_o[BPC][3];            // window origin (block origin - R)
   __shared__ float s_c[BPC];
   __shared__ float s_sxt[BPC];
-  __shared__ float s_sxx[BPC];
+  __shared__ float s_rq[BPC];
+  __shared__ bool s_look[BPC];         // candidates are looked at with unsound_pair
   __shared__ double s_mean[BPC];
   __shared__ int s_nstr[BPC];
   const int tid = threadIdx.x;
@@ -570,12 +645,15 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
         s_o[tid][1] = oy - R;
         s_o[tid][2] = oz - R;
         const BlockStat st = a.bstat[b];
+        const unsigned int unusual = met_unusual(a);
         if (st.mmode == 1) {
           state = 1;
           s_mean[tid] = st.mean;
           s_sxt[tid] = st.sxt;
-          s_sxx[tid] = st.sxx;
+          s_rq[tid] = st.rq;
           s_c[tid] = st.c;  // the block's own position is a candidate
+          if (st.rq < 0.f) tt.cnt[tid] = kK + 1;
+          s_look[tid] = st.rq > 0.f && (st.rq > kRootUsual || unusual);
         } else {
           unsigned int p = atomicAdd(&a.ctl[0], 1u);
           a.gen_list[p] = b;
@@ -599,6 +677,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
       const long long q = ((long long)(s_o[s][2] + R + vz) * ny + (s_o[s][1] + R + vy)) * nx +
                           (s_o[s][0] + R + vx);
       xt[i] = (float)__dsub_rn((double)__ldg(&a.base[q]), s_mean[s]);
+      if (square_leaves(xt[i])) atomicAdd(&tt.cnt[s], kK + 1);
     }
     __syncthreads();
     // partial-sum tables: entry (vz, vy, pattern) = sums of x~ and x~^2 over
@@ -619,6 +698,11 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
       tab[i] = make_float2(s2, s3);
     }
     const bool active = worker && s_state[slot];
+    if (active && s_look[slot])
+      for (int x = lt; x < W; x += TPB)
+        if (s_o[slot][0] + x >= 0 && s_o[slot][0] + x <= nx - BW &&
+            unsound_column<W>(a, s_o[slot][0] + x, s_o[slot][1], s_o[slot][2], s_rq[slot]))
+          atomicAdd(&tt.cnt[slot], kK + 1);
     float sc[TY][W];
     if (active) {
 #pragma unroll
@@ -662,7 +746,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
     float l1 = -3.f, l2 = -3.f;
     int d1 = -1, d2 = -1;
     if (active) {
-      const float sxt = s_sxt[slot], sxx_b = s_sxx[slot], cc = s_c[slot];
+      const float sxt = s_sxt[slot], rq = s_rq[slot], cc = s_c[slot];
       const int pz = s_o[slot][2] + cz;
 #pragma unroll
       for (int j = 0; j < TY; ++j) {
@@ -679,12 +763,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
           float s = -4.f;  // not a candidate
           if (rowok && px >= 0 && px <= nx - BW) {
             const float2 st = __ldg(&a.stats[srow + x]);
-            const float rsyy = rsyy_of(st.y);
-            if (rsyy <= 0.f) {
+            const float ry = root_of(st.y);
+            if (ry <= 0.f) {
               s = -2.f;
             } else if (footprint_in_mask(st.y)) {
               const float sxy = sc[j][x] - (st.x - cc) * sxt;
-              s = sxx_b <= 0.f ? -2.f : __fdividef(sxy * sxy, sxx_b) * rsyy;
+              s = rq == 0.f ? -2.f : score_of(sxy, rq, ry);
             } else {
               // footprint across the mask edge: C1 kept, finished below
               slist[slot * NC + atomicAdd(&s_nstr[slot], 1)] = cl;
@@ -706,6 +790,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
       const unsigned int *rb = bits + slot * NROW;
       const float2 *tb = tab + slot * NTAB;
       const float cc = s_c[slot];
+      float low = kSquaresHi, ry_max = 0.f;  // of the sums, none above the block's own
       for (int i = lt; i < nstr; i += TPB) {
         const int cl = slist[slot * NC + i];
         const int x = cl % W, cy = (cl / W) % W, czz = cl / (W * W);
@@ -723,11 +808,16 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
                             s_o[slot][0] + x;
         const float2 st = __ldg(&a.stats[sidx(a, s_o[slot][0] + x, s_o[slot][1] + cy, s_o[slot][2] + czz)]);
         const float sxy = scs[slot * NC + cl] - (st.x - cc) * c2;
-        const float s = c3 <= 0.f ? -2.f : __fdividef(sxy * sxy, c3) * rsyy_of(st.y);
+        const float rx = root_approx(c3), ry = root_of(st.y);
+        const float s = c3 <= 0.f ? -2.f : score_of(sxy, rx, ry);
+        low = c3 <= 0.f ? low : fminf(low, c3);
+        ry_max = fmaxf(ry_max, ry);
         scs[slot * NC + cl] = s;
         if (s == -2.f) min2_merge(d1, d2, (int)p, -1);  // list order: keep the two smallest
         top2_merge(l1, l2, s, -3.f);
       }
+      if (low < kSquaresLo || (s_look[slot] && unsound_pair(root_approx(low), ry_max)))
+        atomicAdd(&tt.cnt[slot], kK + 1);
     }
     finish_tile<C>(a, tt, scs, s_b, s_o, s_state, l1, l2, d1, d2, true);
   }
@@ -771,6 +861,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const long long nlist = (long long)*(volatile unsigned int *)&a.ctl[0];
 
+  const unsigned int unusual = met_unusual(a);
   for (long long base = (long long)blockIdx.x * BPC; base < nlist; base += (long long)gridDim.x * BPC) {
     __syncthreads();
     if (tid < BPC) {
@@ -791,6 +882,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
         } else {
           state = 1;
           s_mean[tid] = st.mean;
+          if (st.rq < 0.f) tt.cnt[tid] = kK + 1;
         }
       }
       s_state[tid] = state;
@@ -833,6 +925,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
       const float xv = (float)__dsub_rn((double)__ldg(&a.base[q]), s_mean[s]);
       const float mb = __ldg(&a.bmask[q]) ? 1.f : 0.f;
       if (mb != 0.f) atomicOr(&s_rows[s], 1u << (vz * BW + vy));
+      if (square_leaves(xv)) atomicAdd(&tt.cnt[s], kK + 1);
       xb[i] = make_float4(mb * xv, mb * (xv * xv), mb, 0.f);
     }
     __syncthreads();
@@ -899,6 +992,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
     __syncthreads();  // the windows are free: the scores go there
     float l1 = -3.f, l2 = -3.f;
     int d1 = -1, d2 = -1;
+    float top = 0.f, low = kSquaresLo;  // of the sums of squares, those of degenerate ones aside
     if (active) {
       const int pz = s_o[slot][2] + cz;
 #pragma unroll
@@ -914,13 +1008,19 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
           float s = -4.f;  // not a candidate
           if (rowok && px >= 0 && px <= nx - BW) {
             const float sxy = s1[j][x], sxx = s2[j][x], syy = s3[j][x];
-            s = (sxx <= 0.f || syy <= 0.f) ? -2.f : __fdividef(__fdividef(sxy * sxy, sxx), syy);
+            const float lo = fminf(sxx, syy);
+            s = lo <= 0.f ? -2.f : score_of(sxy, root_approx(sxx), root_approx(syy));
+            top = fmaxf(top, fmaxf(sxx, syy));
+            low = lo <= 0.f ? low : fminf(low, lo);
             if (s == -2.f) push_deg(d1, d2, (int)(prow + x));
             top2_merge(l1, l2, s, -3.f);
           }
           scs[slot * NC + (cz * W + cy) * W + x] = s;
         }
       }
+      // (a zero among unusual sums may be squares that left the floats)
+      if (top > kSquaresHi || low < kSquaresLo || (unusual && d1 >= 0))
+        atomicAdd(&tt.cnt[slot], kK + 1);
     }
     finish_tile<C>(a, tt, scs, s_b, s_o, s_state, l1, l2, d1, d2, false);
   }
@@ -986,6 +1086,7 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
   const unsigned seg = (LPS == 32) ? full : (((1u << LPS) - 1u) << src);
   const long long stride = (long long)gridDim.x * WPC * SPW;
 
+  const unsigned int unusual = met_unusual(a);
   for (long long base = ((long long)blockIdx.x * WPC + warp) * SPW; base < a.nblocks; base += stride) {
     const long long bl = base + sl;
     const bool valid = bl < a.nblocks;
@@ -1047,6 +1148,11 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
     __syncwarp();
     // partly masked window -> masked kernel
     bool inmask = true;
+    if (state && (st.rq < 0.f || unusual || st.rq > kRootUsual)) {
+      bool bad = st.rq < 0.f;
+      for (int e = sln; e < W * W * W; e += LPS) bad = bad || unsound_pair(st.rq, root_of(sst[e].y));
+      if (st.rq != 0.f && bad) atomicAdd(&s_cnt[slot], kK + 1);
+    }
     if (state) {
       for (int e = sln; e < W * W * W; e += LPS) {
         const float2 q = sst[e];
@@ -1116,7 +1222,7 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
           }
         }
       }
-      const float sxt = st.sxt, sxx_b = st.sxx;
+      const float sxt = st.sxt;
 #pragma unroll
       for (int j = 0; j < TY; ++j) {
         const int cy = cy0 + j;
@@ -1126,9 +1232,9 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
           if (cy < W) {
             const float2 q = sst[(cz * W + cy) * W + x];
             if (q.x == q.x) {
-              const float rsyy = rsyy_of(q.y);
+              const float ry = root_of(q.y);
               const float sxy = sc[j][x] - (q.x - cc) * sxt;
-              s = (sxx_b <= 0.f || rsyy <= 0.f) ? -2.f : __fdividef(sxy * sxy, sxx_b) * rsyy;
+              s = (st.rq == 0.f || ry <= 0.f) ? -2.f : score_of(sxy, st.rq, ry);
               if (s == -2.f) push_deg(d1, d2, (int)(((long long)(oz + cz) * ny + oy + cy) * nx + ox + x));
               top2_merge(l1, l2, s, -3.f);
             }
@@ -1257,7 +1363,7 @@ __global__ void wand_axis_kernel(const uint8_t *in, uint8_t *out, long long inne
 //     in registers while its P + 3 window planes pass, each feeding only the
 //     candidate planes that use it, so nothing is multiplied for planes that do
 //     not exist and no accumulator moves;
-//   * the statistics come as (mu, 1 / Syy) by one tensor copy per group.
+//   * the statistics come as (mu, 1 / sqrt(Syy)) by one tensor copy per group.
 // After a group its first window planes are dead, and the scores go there (a
 // CTA barrier says so); lanes without a block run along on placeholder data
 // and write nothing.  After the block-level top-2 reduction a pass over the
@@ -1388,6 +1494,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     static_assert(NL == 64, "one lane per voxel of a base block");
     const BlockStat st = a.bstat[b];
     const bool sel = !a.selected || a.selected[b], window_in = !xa.wand || xa.wand[b] != 0;
+    const unsigned int unusual = met_unusual(a);
     float xv[BPW];
     double mv[BPW];
     {
@@ -1444,6 +1551,9 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
 #pragma unroll
     for (int i = 0; i < BPW; ++i)
       xt[i * kXtPitch + lane] = (float)__dsub_rn((double)xv[i], mv[i]);
+    if (state && (st.rq < 0.f || ((unusual || st.rq > kRootUsual) && xok &&
+                                  unsound_column<W>(a, px, oy, oz, st.rq))))
+      atomicAdd(&s_cnt[k], kK + 1);
     // a wait that gives up is the CTA's decision, taken at a barrier, so no
     // thread is left at one
     bool gave_up = !mbar_wait(&s_bar, phase, 1 << 22);
@@ -1464,15 +1574,12 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
         t[2 * i] = pack2(q.x, q.y);
         t[2 * i + 1] = pack2(q.z, q.w);
       }
-      const float c = st.c, sxt = st.sxt, sxx = st.sxx;
+      const float c = st.c, sxt = st.sxt, rq = st.rq;
       const f32x2 mc = pack2(-c, -c);
-      // (finite for a sum below the normal range: its candidates then tie at 0 and
-      // the block is re-scored in FP64)
-      const float rsxx = sxx > 0.f ? fminf(1.f / sxx, FLT_MAX) : 0.f;
       const float *rp = win + (real ? ox - xu : 0) + x;
       const float2 *sl = sst + (real ? ox - xs : 0) + x;
       float *scp = win + lane * W;
-      const bool live = real && xok, flat = sxx <= 0.f;
+      const bool live = real && xok, flat = rq == 0.f;
 #pragma unroll 1
       for (int g = 0; g < Groups::N; ++g) {
         const int cz0 = Groups::first(g), ns = Groups::scored(g);
@@ -1509,7 +1616,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
               const float2 q = sj[cy * xa.spu];
               const float sxy = sum2(acc[j][cy]) - (q.x - c) * sxt;
               // NaN (not a candidate: a row outside the volume) ranks lowest
-              float s = fmaxf(sxy * sxy * rsxx * q.y, -FLT_MAX);
+              float s = fmaxf(score_of(sxy, rq, q.y), -FLT_MAX);
               if (q.y <= 0.f) s = -2.f;
               top2_push(l1, l2, s);
               pm = fmaxf(pm, s);
@@ -1534,7 +1641,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
       s_red[k][x][1] = l2;
     }
     if (__syncthreads_or(gave_up)) {
-      if (lane == 0) atomicExch(&a.ctl[5], 1u);
+      if (lane == 0) atomicExch(&a.ctl[kCtlGaveUp], 1u);
       return;
     }
     float f1 = -3.f, f2 = -3.f;
@@ -1620,8 +1727,10 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
 // General FP32 search: one CTA (128 threads) per block, any mask pattern and
 // block gap, for geometries without the register-blocked kernels.
 // ---------------------------------------------------------------------------
+// Resident CTAs per SM aimed for (registers).
+constexpr int general_ctas(int bw) { return bw <= 4 && bw != 3 ? 9 : (bw < 6 ? 8 : 12 - bw + 1); }
 template <int BW>
-__global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
+__global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccArgs a) {
   constexpr int B = BW * BW * BW;
   extern __shared__ __align__(16) unsigned char smem[];
   const int e3 = a.emax * a.emax * a.emax;
@@ -1635,6 +1744,7 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
   __shared__ int s_deg[4][2];
   const int tid = threadIdx.x;
 
+  const unsigned int unusual = met_unusual(a);
   for (long long b = blockIdx.x; b < a.nblocks; b += gridDim.x) {
     __syncthreads();
     BlockWin w;
@@ -1653,11 +1763,13 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
       if (tid == 0) finish_unmasked_block(a, b);
       continue;
     }
+    bool left = bst.rq < 0.f;
     for (int v = tid; v < B; v += blockDim.x) {
       int vx = v % BW, vy = (v / BW) % BW, vz = v / (BW * BW);
       long long q = obase + ((long long)vz * a.ny + vy) * a.nx + vx;
       xt[v] = (float)__dsub_rn((double)__ldg(&a.base[q]), bst.mean);
       mb[v] = __ldg(&a.bmask[q]);
+      left = left || square_leaves(xt[v]);
     }
     const long long wbase = lin(a, w.sx, w.sy, w.sz);
     const int nwin = w.ex * w.ey * w.ez;
@@ -1673,6 +1785,8 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
     if (tid == 0) s_cnt = 0;
     const int ms_all = __syncthreads_and(all_in);
     const bool fast = bst.mmode == 1 && ms_all;
+    const bool look = bst.rq > kRootUsual || unusual;
+    if (left) atomicAdd(&s_cnt, kK + 1);
     float l1 = -3.f, l2 = -3.f;
     int d1 = -1, d2 = -1;
     // pass 0 scores every candidate (FP32 top-2, first degenerate candidates);
@@ -1716,7 +1830,8 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
         float2 st = __ldg(&a.stats[sidx(a, px, py, pz)]);
         const float mu = st.x;
         const int woff = ((cz * a.g) * w.ey + cy * a.g) * w.ex + cx * a.g;
-        float sxy = 0.f, sxx, syy = 1.f, rsyy = 1.f;
+        const float ryb = root_of(st.y);
+        float sxy = 0.f, rx, ry;
         if (fast) {
           float acc = 0.f;
 #pragma unroll
@@ -1727,8 +1842,9 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
               for (int vx = 0; vx < BW; ++vx)
                 acc = fmaf(xt[(vz * BW + vy) * BW + vx], yw[woff + (vz * w.ey + vy) * w.ex + vx], acc);
           sxy = acc - mu * bst.sxt;
-          sxx = bst.sxx;
-          rsyy = rsyy_of(st.y);
+          rx = bst.rq;
+          ry = ryb;
+          if (look && rx > 0.f && unsound_pair(rx, ry)) atomicAdd(&s_cnt, kK + 1);
         } else {
           float ax = 0.f, ay = 0.f;
 #pragma unroll
@@ -1747,12 +1863,14 @@ __global__ void __launch_bounds__(128) ncc_general_kernel(NccArgs a) {
                   ay = fmaf(d, d, ay);
                 }
               }
-          sxx = ax;
-          if (bst.mmode == 1) rsyy = rsyy_of(st.y);
-          else syy = ay;
+          rx = ax > 0.f ? root_approx(ax) : 0.f;
+          ry = bst.mmode == 1 ? ryb : (ay > 0.f ? root_approx(ay) : 0.f);
+          // (a zero ay among unusual sums may be squares that left the floats)
+          if (unsound_sum(ax) || (ax > 0.f && unsound_pair(rx, ry)) ||
+              (look && bst.mmode != 1 && ay == 0.f))
+            atomicAdd(&s_cnt, kK + 1);
         }
-        float s = (sxx <= 0.f || syy <= 0.f || rsyy <= 0.f) ? -2.f
-                                                              : (sxy * sxy) / sxx / syy * rsyy;
+        const float s = (rx == 0.f || ry == 0.f) ? -2.f : score_of(sxy, rx, ry);
         top2_merge(l1, l2, s, -3.f);
         if (s == -2.f) push_deg(d1, d2, (int)p);
         scs[c] = s;
@@ -2306,6 +2424,18 @@ bool run_fast(NccArgs &a, BmWork &w, cudaStream_t s, mirorr_status &st, cudaEven
 
 }  // namespace
 
+mirorr_status ncc_begin(BmWork &w, cudaStream_t s, unsigned int **unusual) {
+  const void *before = w.ncc_ctl.ptr;
+  MB2_TRY(w.ncc_ctl.ensure(sizeof(unsigned int) * kCtlWords));
+  // the words below kCtlGaveUp restart every call; that one (a bounded wait gave
+  // up) stays set until the host reads it (ncc_take_timeout)
+  MB2_CUDA_TRY(cudaMemsetAsync(w.ncc_ctl.ptr, 0,
+                               sizeof(unsigned int) * (w.ncc_ctl.ptr == before ? kCtlGaveUp : kCtlWords),
+                               s));
+  *unusual = w.ncc_ctl.as<unsigned int>() + kCtlUnusual;
+  return MIRORR_OK;
+}
+
 mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmask,
                          const float *search, const uint8_t *smask, const float2 *stats,
                          const uint8_t *selected, const BmOut &out, BmWork &w,
@@ -2316,14 +2446,8 @@ mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmas
     return MIRORR_EINVAL;
   }
   MB2_TRY(w.ncc_lists.ensure(sizeof(int) * 3 * (g.nblocks + 1)));
-  const void *ctl_before = w.ncc_ctl.ptr;
-  MB2_TRY(w.ncc_ctl.ensure(sizeof(unsigned int) * 8));
   MB2_TRY(w.ncc_rec.ensure(sizeof(NccRec) * g.nblocks));
   MB2_TRY(w.ncc_bstat.ensure(sizeof(BlockStat) * g.nblocks));
-  // counters 0..4 restart every call; [5] (a bounded wait gave up) stays set
-  // until the host reads it (ncc_take_timeout)
-  MB2_CUDA_TRY(cudaMemsetAsync(w.ncc_ctl.ptr, 0,
-                               sizeof(unsigned int) * (w.ncc_ctl.ptr == ctl_before ? 5 : 8), s));
   NccArgs a;
   a.base = base; a.bmask = bmask; a.search = search; a.smask = smask; a.stats = stats;
   a.sp = stats_pitch(g.size[0]);
@@ -2375,15 +2499,15 @@ mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmas
 }
 
 const unsigned int *ncc_timeout_flag(const BmWork &w) {
-  return w.ncc_ctl.ptr ? w.ncc_ctl.as<unsigned int>() + 5 : nullptr;
+  return w.ncc_ctl.ptr ? w.ncc_ctl.as<unsigned int>() + kCtlGaveUp : nullptr;
 }
 
 mirorr_status ncc_give_up_flag(BmWork &w, cudaStream_t s, unsigned int **flag) {
   const void *before = w.ncc_ctl.ptr;
-  MB2_TRY(w.ncc_ctl.ensure(sizeof(unsigned int) * 8));
+  MB2_TRY(w.ncc_ctl.ensure(sizeof(unsigned int) * kCtlWords));
   if (w.ncc_ctl.ptr != before)
-    MB2_CUDA_TRY(cudaMemsetAsync(w.ncc_ctl.ptr, 0, sizeof(unsigned int) * 8, s));
-  *flag = w.ncc_ctl.as<unsigned int>() + 5;
+    MB2_CUDA_TRY(cudaMemsetAsync(w.ncc_ctl.ptr, 0, sizeof(unsigned int) * kCtlWords, s));
+  *flag = w.ncc_ctl.as<unsigned int>() + kCtlGaveUp;
   return MIRORR_OK;
 }
 
@@ -2391,7 +2515,7 @@ mirorr_status ncc_take_timeout(BmWork &w, cudaStream_t s, bool *timed_out) {
   *timed_out = false;
   if (!w.ncc_ctl.ptr) return MIRORR_OK;
   unsigned int f = 0;
-  unsigned int *flag = w.ncc_ctl.as<unsigned int>() + 5;
+  unsigned int *flag = w.ncc_ctl.as<unsigned int>() + kCtlGaveUp;
   MB2_CUDA_TRY(cudaMemcpyAsync(&f, flag, sizeof(f), cudaMemcpyDeviceToHost, s));
   MB2_CUDA_TRY(cudaStreamSynchronize(s));
   if (f) {
