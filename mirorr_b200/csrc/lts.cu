@@ -28,6 +28,7 @@
 
 #include "gridsel.cuh"
 #include "kernels.cuh"
+#include "keyrange.cuh"
 
 namespace mb2 {
 
@@ -35,7 +36,7 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kBins = 2048;
+constexpr int kBins = kKeyBins;
 constexpr int kCandMax = kThreads;  // keys left for the final rank (one per thread)
 constexpr int kRankMax = 96;  // keys ranked by counting without a further histogram
 constexpr int kUnroll = 2;   // pairs a thread has in flight
@@ -51,11 +52,6 @@ constexpr long long kClusterPairs = 16384;
 // round trips (an iteration at 1,000 pairs 25K cycles against 35K on the
 // cluster; equal at about 4,500).
 constexpr long long kSinglePairs = 4096;
-// The first histogram's keys: 64 bins per octave over [2^-12, 2^20) mm^2 (a
-// residual's bit pattern above kKeyLo in steps of 2^46), one bin below and one
-// above.
-constexpr unsigned long long kKeyLo = (1023ULL - 12ULL) << 52;
-constexpr int kKeyShift = 46;
 // Polls of a grid-barrier wait (about 0.84 s with the 100 ns back-off) before
 // the wait gives up, raises the error flag and every CTA returns.
 constexpr long long kDefaultSpinLimit = 1LL << 23;
@@ -204,23 +200,6 @@ __device__ inline double residual(const double (&f)[12], const double (&b)[12], 
     r += d * d;
   }
   return r;
-}
-
-// Bin of a key in the first histogram (see kKeyLo), and the keys [lo, hi] of a
-// bin.
-__device__ inline unsigned int first_bin(unsigned long long key) {
-  if (key < kKeyLo) return 0;
-  const unsigned long long b = (key - kKeyLo) >> kKeyShift;
-  return b < (unsigned long long)(kBins - 2) ? (unsigned int)b + 1u : (unsigned int)(kBins - 1);
-}
-__device__ inline void first_range(int bin, unsigned long long &lo, unsigned long long &hi) {
-  if (bin == 0) {
-    lo = 0;
-    hi = kKeyLo - 1;
-  } else {
-    lo = kKeyLo + ((unsigned long long)(bin - 1) << kKeyShift);
-    hi = bin == kBins - 1 ? ~0ULL : lo + ((1ULL << kKeyShift) - 1);
-  }
 }
 
 // f(key) for this thread's residuals' bit patterns, four loads in flight.
@@ -422,18 +401,14 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, double *resid, int cta, in
         if (pass == 0) {
           first_range(d, lo, hi);
         } else {
-          const unsigned long long top = hi;
-          lo += (unsigned long long)d << shift;
-          hi = lo + ((1ULL << shift) - 1);
-          if (hi > top) hi = top;
+          range_step(lo, hi, shift, d);
         }
         __syncthreads();
         if (bucket <= (unsigned long long)kCandMax || lo == hi) break;
         // more than one CTA's worth of keys is left: the next histogram, of
         // [lo, hi] in kBins steps
         ++pass;
-        shift = 0;
-        while (((hi - lo) >> shift) >= (unsigned long long)kBins) ++shift;
+        shift = range_shift(lo, hi);
         if (!kSingle && cta == 0) {
           unsigned int *zb = a.hist + ((pass + 1) % 3) * kBins;
           for (int i = threadIdx.x; i < kBins; i += kThreads) zb[i] = 0;
@@ -458,7 +433,8 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, double *resid, int cta, in
         for_keys(resid, n, gtid, gstride, [&](unsigned long long key) {
           if (key >= lo && key <= hi) {
             if (kSingle) {
-              ck[atomicAdd(&s_left, 1u)] = key;  // the bucket holds at most kCandMax
+              const unsigned int pos = atomicAdd(&s_left, 1u);
+              if (pos < (unsigned int)kCandMax) ck[pos] = key;
             } else {
               const unsigned long long pos = atomicAdd(&a.ctl->ncand, 1ULL);
               if (pos < (unsigned long long)kCandMax) a.cand[pos] = key;
@@ -480,8 +456,7 @@ __device__ void lts_body(const LtsArgs &a, Sync sync, double *resid, int cta, in
         unsigned long long kk = k < (unsigned long long)nc ? k : (nc > 0 ? nc - 1 : 0);
         if (nc > kRankMax) {
           // one more histogram, of this CTA alone, so that few keys are ranked
-          shift = 0;
-          while (((hi - lo) >> shift) >= (unsigned long long)kBins) ++shift;
+          shift = range_shift(lo, hi);
           for (int i = threadIdx.x; i < kBins; i += kThreads) h[i] = 0;
           __syncthreads();
           if (have) atomicAdd(&h[(mine - lo) >> shift], 1u);
