@@ -2050,7 +2050,7 @@ __global__ void __launch_bounds__(128) ncc_refine_kernel(NccArgs a) {
   // one addition per warp: one per block, all to one address, was a bound
   scored = __reduce_add_sync(0xffffffffu, scored);
   refined = __reduce_add_sync(0xffffffffu, refined);
-  if ((threadIdx.x & 31) == 0 && refined) {
+  if ((threadIdx.x & 31) == 0 && scored) {
     if (a.ncc_count) atomicAdd(a.ncc_count, (unsigned long long)scored);
     atomicAdd(&a.ctl[2], refined);
   }
