@@ -1773,20 +1773,32 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
     }
     const long long wbase = lin(a, w.sx, w.sy, w.sz);
     const int nwin = w.ex * w.ey * w.ez;
+    auto stage = [&](auto put) {
+      for (int k = tid; k < nwin; k += blockDim.x) {
+        int wx = k % w.ex, wy = (k / w.ex) % w.ey, wz = k / (w.ex * w.ey);
+        put(k, wbase + ((long long)wz * a.ny + wy) * a.nx + wx);
+      }
+    };
     int all_in = 1;
-    for (int k = tid; k < nwin; k += blockDim.x) {
-      int wx = k % w.ex, wy = (k / w.ex) % w.ey, wz = k / (w.ex * w.ey);
-      long long q = wbase + ((long long)wz * a.ny + wy) * a.nx + wx;
-      yw[k] = __ldg(&a.search[q]);
+    // the values less the block's constant, as in the other kernels, which keeps
+    // the cross term free of cancellation
+    const float shift = bst.mmode == 1 ? bst.c : 0.f;
+    stage([&](int k, long long q) {
+      yw[k] = __ldg(&a.search[q]) - shift;
       uint8_t m = __ldg(&a.smask[q]);
       mw[k] = m;
       if (!m) all_in = 0;
-    }
+    });
     if (tid == 0) s_cnt = 0;
     const int ms_all = __syncthreads_and(all_in);
     const bool fast = bst.mmode == 1 && ms_all;
     const bool look = bst.rq > kRootUsual || unusual;
     if (left) atomicAdd(&s_cnt, kK + 1);
+    if (bst.mmode == 1 && !ms_all) {
+      // a partly masked window after all: its values as they are
+      stage([&](int k, long long q) { yw[k] = __ldg(&a.search[q]); });
+      __syncthreads();
+    }
     float l1 = -3.f, l2 = -3.f;
     int d1 = -1, d2 = -1;
     // pass 0 scores every candidate (FP32 top-2, first degenerate candidates);
@@ -1841,7 +1853,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
 #pragma unroll
               for (int vx = 0; vx < BW; ++vx)
                 acc = fmaf(xt[(vz * BW + vy) * BW + vx], yw[woff + (vz * w.ey + vy) * w.ex + vx], acc);
-          sxy = acc - mu * bst.sxt;
+          sxy = acc - (mu - bst.c) * bst.sxt;
           rx = bst.rq;
           ry = ryb;
           if (look && rx > 0.f && unsound_pair(rx, ry)) atomicAdd(&s_cnt, kK + 1);
