@@ -2328,7 +2328,7 @@ mirorr_status batch_issue(mirorr_batch b, int njobs, long long max_vox, int ncal
                                true));
   MB2_TRY(launch_postfilter_batch(b->d_pf.as<PfCall>(), ncalls, max_blocks, st));
   MB2_TRY(lts_batch_launch(b->fits.data(), nfits, b->d_lts_args, b->h_lts_args, st));
-  // read back: fit states, point counts, the search's and the fits' give-up flags
+  // read back: fit states, point counts, the search's give-up flags
   unsigned char *rd = b->h_rd.as<unsigned char>();
   MB2_CUDA_TRY(cudaMemcpyAsync(rd, b->d_states.ptr, sizeof(LtsState) * S, cudaMemcpyDeviceToHost, st));
   MB2_CUDA_TRY(cudaMemcpyAsync(rd + sizeof(LtsState) * S, b->d_counts.ptr, sizeof(long long) * 4 * S,

@@ -329,9 +329,6 @@ size_t lts_args_bytes();
 // reused across calls.
 mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, DevBuf &args_dev,
                                HostBuf &args_host, cudaStream_t st);
-// The device word of a fit's scratch that is non-zero when one of its
-// barrier waits gave up.
-const int *lts_fit_error_flag(const void *scratch);
 // lts_run with every scratch buffer in a static device array sized for
 // MIRORR_LTS_NOALLOC_MAX_POINTS pairs: allocates no device memory.  n is the
 // number of pairs (no device counters).  Calls on one device must not overlap.

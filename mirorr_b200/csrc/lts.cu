@@ -618,7 +618,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
   lts_cluster_body(a, blockIdx.x % kClusterCtas);
 }
 
-// Zeroes each fit's barrier, select control and histograms (CTA f: fit f) so
+// Zeroes each fit's select control and histograms (CTA f: fit f) so
 // a batch's launch sequence has the same nodes whatever the number of fits.
 __global__ void lts_batch_zero_kernel(const LtsArgs *args, unsigned long long words) {
   uint4 *p = reinterpret_cast<uint4 *>(args[blockIdx.x].ctl);
@@ -790,12 +790,12 @@ mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, DevBuf &args_dev,
     a.partial = reinterpret_cast<double *>(p);
     p += up(sizeof(double) * kPartial * (size_t)kClusterCtas);
     a.resid = reinterpret_cast<double *>(p);
-    a.spin_limit = kDefaultSpinLimit;
+    a.spin_limit = 0;  // no fit of a batch waits at the grid barrier
   }
   MB2_CUDA_TRY(cudaMemcpyAsync(args_dev.ptr, ha, sizeof(LtsArgs) * nfits, cudaMemcpyHostToDevice, st));
   const LtsArgs *dargs = args_dev.as<LtsArgs>();
-  // zeroed barrier, select control and histograms of every fit (the scratch
-  // starts 256-byte aligned: the region is whole 16-byte words)
+  // zeroed select control and histograms of every fit (the scratch starts 256-byte
+  // aligned: the region is whole 16-byte words)
   const size_t zbytes = up(sizeof(LtsCtl)) + up(sizeof(unsigned int) * 3 * kBins);
   lts_batch_zero_kernel<<<nfits, 256, 0, st>>>(dargs, (unsigned long long)(zbytes / 16));
   MB2_LAUNCH_CHECK();
@@ -804,11 +804,6 @@ mirorr_status lts_batch_launch(const LtsFit *fits, int nfits, DevBuf &args_dev,
   lts_batch_kernel<<<nfits * kClusterCtas, kThreads, kClusterSmem, st>>>(dargs);
   MB2_LAUNCH_CHECK();
   return MIRORR_OK;
-}
-
-// Error flag of fit f's barrier (device word of its scratch).
-const int *lts_fit_error_flag(const void *scratch) {
-  return &static_cast<const LtsCtl *>(scratch)->bar.err;
 }
 
 // ---- allocation-free variant ----------------------------------------------------

@@ -102,8 +102,9 @@ __device__ __forceinline__ void nearest_voxel(const ResampleArgs &a, const doubl
 // clamped into the image, so every voxel is evaluated and the inside test
 // selects the result (straight-line code: the voxels of a run overlap); inside
 // the image the clamps change nothing, as floor(c) lies in [-1, n - 1].  The
-// floor is one saturating conversion (NaN gives 0) and the clamps are integer
-// ones; t <= 0 becomes 0 by its sign bit (c >= 0 has t >= 0).
+// floor is one saturating conversion and the clamps are integer ones, of which the
+// one at 0 also takes what a NaN converts to (the least integer); t <= 0 becomes 0
+// by its sign bit (c >= 0 has t >= 0).
 struct Cell {
   long long q;     // the base neighbour's index
   int dx, dy, dz;  // to the others (a slice holds fewer than 2^31 voxels,

@@ -1,5 +1,13 @@
 // tfm.cuh -- FP64 transform algebra for the registration path, usable on the
-// host and on the device (the LTS solve runs in one device thread).
+// host and on the device.
+//
+// On the device a whole aligned quad of lanes calls together, all four active with
+// the same arguments: functions that take three angles' sines, cosines or arc
+// tangents (sincos3, atan2_3, and through them euler_zxy_matrix, euler_zxy_angles,
+// quat_euler_angles, tfm_set_params, tfm_set_matrix, tfm_compose, tfm_inverse and
+// the fits of a rigid transform) share them out over the quad's lanes by shuffles,
+// which a lone thread or a partial quad would leave waiting.  The LTS solve runs
+// so in one warp (lts.cu).
 //
 // It restates the semantics the reference relies on:
 //   * itk::MatrixOffsetTransformBase: y = M (x - c) + c + t = M x + offset,
@@ -20,8 +28,10 @@
 #include <math.h>
 
 // Every loop over matrix entries has constant bounds and is unrolled on the
-// device, and every index is a constant then, so the matrices live in
-// registers (an index known only at run time would put them into local memory).
+// device, and every index is a constant then, so that the compiler can hold the
+// matrices in registers (an index known only at run time would put them into local
+// memory).  The classic solve's all fit; the symmetric one, at 128 registers a
+// thread, spills 1.3 to 1.4 KB of them.
 #ifdef __CUDACC__
 #define MB2_HD __host__ __device__ inline
 #define MB2_UNROLL _Pragma("unroll")
@@ -181,8 +191,8 @@ MB2_HD void jacobi_rotate(double *a, double *v) {
 // Cyclic Jacobi eigen-decomposition of a symmetric NxN matrix (N = 3 or 4).
 // On return w[] holds eigenvalues in ascending order and column k of v is the
 // eigenvector of w[k].  For N = 4 a sweep takes the planes in three pairs of
-// disjoint ones, whose angles depend on different entries: the two divisions
-// and square roots of a pair overlap.
+// disjoint ones, whose angles depend on different entries: the reciprocal square
+// roots of a pair overlap.
 template <int N>
 MB2_HD void jacobi_eigen(const double *a_in, double *w, double *v) {
   static_assert(N == 3 || N == 4, "3x3 or 4x4");
