@@ -1727,8 +1727,9 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
 // General FP32 search: one CTA (128 threads) per block, any mask pattern and
 // block gap, for geometries without the register-blocked kernels.
 // ---------------------------------------------------------------------------
-// Resident CTAs per SM aimed for (registers).
-constexpr int general_ctas(int bw) { return bw <= 4 && bw != 3 ? 9 : (bw < 6 ? 8 : 12 - bw + 1); }
+// Resident CTAs per SM aimed for (registers); 0: left to the compiler, which for
+// width 4 is faster at 8 (with masks 72 us) than when told so (76) or told 9 (75).
+constexpr int general_ctas(int bw) { return bw == 4 ? 0 : (bw <= 2 ? 9 : (bw <= 5 ? 8 : 13 - bw)); }
 template <int BW>
 __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccArgs a) {
   constexpr int B = BW * BW * BW;
@@ -1742,9 +1743,10 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
   __shared__ int s_cnt, s_list[kK];
   __shared__ float s_red[4][2];
   __shared__ int s_deg[4][2];
+  __shared__ bool s_look;  // candidates are looked at with unsound_pair
   const int tid = threadIdx.x;
+  if (tid == 0) s_cnt = 0;
 
-  const unsigned int unusual = met_unusual(a);
   for (long long b = blockIdx.x; b < a.nblocks; b += gridDim.x) {
     __syncthreads();
     BlockWin w;
@@ -1763,42 +1765,34 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
       if (tid == 0) finish_unmasked_block(a, b);
       continue;
     }
-    bool left = bst.rq < 0.f;
+    if (tid == 0) {
+      s_look = bst.rq > kRootUsual || met_unusual(a);
+      if (bst.rq < 0.f) atomicAdd(&s_cnt, kK + 1);
+    }
     for (int v = tid; v < B; v += blockDim.x) {
       int vx = v % BW, vy = (v / BW) % BW, vz = v / (BW * BW);
       long long q = obase + ((long long)vz * a.ny + vy) * a.nx + vx;
       xt[v] = (float)__dsub_rn((double)__ldg(&a.base[q]), bst.mean);
       mb[v] = __ldg(&a.bmask[q]);
-      left = left || square_leaves(xt[v]);
+      if (square_leaves(xt[v])) atomicAdd(&s_cnt, kK + 1);
     }
     const long long wbase = lin(a, w.sx, w.sy, w.sz);
     const int nwin = w.ex * w.ey * w.ez;
-    auto stage = [&](auto put) {
-      for (int k = tid; k < nwin; k += blockDim.x) {
-        int wx = k % w.ex, wy = (k / w.ex) % w.ey, wz = k / (w.ex * w.ey);
-        put(k, wbase + ((long long)wz * a.ny + wy) * a.nx + wx);
-      }
-    };
     int all_in = 1;
     // the values less the block's constant, as in the other kernels, which keeps
-    // the cross term free of cancellation
+    // the cross term free of cancellation; as they are when the base block is
+    // partly masked (every term is then formed from them)
     const float shift = bst.mmode == 1 ? bst.c : 0.f;
-    stage([&](int k, long long q) {
+    for (int k = tid; k < nwin; k += blockDim.x) {
+      int wx = k % w.ex, wy = (k / w.ex) % w.ey, wz = k / (w.ex * w.ey);
+      long long q = wbase + ((long long)wz * a.ny + wy) * a.nx + wx;
       yw[k] = __ldg(&a.search[q]) - shift;
       uint8_t m = __ldg(&a.smask[q]);
       mw[k] = m;
       if (!m) all_in = 0;
-    });
-    if (tid == 0) s_cnt = 0;
+    }
     const int ms_all = __syncthreads_and(all_in);
     const bool fast = bst.mmode == 1 && ms_all;
-    const bool look = bst.rq > kRootUsual || unusual;
-    if (left) atomicAdd(&s_cnt, kK + 1);
-    if (bst.mmode == 1 && !ms_all) {
-      // a partly masked window after all: its values as they are
-      stage([&](int k, long long q) { yw[k] = __ldg(&a.search[q]); });
-      __syncthreads();
-    }
     float l1 = -3.f, l2 = -3.f;
     int d1 = -1, d2 = -1;
     // pass 0 scores every candidate (FP32 top-2, first degenerate candidates);
@@ -1840,7 +1834,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
           continue;
         }
         float2 st = __ldg(&a.stats[sidx(a, px, py, pz)]);
-        const float mu = st.x;
+        const float mu = st.x - shift;  // the mean of the staged values
         const int woff = ((cz * a.g) * w.ey + cy * a.g) * w.ex + cx * a.g;
         const float ryb = root_of(st.y);
         float sxy = 0.f, rx, ry;
@@ -1853,10 +1847,10 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
 #pragma unroll
               for (int vx = 0; vx < BW; ++vx)
                 acc = fmaf(xt[(vz * BW + vy) * BW + vx], yw[woff + (vz * w.ey + vy) * w.ex + vx], acc);
-          sxy = acc - (mu - bst.c) * bst.sxt;
+          sxy = acc - mu * bst.sxt;
           rx = bst.rq;
           ry = ryb;
-          if (look && rx > 0.f && unsound_pair(rx, ry)) atomicAdd(&s_cnt, kK + 1);
+          if (s_look && rx > 0.f && unsound_pair(rx, ry)) atomicAdd(&s_cnt, kK + 1);
         } else {
           float ax = 0.f, ay = 0.f;
 #pragma unroll
@@ -1879,7 +1873,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
           ry = bst.mmode == 1 ? ryb : (ay > 0.f ? root_approx(ay) : 0.f);
           // (a zero ay among unusual sums may be squares that left the floats)
           if (unsound_sum(ax) || (ax > 0.f && unsound_pair(rx, ry)) ||
-              (look && bst.mmode != 1 && ay == 0.f))
+              (s_look && bst.mmode != 1 && ay == 0.f))
             atomicAdd(&s_cnt, kK + 1);
         }
         const float s = (rx == 0.f || ry == 0.f) ? -2.f : score_of(sxy, rx, ry);
@@ -1892,6 +1886,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
     if (tid == 0) {
       NccRec &rc = a.rec[b];
       int cnt = s_cnt;
+      s_cnt = 0;
       rc.f1 = l1;
       rc.f2 = l2;
       if (cnt <= kK) {
