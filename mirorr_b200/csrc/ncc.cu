@@ -1779,14 +1779,10 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
     const long long wbase = lin(a, w.sx, w.sy, w.sz);
     const int nwin = w.ex * w.ey * w.ez;
     int all_in = 1;
-    // the values less the block's constant, as in the other kernels, which keeps
-    // the cross term free of cancellation; as they are when the base block is
-    // partly masked (every term is then formed from them)
-    const float shift = bst.mmode == 1 ? bst.c : 0.f;
     for (int k = tid; k < nwin; k += blockDim.x) {
       int wx = k % w.ex, wy = (k / w.ex) % w.ey, wz = k / (w.ex * w.ey);
       long long q = wbase + ((long long)wz * a.ny + wy) * a.nx + wx;
-      yw[k] = __ldg(&a.search[q]) - shift;
+      yw[k] = __ldg(&a.search[q]);
       uint8_t m = __ldg(&a.smask[q]);
       mw[k] = m;
       if (!m) all_in = 0;
@@ -1834,7 +1830,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
           continue;
         }
         float2 st = __ldg(&a.stats[sidx(a, px, py, pz)]);
-        const float mu = st.x - shift;  // the mean of the staged values
+        const float mu = st.x;
         const int woff = ((cz * a.g) * w.ey + cy * a.g) * w.ex + cx * a.g;
         const float ryb = root_of(st.y);
         float sxy = 0.f, rx, ry;
