@@ -16,8 +16,8 @@
 //      masked sum of squares come from box_stats, the base block's from
 //      block_stats).  Per block the stage records the FP32 best and second
 //      and the list of candidates whose FP32 score lies within 2*delta of the
-//      FP32 second-best (delta bounds |FP32 - FP64|), plus the first two
-//      degenerate candidates when fewer than two are non-degenerate.  The score
+//      FP32 second-best (delta bounds |FP32 - FP64|, ShiftBound), plus the first
+//      two degenerate candidates when fewer than two are non-degenerate.  The score
 //      is formed as (Sxy / sqrt(Sxx) / sqrt(Syy))^2 from stored reciprocal
 //      roots, so that no square of a sum is ever formed: for images of any
 //      scale the factors are floats where the sums' squares, or 1 / Syy, need
@@ -51,7 +51,28 @@ namespace mb2 {
 namespace {
 
 constexpr int kK = 8;              // refinement list capacity per block
-constexpr float kDelta = 1e-4f;    // bound on |FP32 score - FP64 score|
+constexpr float kDelta = 1e-4f;    // bound on |FP32 score - FP64 score|, and more
+                                   // where ShiftBound says so
+// The cross term sum x~ (y - c) carries the roundings of partial sums that grow
+// with |mu - c|, the candidate's mean beside the constant it is summed about, and a
+// score divides them by the candidate's contrast.  With u = |mu - c| / sqrt(Syy)
+// the root of a score is off by at most 4e-8 B u (measured in FP32 over random,
+// ramp and step blocks of B = 8 to 512 voxels in raster order, 100,000 each: 3.9e-8),
+// 2e-8 B u where two halves are summed apart (PAIRED: 1.9e-8).  So a block's bound
+// is delta or, with u above 20 at width 4, what its largest u asks for.  (Ordinary
+// images have u of 1 to 25; a contrast of 0.01 beside values of 1,000 has 10,000.)
+// A thread's largest u goes to its block's shared word only where it asks for more.
+template <int B, bool PAIRED = false>
+struct ShiftBound {
+  static constexpr float kPerU = (PAIRED ? 4e-8f : 8e-8f) * B;
+  static __device__ __forceinline__ void note(int *word, float u) {
+    if (u > kDelta / kPerU) atomicMax(word, __float_as_int(u));  // (u >= 0: the bits' order)
+  }
+  static __device__ __forceinline__ float delta(int word) {
+    const float k = kPerU * __int_as_float(word);  // 2 e + e^2 with e = k / 2
+    return fmaxf(kDelta, k * (1.f + 0.25f * k));
+  }
+};
 // Words of NccArgs::ctl.
 constexpr int kCtlWords = 8;
 constexpr int kCtlUnusual = 5;     // box statistics met an unusual sum of squares
@@ -74,7 +95,7 @@ struct NccRec {
 struct BlockStat {
   double mean;
   float rq;    // 1 / sqrt(sum over masked voxels of (x - mean)^2), 0 for a sum of 0;
-               // negated when it is outside [kRootLo, kRootHi]
+               // negated where the FP32 scores are not to be trusted (block_unsound)
   float sxt;   // sum over masked voxels of (x - mean)
   int mmode;   // base mask over the block: 1 every voxel non-zero, 2 every voxel zero, 0 mixed
   float c;     // window shift: mean of the block's own candidate footprint
@@ -299,27 +320,12 @@ __device__ inline bool unsound_sum(float ss) {
   return ss > kSquaresHi || (ss > 0.f && ss < kSquaresLo);
 }
 __device__ inline bool square_leaves(float v) { return v != 0.f && fabsf(v) < 1e-19f; }
+// Only blocks with a small mean are looked through for one: floats of 1e-9 that
+// differ do so by 6e-17, and by 1e-19 from the mean of 512 of them.
+__device__ inline bool small_mean(double mean) { return fabs(mean) < 1e-9; }
 // Not 0 when the call's box statistics hold an unusual sum; if 0, the pairs of a
-// block with rx <= kRootUsual need no look.  (The kernels load it with their
-// other set-up and compare it where it is used.)
+// block with rx <= kRootUsual need no look.
 __device__ inline unsigned int met_unusual(const NccArgs &a) { return __ldcg(&a.ctl[kCtlUnusual]); }
-// Some candidate of the W x W column of candidates from st (statistics, rows of
-// sp, planes of sz) on makes an unsound pair with rx > 0 (out of line: few calls
-// meet an unusual sum).
-__device__ __noinline__ bool unsound_column(const float2 *st, int sp, long long sz, int y0, int y1,
-                                            int z0, int z1, float rx) {
-  bool bad = false;
-  for (int z = z0; z < z1; ++z)
-    for (int y = y0; y < y1; ++y)
-      bad = bad || unsound_pair(rx, root_of(__ldg(&st[z * sz + (long long)y * sp].y)));
-  return bad;
-}
-// The same for the column at origin x of the window from (y0, z0) on.
-template <int W>
-__device__ __forceinline__ bool unsound_column(const NccArgs &a, int x, int y0, int z0, float rx) {
-  return unsound_column(a.stats + x, a.sp, (long long)a.sp * a.ny, max(y0, 0),
-                        min(y0 + W, a.ny - a.bw + 1), max(z0, 0), min(z0 + W, a.nz - a.bw + 1), rx);
-}
 
 __device__ inline void push_deg(int &d1, int &d2, int p) {
   if (d1 < 0) d1 = p;
@@ -349,14 +355,38 @@ __device__ inline void finish_unmasked_block(const NccArgs &a, long long b) {
 __device__ __forceinline__ float block_root(double sxx) {
   const bool tiny = sxx < (double)kSquaresLo;
   const float r = rsqrtf((float)(tiny ? sxx * 0x1p200 : sxx)) * (tiny ? 0x1p100f : 1.f);
-  if (sxx <= 0.0) return 0.f;
-  return r > kRootHi || r < kRootLo ? -fmaxf(fminf(r, FLT_MAX), FLT_MIN) : r;
+  return sxx > 0.0 ? fmaxf(fminf(r, FLT_MAX), FLT_MIN) : (sxx <= 0.0 ? 0.f : r);
+}
+
+// Whether block b, with the root rq > 0 of its own sum, has an unsound pair among
+// its candidates, is out of range itself, or has a voxel whose square leaves the
+// floats (which a mask may leave alone with others like it).  Few calls come here.
+__device__ __forceinline__ bool block_unsound(const NccArgs &a, long long b, double mean, float rq) {
+  if (rq > kRootHi || rq < kRootLo) return true;
+  BlockWin w;
+  if (!block_window(a, b, w)) return false;
+  bool bad = false;
+  if (small_mean(mean))
+#pragma unroll 1
+    for (int i = 0; i < a.bw * a.bw * a.bw; ++i) {
+      const int x = i % a.bw, y = (i / a.bw) % a.bw, z = i / (a.bw * a.bw);
+      const double v = (double)__ldg(&a.base[lin(a, w.ox + x, w.oy + y, w.oz + z)]);
+      bad = bad || square_leaves((float)__dsub_rn(v, mean));
+    }
+#pragma unroll 1
+  for (int i = 0; i < w.nc && !bad; ++i) {
+    const int x = i % w.nx, y = (i / w.nx) % w.ny, z = i / (w.nx * w.ny);
+    bad = unsound_pair(rq, root_of(__ldg(&a.stats[sidx(a, w.sx + x * a.g, w.sy + y * a.g,
+                                                       w.sz + z * a.g)].y)));
+  }
+  return bad;
 }
 
 // BW > 0: the block width known at compile time (the block's loads are all
 // issued before the sums); BW = 0: a.bw at run time.  Same arithmetic order.
 template <int BW, bool MASK>
 __global__ void block_stat_kernel(NccArgs a) {
+  const unsigned int unusual = met_unusual(a);
   for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < a.nblocks;
        b += (long long)gridDim.x * blockDim.x) {
     int bx = (int)(b % a.nbx), by = (int)((b / a.nbx) % a.nby), bz = (int)(b / ((long long)a.nbx * a.nby));
@@ -392,6 +422,9 @@ __global__ void block_stat_kernel(NccArgs a) {
     BlockStat s;
     s.mean = mean;
     s.rq = block_root(sxx);
+    if (s.rq > 0.f && (s.rq > kRootUsual || s.rq < kRootLo || unusual || small_mean(mean)) &&
+        block_unsound(a, b, mean, s.rq))
+      s.rq = -s.rq;
     s.sxt = (float)sxt;
     s.mmode = nin == bw * bw * bw ? 1 : (nin == 0 ? 2 : 0);
     s.c = __ldg(&a.stats[sidx(a, a.stx + bx * a.G, a.sty + by * a.G, a.stz + bz * a.G)]).x;
@@ -456,10 +489,12 @@ struct MaskedCfg : FastCfg<BW_, W_, 1, 1> {
   static constexpr int MINB = F::NT <= 64 ? 16 : (F::NT <= 96 ? 10 : 8);
 };
 
-// Shared state of the per-block reduction that ends a CTA tile.
-template <int BPC, int TPB>
+// Shared state of the per-block reduction that ends a CTA tile.  U: the kernel
+// sums about a constant, and notes its threads' largest u.
+template <int BPC, int TPB, bool U>
 struct TileTail {
   float red[BPC][TPB][2];
+  int u[U ? BPC : 1];  // largest u (ShiftBound), zeroed with cnt
   int deg[BPC][TPB][2];
   float f[BPC][2];
   int d[BPC][2];
@@ -472,8 +507,8 @@ struct TileTail {
 // per block), then the candidates within 2 delta of the second-best from the
 // stored scores (scs: W^3 per block, -4 where not a candidate), then the
 // block's record.  count_fast adds the block to the register-blocked count.
-template <class C>
-__device__ void finish_tile(const NccArgs &a, TileTail<C::BPC, C::TPB> &tt, const float *scs,
+template <class C, bool U>
+__device__ void finish_tile(const NccArgs &a, TileTail<C::BPC, C::TPB, U> &tt, const float *scs,
                             const int *s_b, const int (*s_o)[3], const int *s_state, float l1,
                             float l2, int d1, int d2, bool count_fast) {
   constexpr int BPC = C::BPC, TPB = C::TPB, TY = C::TY, W = C::W, NC = C::NC, NYG = C::NYG;
@@ -521,7 +556,8 @@ __device__ void finish_tile(const NccArgs &a, TileTail<C::BPC, C::TPB> &tt, cons
   }
   __syncthreads();
   if (active) {
-    const float T = tt.f[slot][1] - 2.f * kDelta;
+    float T = tt.f[slot][1] - 2.f * kDelta;
+    if constexpr (U) T = tt.f[slot][1] - 2.f * ShiftBound<C::B>::delta(tt.u[slot]);
     const int pz = s_o[slot][2] + cz;
 #pragma unroll
     for (int j = 0; j < TY; ++j) {
@@ -611,14 +647,13 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
   // the list of candidates whose footprint straddles the mask edge
   float *scs = sm;                                                // BPC * NC
   int *slist = reinterpret_cast<int *>(sm + BPC * NC);           // BPC * NC
-  __shared__ TileTail<BPC, TPB> tt;
+  __shared__ TileTail<BPC, TPB, true> tt;
   __shared__ int s_state[BPC];           // 1 compute, 0 skip
   __shared__ int s_b[BPC];
   __shared__ int s_o[BPC][3];            // window origin (block origin - R)
   __shared__ float s_c[BPC];
   __shared__ float s_sxt[BPC];
   __shared__ float s_rq[BPC];
-  __shared__ bool s_look[BPC];         // candidates are looked at with unsound_pair
   __shared__ double s_mean[BPC];
   __shared__ int s_nstr[BPC];
   const int tid = threadIdx.x;
@@ -635,7 +670,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
     if (tid < BPC) {
       long long i = base + tid;
       int state = 0;
-      tt.cnt[tid] = 0;
+      tt.cnt[tid] = tt.u[tid] = 0;
       if (i < nlist) {
         const int b = a.gen_list[a.nblocks + 1 + i];
         s_b[tid] = b;
@@ -645,7 +680,6 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
         s_o[tid][1] = oy - R;
         s_o[tid][2] = oz - R;
         const BlockStat st = a.bstat[b];
-        const unsigned int unusual = met_unusual(a);
         if (st.mmode == 1) {
           state = 1;
           s_mean[tid] = st.mean;
@@ -653,7 +687,6 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
           s_rq[tid] = st.rq;
           s_c[tid] = st.c;  // the block's own position is a candidate
           if (st.rq < 0.f) tt.cnt[tid] = kK + 1;
-          s_look[tid] = st.rq > 0.f && (st.rq > kRootUsual || unusual);
         } else {
           unsigned int p = atomicAdd(&a.ctl[0], 1u);
           a.gen_list[p] = b;
@@ -677,7 +710,6 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
       const long long q = ((long long)(s_o[s][2] + R + vz) * ny + (s_o[s][1] + R + vy)) * nx +
                           (s_o[s][0] + R + vx);
       xt[i] = (float)__dsub_rn((double)__ldg(&a.base[q]), s_mean[s]);
-      if (square_leaves(xt[i])) atomicAdd(&tt.cnt[s], kK + 1);
     }
     __syncthreads();
     // partial-sum tables: entry (vz, vy, pattern) = sums of x~ and x~^2 over
@@ -698,11 +730,6 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
       tab[i] = make_float2(s2, s3);
     }
     const bool active = worker && s_state[slot];
-    if (active && s_look[slot])
-      for (int x = lt; x < W; x += TPB)
-        if (s_o[slot][0] + x >= 0 && s_o[slot][0] + x <= nx - BW &&
-            unsound_column<W>(a, s_o[slot][0] + x, s_o[slot][1], s_o[slot][2], s_rq[slot]))
-          atomicAdd(&tt.cnt[slot], kK + 1);
     float sc[TY][W];
     if (active) {
 #pragma unroll
@@ -746,6 +773,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
     float l1 = -3.f, l2 = -3.f;
     int d1 = -1, d2 = -1;
     if (active) {
+      float um = 0.f;
       const float sxt = s_sxt[slot], rq = s_rq[slot], cc = s_c[slot];
       const int pz = s_o[slot][2] + cz;
 #pragma unroll
@@ -764,6 +792,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
           if (rowok && px >= 0 && px <= nx - BW) {
             const float2 st = __ldg(&a.stats[srow + x]);
             const float ry = root_of(st.y);
+            um = fmaxf(um, fabsf(st.x - cc) * ry);
             if (ry <= 0.f) {
               s = -2.f;
             } else if (footprint_in_mask(st.y)) {
@@ -781,6 +810,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
           scs[slot * NC + cl] = s;
         }
       }
+      ShiftBound<B>::note(&tt.u[slot], um);
     }
     __syncthreads();
     if (active) {
@@ -816,7 +846,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ncc_masked_kernel(NccArgs a) {
         if (s == -2.f) min2_merge(d1, d2, (int)p, -1);  // list order: keep the two smallest
         top2_merge(l1, l2, s, -3.f);
       }
-      if (low < kSquaresLo || (s_look[slot] && unsound_pair(root_approx(low), ry_max)))
+      if (low < kSquaresLo || unsound_pair(root_approx(low), ry_max))
         atomicAdd(&tt.cnt[slot], kK + 1);
     }
     finish_tile<C>(a, tt, scs, s_b, s_o, s_state, l1, l2, d1, d2, true);
@@ -846,7 +876,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
   float *mwin = sm + BPC * WIN;                                  // BPC * WIN: ms
   float4 *xb = reinterpret_cast<float4 *>(sm + 2 * BPC * WIN);  // BPC * B: mb x~, mb x~^2, mb
   float *scs = sm;  // after the correlation pass: BPC * NC scores
-  __shared__ TileTail<BPC, TPB> tt;
+  __shared__ TileTail<BPC, TPB, false> tt;
   __shared__ int s_state[BPC];
   __shared__ int s_b[BPC];
   __shared__ int s_o[BPC][3];
@@ -925,7 +955,6 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
       const float xv = (float)__dsub_rn((double)__ldg(&a.base[q]), s_mean[s]);
       const float mb = __ldg(&a.bmask[q]) ? 1.f : 0.f;
       if (mb != 0.f) atomicOr(&s_rows[s], 1u << (vz * BW + vy));
-      if (square_leaves(xv)) atomicAdd(&tt.cnt[s], kK + 1);
       xb[i] = make_float4(mb * xv, mb * (xv * xv), mb, 0.f);
     }
     __syncthreads();
@@ -1086,7 +1115,6 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
   const unsigned seg = (LPS == 32) ? full : (((1u << LPS) - 1u) << src);
   const long long stride = (long long)gridDim.x * WPC * SPW;
 
-  const unsigned int unusual = met_unusual(a);
   for (long long base = ((long long)blockIdx.x * WPC + warp) * SPW; base < a.nblocks; base += stride) {
     const long long bl = base + sl;
     const bool valid = bl < a.nblocks;
@@ -1116,7 +1144,7 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
         }
       }
     }
-    if (sln == 0) s_cnt[slot] = 0;
+    if (sln == 0) s_cnt[slot] = st.rq < 0.f ? kK + 1 : 0;
     const float cc = st.c;
     // ---- staging: coalesced asynchronous copies (x fastest across lanes) ---
     if (state) {
@@ -1148,11 +1176,6 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
     __syncwarp();
     // partly masked window -> masked kernel
     bool inmask = true;
-    if (state && (st.rq < 0.f || unusual || st.rq > kRootUsual)) {
-      bool bad = st.rq < 0.f;
-      for (int e = sln; e < W * W * W; e += LPS) bad = bad || unsound_pair(st.rq, root_of(sst[e].y));
-      if (st.rq != 0.f && bad) atomicAdd(&s_cnt[slot], kK + 1);
-    }
     if (state) {
       for (int e = sln; e < W * W * W; e += LPS) {
         const float2 q = sst[e];
@@ -1183,7 +1206,7 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
     __syncwarp();
     // ---- FP32 scores of the lane's tile -----------------------------------
     float sc[TY][W];
-    float l1 = -3.f, l2 = -3.f;
+    float l1 = -3.f, l2 = -3.f, um = 0.f;
     int d1 = -1, d2 = -1;
     const bool active = state && worker;
     if (active) {
@@ -1234,6 +1257,7 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
             if (q.x == q.x) {
               const float ry = root_of(q.y);
               const float sxy = sc[j][x] - (q.x - cc) * sxt;
+              um = fmaxf(um, fabsf(q.x - cc) * ry);
               s = (st.rq == 0.f || ry <= 0.f) ? -2.f : score_of(sxy, st.rq, ry);
               if (s == -2.f) push_deg(d1, d2, (int)(((long long)(oz + cz) * ny + oy + cy) * nx + ox + x));
               top2_merge(l1, l2, s, -3.f);
@@ -1252,12 +1276,14 @@ __global__ void __launch_bounds__(C::WPC * 32, C::MINB) ncc_warp_kernel(NccArgs 
       int e2 = __shfl_down_sync(full, d2, off, LPS);
       top2_merge(l1, l2, o1, o2);
       min2_merge(d1, d2, e1, e2);
+      um = fmaxf(um, __shfl_down_sync(full, um, off, LPS));
     }
+    um = __shfl_sync(full, um, src);
     const float f1 = __shfl_sync(full, l1, src), f2 = __shfl_sync(full, l2, src);
     d1 = __shfl_sync(full, d1, src);
     d2 = __shfl_sync(full, d2, src);
     if (active) {
-      const float T = f2 - 2.f * kDelta;
+      const float T = f2 - 2.f * ShiftBound<B>::delta(__float_as_int(um));
 #pragma unroll
       for (int j = 0; j < TY; ++j)
 #pragma unroll
@@ -1459,7 +1485,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
   // first barrier, so that a tile's end needs none
   __shared__ float s_red[BPW][W][2];
   __shared__ int s_deg[BPW][W][2];
-  __shared__ int s_cnt[BPW];
+  __shared__ int s_cnt[BPW], s_um[BPW];
   __shared__ int s_list[BPW][kK];
   unsigned int blocks_done = 0;
   const int lane = threadIdx.x;
@@ -1469,7 +1495,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     mbar_init(&s_bar, 1);
     mbar_init(&s_sbar, 1);
   }
-  if (lane < BPW) s_cnt[lane] = 0;
+  if (lane < BPW) s_cnt[lane] = s_um[lane] = 0;
   __syncthreads();
   unsigned int phase = 0, sphase = 0;
   const unsigned int win_bytes = (unsigned int)(E * E * rpu * sizeof(float));
@@ -1494,7 +1520,6 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     static_assert(NL == 64, "one lane per voxel of a base block");
     const BlockStat st = a.bstat[b];
     const bool sel = !a.selected || a.selected[b], window_in = !xa.wand || xa.wand[b] != 0;
-    const unsigned int unusual = met_unusual(a);
     float xv[BPW];
     double mv[BPW];
     {
@@ -1551,16 +1576,14 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
 #pragma unroll
     for (int i = 0; i < BPW; ++i)
       xt[i * kXtPitch + lane] = (float)__dsub_rn((double)xv[i], mv[i]);
-    if (state && (st.rq < 0.f || ((unusual || st.rq > kRootUsual) && xok &&
-                                  unsound_column<W>(a, px, oy, oz, st.rq))))
-      atomicAdd(&s_cnt[k], kK + 1);
+    if (state && st.rq < 0.f) atomicAdd(&s_cnt[k], kK + 1);
     // a wait that gives up is the CTA's decision, taken at a barrier, so no
     // thread is left at one
     bool gave_up = !mbar_wait(&s_bar, phase, 1 << 22);
     phase ^= 1u;
     __syncthreads();
     // ---- FP32 scores ---------------------------------------------------------
-    float l1 = -3.f, l2 = -3.f;
+    float l1 = -3.f, l2 = -3.f, um = 0.f;
     const int E_rpu = E * rpu;
     {
       // every thread runs the plane loop (it holds CTA barriers); a lane
@@ -1610,11 +1633,12 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
               xt[lane * W + cz] = -2.f;
               continue;
             }
-            float pm = -FLT_MAX;
+            float pm = -FLT_MAX, uu[W];
 #pragma unroll
             for (int cy = 0; cy < W; ++cy) {
               const float2 q = sj[cy * xa.spu];
               const float sxy = sum2(acc[j][cy]) - (q.x - c) * sxt;
+              uu[cy] = fabsf(q.x - c) * q.y;
               // NaN (not a candidate: a row outside the volume) ranks lowest
               float s = fmaxf(score_of(sxy, rq, q.y), -FLT_MAX);
               if (q.y <= 0.f) s = -2.f;
@@ -1622,6 +1646,9 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
               pm = fmaxf(pm, s);
               sc[cy] = s;
             }
+#pragma unroll
+            for (int cy = 0; cy + 1 < W; cy += 2) um = fmaxf(um, fmaxf(uu[cy], uu[cy + 1]));
+            um = fmaxf(um, uu[W - 1]);
             xt[lane * W + cz] = pm;  // (the base blocks are in registers by now)
           }
         }
@@ -1639,6 +1666,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     if (state) {
       s_red[k][x][0] = l1;
       s_red[k][x][1] = l2;
+      ShiftBound<64, true>::note(&s_um[k], um);
     }
     if (__syncthreads_or(gave_up)) {
       if (lane == 0) atomicExch(&a.ctl[kCtlGaveUp], 1u);
@@ -1652,7 +1680,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     if (state && xok) {
       // candidates within 2 delta of the block's FP32 second-best, looked for in
       // the planes whose largest score is one
-      const float T2 = fmaxf(f2 - 2.f * kDelta, -1.999999f);
+      const float T2 = fmaxf(f2 - 2.f * ShiftBound<64, true>::delta(s_um[k]), -1.999999f);
       unsigned int planes = 0, valid = 0;
 #pragma unroll
       for (int cz = 0; cz < W; ++cz) {
@@ -1690,7 +1718,7 @@ __global__ void __launch_bounds__(32 * NW, kXCtasPerSM)
     if (state && x == 0) {
       NccRec &rc = a.rec[b];
       int cnt = s_cnt[k];
-      s_cnt[k] = 0;
+      s_cnt[k] = s_um[k] = 0;
       rc.f1 = f1;
       rc.f2 = f2;
       if (cnt <= kK) {
@@ -1740,12 +1768,12 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
   float *scs = yw + e3;                          // W^3 candidate scores
   uint8_t *mb = reinterpret_cast<uint8_t *>(scs + a.W * a.W * a.W);
   uint8_t *mw = mb + B;
-  __shared__ int s_cnt, s_list[kK];
+  __shared__ int s_cnt, s_um, s_list[kK];
   __shared__ float s_red[4][2];
   __shared__ int s_deg[4][2];
-  __shared__ bool s_look;  // candidates are looked at with unsound_pair
+  __shared__ unsigned int s_unusual;
   const int tid = threadIdx.x;
-  if (tid == 0) s_cnt = 0;
+  if (tid == 0) s_cnt = s_um = 0;
 
   for (long long b = blockIdx.x; b < a.nblocks; b += gridDim.x) {
     __syncthreads();
@@ -1766,7 +1794,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
       continue;
     }
     if (tid == 0) {
-      s_look = bst.rq > kRootUsual || met_unusual(a);
+      s_unusual = met_unusual(a);
       if (bst.rq < 0.f) atomicAdd(&s_cnt, kK + 1);
     }
     for (int v = tid; v < B; v += blockDim.x) {
@@ -1774,7 +1802,6 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
       long long q = obase + ((long long)vz * a.ny + vy) * a.nx + vx;
       xt[v] = (float)__dsub_rn((double)__ldg(&a.base[q]), bst.mean);
       mb[v] = __ldg(&a.bmask[q]);
-      if (square_leaves(xt[v])) atomicAdd(&s_cnt, kK + 1);
     }
     const long long wbase = lin(a, w.sx, w.sy, w.sz);
     const int nwin = w.ex * w.ey * w.ez;
@@ -1789,7 +1816,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
     }
     const int ms_all = __syncthreads_and(all_in);
     const bool fast = bst.mmode == 1 && ms_all;
-    float l1 = -3.f, l2 = -3.f;
+    float l1 = -3.f, l2 = -3.f, um = 0.f;
     int d1 = -1, d2 = -1;
     // pass 0 scores every candidate (FP32 top-2, first degenerate candidates);
     // pass 1 lists those within 2 delta of the second-best from the stored scores
@@ -1805,6 +1832,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
           top2_merge(l1, l2, o1, o2);
           min2_merge(d1, d2, e1, e2);
         }
+        ShiftBound<B>::note(&s_um, um);
         if ((tid & 31) == 0) {
           s_red[tid >> 5][0] = l1; s_red[tid >> 5][1] = l2;
           s_deg[tid >> 5][0] = d1; s_deg[tid >> 5][1] = d2;
@@ -1815,7 +1843,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
           top2_merge(l1, l2, s_red[k][0], s_red[k][1]);
           min2_merge(d1, d2, s_deg[k][0], s_deg[k][1]);
         }
-        T = l2 - 2.f * kDelta;
+        T = l2 - 2.f * ShiftBound<B>::delta(s_um);
       }
       for (int c = tid; c < w.nc; c += blockDim.x) {
         int cx = c % w.nx, cy = (c / w.nx) % w.ny, cz = c / (w.nx * w.ny);
@@ -1844,9 +1872,9 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
               for (int vx = 0; vx < BW; ++vx)
                 acc = fmaf(xt[(vz * BW + vy) * BW + vx], yw[woff + (vz * w.ey + vy) * w.ex + vx], acc);
           sxy = acc - mu * bst.sxt;
+          um = fmaxf(um, fabsf(mu) * ryb);
           rx = bst.rq;
           ry = ryb;
-          if (s_look && rx > 0.f && unsound_pair(rx, ry)) atomicAdd(&s_cnt, kK + 1);
         } else {
           float ax = 0.f, ay = 0.f;
 #pragma unroll
@@ -1869,7 +1897,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
           ry = bst.mmode == 1 ? ryb : (ay > 0.f ? root_approx(ay) : 0.f);
           // (a zero ay among unusual sums may be squares that left the floats)
           if (unsound_sum(ax) || (ax > 0.f && unsound_pair(rx, ry)) ||
-              (s_look && bst.mmode != 1 && ay == 0.f))
+              (s_unusual && bst.mmode != 1 && ay == 0.f))
             atomicAdd(&s_cnt, kK + 1);
         }
         const float s = (rx == 0.f || ry == 0.f) ? -2.f : score_of(sxy, rx, ry);
@@ -1882,7 +1910,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
     if (tid == 0) {
       NccRec &rc = a.rec[b];
       int cnt = s_cnt;
-      s_cnt = 0;
+      s_cnt = s_um = 0;
       rc.f1 = l1;
       rc.f2 = l2;
       if (cnt <= kK) {
