@@ -1396,11 +1396,11 @@ __global__ void wand_axis_kernel(const uint8_t *in, uint8_t *out, long long inne
 // scores lists the candidates within 2 delta of the block's FP32 second-best.
 // Measured (256 x 256 x 128, W = 9, spacing 3, 211 M candidates): 1.83 ms with
 // scalar multiply-adds, four accumulator planes rotating and a division per
-// candidate (14.7 TFLOP/s, 20 % of the nominal FP32 peak); 1.11 ms now (24.3
-// TFLOP/s).  7.1K instructions per warp and tile (were about 15K), 2.8K of them
-// packed multiply-adds; issue is 47 % busy and the FMA pipe 50 %, and the
-// latency of a tile's phases at 12 warps per SM is what is left.  W = 5 (131 x 117 x 61, spacing 2): 0.81 ms in the
-// general kernel, 0.10 ms here.
+// candidate (14.7 TFLOP/s, 20 % of the nominal FP32 peak); 1.12 ms now (24.1
+// TFLOP/s).  7.2K instructions per warp and tile (were about 15K), 2.8K of them
+// packed multiply-adds; issue is 48 % busy and the FMA pipe 51 %, and the
+// latency of a tile's phases at 12 warps per SM is what is left.  W = 5
+// (131 x 117 x 61, spacing 2): 0.81 ms in the general kernel, 0.10 ms here.
 //
 // Blocks whose window is partly masked (window-AND of the footprint flags) go
 // to the masked kernel, blocks with a partly masked base block to the base-mask

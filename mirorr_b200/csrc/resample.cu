@@ -185,7 +185,7 @@ __device__ __forceinline__ unsigned int resample_voxel(const ResampleArgs &a, in
 // launcher).  Per voxel the index map is the same FP64 expression as a plain
 // evaluation; only the j and k products are shared along the run.  Instruction
 // issue is the bound: with the floor and the clamps in integers, 64 registers
-// and four CTAs per SM, a 256 x 256 x 128 image + mask pass takes 97 us (101
+// and four CTAs per SM, a 256 x 256 x 128 image + mask pass takes 97 us (103
 // before), with the default mask 60 us a pass of a registration's finest level
 // (it is not read), and the eight registrations' passes of a batch 279 us (334).
 // Interpolating only the mask's edge voxels, after the run, was slower (118 us;
