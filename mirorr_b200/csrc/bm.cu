@@ -99,8 +99,8 @@ __device__ __noinline__ double box_ss64(const float *__restrict__ y,
 }
 
 // 1 / sqrt of a position's sum of squares when it does not follow from the FP32
-// sum fs alone (out of line: few positions, if any); *unusual is raised for an
-// unusual one.  NaN, which never scores, stays.
+// sum fs alone (out of line: few positions, if any); *unusual becomes infinite for
+// a sum above the usual ones.  NaN, which never scores, stays.
 template <int BW>
 __device__ __noinline__ float box_root(const float *__restrict__ y,
                                        const uint8_t *__restrict__ ms, long long o, int nx, int ny,
@@ -108,7 +108,7 @@ __device__ __noinline__ float box_root(const float *__restrict__ y,
   double ss = (double)fs;
   if (fs < 1e-30f) ss = box_ss64<BW>(y, ms, o, nx, ny, mean);
   if (ss == 0.0) return 0.f;
-  if (ss < (double)kSquaresLo || ss > (double)kSquaresHi) *unusual = 1u;
+  if (ss > (double)kSquaresHi) *unusual = 0x7f800000u;
   return (float)(ss > 0.0 ? fmax(fmin(rsqrt(ss), (double)FLT_MAX), (double)FLT_MIN) : ss);
 }
 
@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(256, BW <= 5 ? 3 : 2) box_stats_kernel(const f
   constexpr int PZ = kBoxPZ, NP = PZ + BW - 1;
   const int ngz = (nz + PZ - 1) / PZ;
   const long long n = (long long)nx * ny * ngz;
+  float top = 0.f;  // this thread's largest root
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n;
        p += (long long)gridDim.x * blockDim.x) {
     int x, yy, gz;
@@ -214,11 +215,15 @@ __global__ void __launch_bounds__(256, BW <= 5 ? 3 : 2) box_stats_kernel(const f
         if (!(fs >= 1e-30f && fs <= kSquaresHi) && any_in[j] &&
             (fs != 0.f || (double)mu != mean[j] || (mu != 0.f && fabsf(mu) < 1e-14f)))
           rs = box_root<BW>(y, ms, o + j * plane, nx, ny, mean[j], fs, unusual);
+        top = fmaxf(top, rs);
         r = make_float2(mu, all_in[j] ? rs : -rs);
       }
       out[((long long)(z0 + j) * ny + yy) * sp + x] = r;
     }
   }
+  // one word per call: few warps, if any, have a larger one to tell
+  const unsigned int bits = __float_as_uint(top);
+  if (top > kRootUsual && bits > __ldcg(unusual)) atomicMax(unusual, bits);
 }
 
 mirorr_status launch_box_stats(const BmGeom &g, const float *search, const uint8_t *smask,

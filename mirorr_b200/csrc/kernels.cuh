@@ -57,14 +57,16 @@ void point_geom(const double origin[3], const double spacing[3], const double di
 inline int stats_pitch(int nx) { return (nx + 1) & ~1; }
 // Masked sums of squares that the float32 search takes as they come: within this
 // range neither they nor the cross terms of two of them leave the normal floats.
-// Any other, but 0, is unusual, and the search looks at each before it trusts
-// its FP32 score (ncc.cu: unsound_pair).
+// Any other, but 0, is unusual, and the search looks for such before it trusts
+// its FP32 scores (ncc.cu: unsound_pair).
 constexpr float kSquaresLo = 1e-37f, kSquaresHi = 1e30f;
+constexpr float kRootUsual = 3.1e18f;  // largest reciprocal root of a usual sum
 // stats: (mean, 1 / square root of the masked sum of squares) per candidate
 // origin; the second is 0 when the sum is, NaN where the footprint leaves the
 // volume, and its sign bit is set when some voxel of the footprint is outside
-// the search mask.  *unusual (the word of ncc_begin) becomes 1 when some sum is
-// unusual.
+// the search mask.  *unusual (the word of ncc_begin, 0 before) becomes the largest
+// of the reciprocal roots above kRootUsual (its bits), infinity when some sum is
+// above kSquaresHi.
 // no_masks (here and in launch_ncc, launch_match16): the caller set no mask, so
 // the mask buffers hold 255 everywhere; what masks decide is not launched and
 // most kernels do not read them.
@@ -87,7 +89,7 @@ mirorr_status launch_variance_selection(const BmGeom &g, const void *base, doubl
 // scores evaluated.  Profiling (optional): kev[0], kev[1] are recorded around
 // the per-x-lane search kernel's launch and xl_count adds up the candidates it
 // scores; *xl_ran tells whether that kernel ran.
-// Starts a call's counters and its unusual-sums word, before launch_box_stats.
+// Starts a call's counters and its word of unusual sums, before launch_box_stats.
 mirorr_status ncc_begin(BmWork &w, cudaStream_t s, unsigned int **unusual);
 mirorr_status launch_ncc(const BmGeom &g, const float *base, const uint8_t *bmask,
                          const float *search, const uint8_t *smask, const float2 *stats,

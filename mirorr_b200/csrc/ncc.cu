@@ -75,12 +75,12 @@ struct ShiftBound {
 };
 // Words of NccArgs::ctl.
 constexpr int kCtlWords = 8;
-constexpr int kCtlUnusual = 5;     // box statistics met an unusual sum of squares
+constexpr int kCtlUnusual = 5;     // largest unusual root of the box statistics
 constexpr int kCtlGaveUp = 6;      // kept until the host reads it
-// Reciprocal roots of the usual sums of squares (kernels.cuh), and the largest
-// that the search takes one by one: at 1e31 the values' differences are about
-// 1e-32, still floats of full precision.
-constexpr float kRootLo = 1e-15f, kRootUsual = 3.1e18f, kRootHi = 1e31f;
+// Reciprocal roots of sums that the search takes (the usual ones have kRootLo to
+// kRootUsual): at 1e31 the values' differences are about 1e-32, still floats of
+// full precision.
+constexpr float kRootLo = 1e-15f, kRootHi = 1e31f;
 
 // Per-block result of the FP32 stage.
 struct NccRec {
@@ -323,9 +323,11 @@ __device__ inline bool square_leaves(float v) { return v != 0.f && fabsf(v) < 1e
 // Only blocks with a small mean are looked through for one: floats of 1e-9 that
 // differ do so by 6e-17, and by 1e-19 from the mean of 512 of them.
 __device__ inline bool small_mean(double mean) { return fabs(mean) < 1e-9; }
-// Not 0 when the call's box statistics hold an unusual sum; if 0, the pairs of a
-// block with rx <= kRootUsual need no look.
-__device__ inline unsigned int met_unusual(const NccArgs &a) { return __ldcg(&a.ctl[kCtlUnusual]); }
+// The largest unusual root of the call's box statistics (launch_box_stats), 0 with
+// none.
+__device__ inline float unusual_root(const NccArgs &a) {
+  return __uint_as_float(__ldcg(&a.ctl[kCtlUnusual]));
+}
 
 __device__ inline void push_deg(int &d1, int &d2, int p) {
   if (d1 < 0) d1 = p;
@@ -359,9 +361,11 @@ __device__ __forceinline__ float block_root(double sxx) {
 }
 
 // Whether block b, with the root rq > 0 of its own sum, has an unsound pair among
-// its candidates, is out of range itself, or has a voxel whose square leaves the
-// floats (which a mask may leave alone with others like it).  Few calls come here.
-__device__ __forceinline__ bool block_unsound(const NccArgs &a, long long b, double mean, float rq) {
+// its candidates (pairs: it may), is out of range itself, or has a voxel whose
+// square leaves the floats (which a mask may leave alone with others like it).  Few
+// calls come here.
+__device__ __forceinline__ bool block_unsound(const NccArgs &a, long long b, double mean, float rq,
+                                              bool pairs) {
   if (rq > kRootHi || rq < kRootLo) return true;
   BlockWin w;
   if (!block_window(a, b, w)) return false;
@@ -374,7 +378,7 @@ __device__ __forceinline__ bool block_unsound(const NccArgs &a, long long b, dou
       bad = bad || square_leaves((float)__dsub_rn(v, mean));
     }
 #pragma unroll 1
-  for (int i = 0; i < w.nc && !bad; ++i) {
+  for (int i = 0; i < (pairs ? w.nc : 0) && !bad; ++i) {
     const int x = i % w.nx, y = (i / w.nx) % w.ny, z = i / (w.nx * w.ny);
     bad = unsound_pair(rq, root_of(__ldg(&a.stats[sidx(a, w.sx + x * a.g, w.sy + y * a.g,
                                                        w.sz + z * a.g)].y)));
@@ -386,7 +390,7 @@ __device__ __forceinline__ bool block_unsound(const NccArgs &a, long long b, dou
 // issued before the sums); BW = 0: a.bw at run time.  Same arithmetic order.
 template <int BW, bool MASK>
 __global__ void block_stat_kernel(NccArgs a) {
-  const unsigned int unusual = met_unusual(a);
+  const float unusual = unusual_root(a);
   for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < a.nblocks;
        b += (long long)gridDim.x * blockDim.x) {
     int bx = (int)(b % a.nbx), by = (int)((b / a.nbx) % a.nby), bz = (int)(b / ((long long)a.nbx * a.nby));
@@ -422,8 +426,9 @@ __global__ void block_stat_kernel(NccArgs a) {
     BlockStat s;
     s.mean = mean;
     s.rq = block_root(sxx);
-    if (s.rq > 0.f && (s.rq > kRootUsual || s.rq < kRootLo || unusual || small_mean(mean)) &&
-        block_unsound(a, b, mean, s.rq))
+    const bool pairs = unusual > kRootHi || s.rq * fmaxf(unusual, kRootUsual) > 1e37f;
+    if (s.rq > 0.f && (pairs || s.rq < kRootLo || small_mean(mean)) &&
+        block_unsound(a, b, mean, s.rq, pairs))
       s.rq = -s.rq;
     s.sxt = (float)sxt;
     s.mmode = nin == bw * bw * bw ? 1 : (nin == 0 ? 2 : 0);
@@ -891,7 +896,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const long long nlist = (long long)*(volatile unsigned int *)&a.ctl[0];
 
-  const unsigned int unusual = met_unusual(a);
+  const float unusual = unusual_root(a);
   for (long long base = (long long)blockIdx.x * BPC; base < nlist; base += (long long)gridDim.x * BPC) {
     __syncthreads();
     if (tid < BPC) {
@@ -1048,7 +1053,7 @@ __global__ void __launch_bounds__(C::NT, 2) ncc_basemask_kernel(NccArgs a) {
         }
       }
       // (a zero among unusual sums may be squares that left the floats)
-      if (top > kSquaresHi || low < kSquaresLo || (unusual && d1 >= 0))
+      if (top > kSquaresHi || low < kSquaresLo || (unusual > 0.f && d1 >= 0))
         atomicAdd(&tt.cnt[slot], kK + 1);
     }
     finish_tile<C>(a, tt, scs, s_b, s_o, s_state, l1, l2, d1, d2, false);
@@ -1771,7 +1776,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
   __shared__ int s_cnt, s_um, s_list[kK];
   __shared__ float s_red[4][2];
   __shared__ int s_deg[4][2];
-  __shared__ unsigned int s_unusual;
+  __shared__ bool s_unusual;
   const int tid = threadIdx.x;
   if (tid == 0) s_cnt = s_um = 0;
 
@@ -1794,7 +1799,7 @@ __global__ void __launch_bounds__(128, general_ctas(BW)) ncc_general_kernel(NccA
       continue;
     }
     if (tid == 0) {
-      s_unusual = met_unusual(a);
+      s_unusual = unusual_root(a) > 0.f;
       if (bst.rq < 0.f) atomicAdd(&s_cnt, kK + 1);
     }
     for (int v = tid; v < B; v += blockDim.x) {
