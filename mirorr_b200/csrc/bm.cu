@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256, BW <= 5 ? 3 : 2) box_stats_kernel(const f
                                                         const uint8_t *__restrict__ ms, int nx,
                                                         int ny, int nz, int sp,
                                                         float2 *__restrict__ out,
-                                                        unsigned int *__restrict__ unusual) {
+                                                        unsigned int *unusual) {
   constexpr int PZ = kBoxPZ, NP = PZ + BW - 1;
   const int ngz = (nz + PZ - 1) / PZ;
   const long long n = (long long)nx * ny * ngz;
